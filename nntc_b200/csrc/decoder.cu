@@ -170,33 +170,63 @@ __global__ void __launch_bounds__(NE_THREADS, 4) k_ls_accumulate_mma(Planes P, c
     }
 }
 
-__global__ void k_ls_reduce(const double* partial, int entries, int planes, const double* omega, double* out)
+// One block per entry: the planes' LS_GRID partials of the entry staged in shared memory by the whole block, then one
+// thread per plane adds its own run in block order, and thread 0 adds the planes in index order with their weights -
+// the order of one thread walking all of it, which was bound by the latency of its strided loads (322 us a launch at
+// 4 x 1024 x 1024 whatever the size of the entry; staged, the chain of LS_GRID additions is what is left).
+constexpr int LR_THREADS = 256;
+
+__global__ void __launch_bounds__(LR_THREADS) k_ls_reduce(const double* partial, int entries, int planes,
+                                                          const double* omega, double* out)
 {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= entries)
-        return;
-    double total = 0.0;
+    extern __shared__ double lr_rows[];   // [plane][LS_GRID + 1]
+    __shared__ double lr_sum[MAX_PLANES];
+    const int e = blockIdx.x;
     for (int p = 0; p < planes; p++)
     {
         const double* row = partial + ((size_t)p * entries + e) * LS_GRID;
+        for (int b = threadIdx.x; b < LS_GRID; b += LR_THREADS)
+            lr_rows[p * (LS_GRID + 1) + b] = row[b];
+    }
+    __syncthreads();
+    if ((int)threadIdx.x < planes)
+    {
+        const double* row = lr_rows + threadIdx.x * (LS_GRID + 1);
         double sum = 0.0;
+#pragma unroll 16
         for (int b = 0; b < LS_GRID; b++)
             sum += row[b];
-        total += omega[p] * sum;
+        lr_sum[threadIdx.x] = sum;
     }
-    out[e] = total;
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        double total = 0.0;
+        for (int p = 0; p < planes; p++)
+            total += omega[p] * lr_sum[p];
+        out[e] = total;
+    }
 }
 
-// Each plane's three objective sums from the normal equations' pass, its CTAs' partials added in block order.
-__global__ void k_ls_obj_reduce(const double* partial, int planes, double* out)
+// Each plane's three objective sums from the normal equations' pass, its CTAs' partials added in block order (staged
+// first, as in k_ls_reduce).
+__global__ void __launch_bounds__(LR_THREADS) k_ls_obj_reduce(const double* partial, int planes, double* out)
 {
-    const int pl = blockIdx.x, q = threadIdx.x;
-    if (pl >= planes || q >= 3)
+    __shared__ double rows[3][LS_GRID + 1];
+    const int pl = blockIdx.x;
+    if (pl >= planes)
         return;
-    double t = 0.0;
-    for (int b = 0; b < LS_GRID; b++)
-        t += partial[((size_t)pl * 3 + q) * LS_GRID + b];
-    out[3 * pl + q] = t;
+    for (int i = threadIdx.x; i < 3 * LS_GRID; i += LR_THREADS)
+        rows[i / LS_GRID][i % LS_GRID] = partial[(size_t)pl * 3 * LS_GRID + i];
+    __syncthreads();
+    if (threadIdx.x < 3)
+    {
+        double t = 0.0;
+#pragma unroll 16
+        for (int b = 0; b < LS_GRID; b++)
+            t += rows[threadIdx.x][b];
+        out[3 * pl + threadIdx.x] = t;
+    }
 }
 
 // obj_sums (the mixed-precision Gram only): also the objective's three raw sums per plane of the decoder on the device,
@@ -255,14 +285,15 @@ int normal_equations(nntc_b200_device* d, int k, const double* per_site, double*
         NB_TRY(ktimer_end(d));
         NB_LAUNCHED();
     }
-    k_ls_reduce<<<grid_for((size_t)entries, 128), 128, 0, d->stream>>>(d->ls_partial, entries, P.n, omega,
-                                                                      d->reduction);
+    const size_t lr_shared = (size_t)P.n * (LS_GRID + 1) * sizeof(double);
+    NB_CUDA(cudaFuncSetAttribute(k_ls_reduce, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lr_shared));
+    k_ls_reduce<<<entries, LR_THREADS, lr_shared, d->stream>>>(d->ls_partial, entries, P.n, omega, d->reduction);
     NB_LAUNCHED();
     const bool with_obj = obj_sums && d->mixed_gram;
     double* obj_out = d->ls_obj + (size_t)P.n * 3 * LS_GRID;
     if (with_obj)
     {
-        k_ls_obj_reduce<<<P.n, 32, 0, d->stream>>>(d->ls_obj, P.n, obj_out);
+        k_ls_obj_reduce<<<P.n, LR_THREADS, 0, d->stream>>>(d->ls_obj, P.n, obj_out);
         NB_LAUNCHED();
     }
     NB_TRY(block_end(d, ms));
