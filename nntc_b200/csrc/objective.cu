@@ -457,22 +457,33 @@ __global__ void __launch_bounds__(OBJ_P_THREADS, 8)
 
 int ensure_site_targets(nntc_b200_device* d, int k, int level0);
 
-// One block per plane: the plane's block partials added in a fixed order (a strided pass, then a fixed tree).
-__global__ void k_objective_reduce(Planes P, const double* partial, int nblocks, double* out, int bthreads)
+// One block per plane and sum: the plane's block partials added in a fixed order (a strided pass, then a fixed tree).
+// Eight loads in flight per thread: one at a time, each thread's run waited out an L2 latency per partial (60 us a
+// pass at 6 x 2048 x 2048, where a thread has 171 of them).
+__global__ void __launch_bounds__(256) k_objective_reduce(Planes P, const double* __restrict__ partial, int nblocks,
+                                                          double* __restrict__ out, int bthreads)
 {
     __shared__ double red[32];
-    const int pl = blockIdx.x;
+    const int pl = blockIdx.x, row = blockIdx.y;
     const long long b0 = P.start[pl] / bthreads, b1 = P.start[pl + 1] / bthreads;
-    for (int row = 0; row < 3; row++)
+    const double* p = partial + (size_t)row * nblocks;
+    double s = 0.0;
+    long long b = b0 + threadIdx.x;
+    for (; b + 7 * 256 < b1; b += 8 * 256)
     {
-        double s = 0.0;
-        for (long long b = b0 + threadIdx.x; b < b1; b += blockDim.x)
-            s += partial[(size_t)row * nblocks + b];
-        const double t = block_sum(s, red);
-        if (threadIdx.x == 0)
-            out[3 * pl + row] = t;
-        __syncthreads();
+        double v[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+            v[i] = __ldg(p + b + i * 256);
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+            s += v[i];
     }
+    for (; b < b1; b += 256)
+        s += __ldg(p + b);
+    const double t = block_sum(s, red);
+    if (threadIdx.x == 0)
+        out[3 * pl + row] = t;
 }
 
 // The recon decode at texel centres: saturate, then lroundf(acc * 255) (src/objective.cu:53-75).
@@ -677,7 +688,7 @@ int objective_sums(nntc_b200_device* d, int k, std::vector<double>& acc, double*
         }
         NB_TRY(ktimer_end(d));
         NB_LAUNCHED();
-        k_objective_reduce<<<P.n, 256, 0, d->stream>>>(P, d->obj_partial, nblocks, sums, bthreads);
+        k_objective_reduce<<<dim3(P.n, 3), 256, 0, d->stream>>>(P, d->obj_partial, nblocks, sums, bthreads);
         NB_LAUNCHED();
         NB_TRY(block_end(d, ms));
         acc.assign((size_t)3 * P.n, 0.0);
@@ -697,7 +708,7 @@ int objective_sums(nntc_b200_device* d, int k, std::vector<double>& acc, double*
     }
     NB_TRY(ktimer_end(d));
     NB_LAUNCHED();
-    k_objective_reduce<<<P.n, 256, 0, d->stream>>>(P, d->obj_partial, nblocks, sums, bthreads);
+    k_objective_reduce<<<dim3(P.n, 3), 256, 0, d->stream>>>(P, d->obj_partial, nblocks, sums, bthreads);
     NB_LAUNCHED();
     NB_TRY(block_end(d, ms));
     acc.assign((size_t)3 * P.n, 0.0);
@@ -931,7 +942,7 @@ extern "C" int nntc_b200_objective_plane_noalloc(const float* v0, int w0, int h0
     const cudaStream_t s = (cudaStream_t)stream;
     k_objective<<<nblocks, OBJ_THREADS, 0, s>>>(P, ObjArgs{ weights, bias, cw, partial });
     NB_LAUNCHED();
-    k_objective_reduce<<<1, 256, 0, s>>>(P, partial, nblocks, sums, OBJ_THREADS);
+    k_objective_reduce<<<dim3(1, 3), 256, 0, s>>>(P, partial, nblocks, sums, OBJ_THREADS);
     NB_LAUNCHED();
     return NNTC_B200_OK;
 }

@@ -15,7 +15,7 @@
 // - the stencil stored structure-of-arrays [slot][i][j][texel], coalesced for a warp of consecutive texels;
 // - the gather's 5 x nmono monomial sums live in shared memory (registers spill at C = 4);
 // - the conjugate-gradient iteration is 5 launches (matvec + <p,Ap>, alpha, update + preconditioner + <r,r> +
-//   <r,z>, beta, direction) instead of 13, all planes in lockstep, and the stop is decided ON THE DEVICE with the
+//   <r,z>, beta, direction) and nothing else instead of 13, all planes in lockstep, and the stop is decided ON THE DEVICE with the
 //   reference's rule (a plane leaves at an iteration that is a multiple of CG_PROBE once its residual is below the
 //   tolerance); the host reads one active-plane count every CG_PROBE iterations, the reference's probe cadence.
 // - every dot product is a fixed-order two-stage reduction: one partial per 256-texel block, added per plane in
@@ -338,18 +338,72 @@ __device__ __forceinline__ void block_reduce(double (&v)[N], const int (&kind)[N
         }
 }
 
-// One warp per plane: the plane's block partials of `rows` rows added in block order (strided by lane, then a tree).
-__device__ __forceinline__ double plane_total(const double* partial, size_t nblocks, long long b0, long long b1,
-                                              int row, int kind)
+// The totals of ROWS rows of one plane's block partials, on every thread of a FOLD_THREADS block. Each row is folded
+// by one warp in a fixed order - lane l adds partials l, l + 32, l + 64, ... of the plane, then the warp's tree - from
+// shared memory, where the whole block stages the rows CHUNK partials at a time, the next chunk's loads in flight
+// while this one is folded. A single warp walking the partials in global memory waited out one L2 latency per 32 of
+// them: at 6 x 2048 x 2048 (21.8 k partials) the CG's two folds took 118 and 48 us an iteration; the chain of
+// additions is now what bounds them.
+constexpr int FOLD_THREADS = 256;
+
+template <int ROWS>
+__device__ __forceinline__ void plane_totals(const double* partial, size_t nblocks, long long b0, long long b1,
+                                             const int (&row)[ROWS], const int (&kind)[ROWS], double (&out)[ROWS])
 {
-    const int lane = threadIdx.x & 31;
-    double s = kind == 0 ? 0.0 : (kind == 1 ? 1e300 : -1e300);
-    for (long long b = b0 + lane; b < b1; b += 32)
+    constexpr int PER = ROWS < 3 ? 8 : 6, CHUNK = FOLD_THREADS * PER;   // within 48 KB of shared memory
+    __shared__ double buf[ROWS][CHUNK];
+    __shared__ double total[ROWS];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const long long n = b1 - b0;
+    double v[ROWS][PER];
+    auto fetch = [&](long long at) {
+#pragma unroll
+        for (int q = 0; q < ROWS; q++)
+#pragma unroll
+            for (int i = 0; i < PER; i++)
+            {
+                const long long b = at + i * FOLD_THREADS + tid;
+                v[q][i] = b < n ? __ldg(partial + (size_t)row[q] * nblocks + (size_t)(b0 + b)) : 0.0;
+            }
+    };
+    int my_kind = 0;
+#pragma unroll
+    for (int q = 0; q < ROWS; q++)
+        my_kind = warp == q ? kind[q] : my_kind;
+    double s = my_kind == 0 ? 0.0 : (my_kind == 1 ? 1e300 : -1e300);
+    fetch(0);
+    for (long long at = 0; at < n; at += CHUNK)
     {
-        const double x = partial[(size_t)row * nblocks + b];
-        s = kind == 0 ? s + x : (kind == 1 ? fmin(s, x) : fmax(s, x));
+#pragma unroll
+        for (int q = 0; q < ROWS; q++)
+#pragma unroll
+            for (int i = 0; i < PER; i++)
+                buf[q][i * FOLD_THREADS + tid] = v[q][i];
+        __syncthreads();
+        fetch(at + CHUNK);
+        if (warp < ROWS)
+        {
+            const int left = (int)(n - at < CHUNK ? n - at : CHUNK);
+            const double* mine = buf[warp];
+#pragma unroll 8
+            for (int b = lane; b < left; b += 32)
+            {
+                const double x = mine[b];
+                s = my_kind == 0 ? s + x : (my_kind == 1 ? fmin(s, x) : fmax(s, x));
+            }
+        }
+        __syncthreads();
     }
-    return kind == 0 ? warp_sum(s) : (kind == 1 ? warp_min(s) : warp_max(s));
+    if (warp < ROWS)
+    {
+        s = my_kind == 0 ? warp_sum(s) : (my_kind == 1 ? warp_min(s) : warp_max(s));
+        if (lane == 0)
+            total[warp] = s;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < ROWS; q++)
+        out[q] = total[q];
 }
 
 struct Red
@@ -433,15 +487,15 @@ __global__ void __launch_bounds__(THREADS) k_diag(Planes P, Red R)
             R.partial[(size_t)q * R.nblocks + blockIdx.x] = v[q];
 }
 
-__global__ void k_diag_reduce(Planes P, Red R, double ridge)
+__global__ void __launch_bounds__(FOLD_THREADS) k_diag_reduce(Planes P, Red R, double ridge)
 {
     const int pl = blockIdx.x;
     const long long b0 = P.start[pl] / THREADS, b1 = P.start[pl + 1] / THREADS;
-    const double sum = plane_total(R.partial, R.nblocks, b0, b1, 0, 0);
-    const double lo = plane_total(R.partial, R.nblocks, b0, b1, 1, 1);
-    const double hi = plane_total(R.partial, R.nblocks, b0, b1, 2, 2);
+    double total[3];
+    plane_totals<3>(R.partial, R.nblocks, b0, b1, { 0, 1, 2 }, { 0, 1, 2 }, total);
     if (threadIdx.x == 0)
     {
+        const double sum = total[0], lo = total[1], hi = total[2];
         double* s = R.scalars + (size_t)pl * S_COUNT;
         const size_t unknowns = (size_t)P.p[pl].w * P.p[pl].h * P.c;
         s[S_DIAG_SUM] = sum;
@@ -626,17 +680,17 @@ __global__ void __launch_bounds__(THREADS) k_precondition_init(Planes P, Red R)
     }
 }
 
-__global__ void k_cg_start(Planes P, Red R)
+__global__ void __launch_bounds__(FOLD_THREADS) k_cg_start(Planes P, Red R)
 {
     const int pl = blockIdx.x;
     const long long b0 = P.start[pl] / THREADS, b1 = P.start[pl + 1] / THREADS;
-    const double rr = plane_total(R.partial, R.nblocks, b0, b1, 0, 0);
-    const double rz = plane_total(R.partial, R.nblocks, b0, b1, 1, 0);
+    double total[2];
+    plane_totals<2>(R.partial, R.nblocks, b0, b1, { 0, 1 }, { 0, 0 }, total);
     if (threadIdx.x == 0)
     {
         double* s = R.scalars + (size_t)pl * S_COUNT;
-        s[S_RHS2] = rr;
-        s[S_RZ] = rz;
+        s[S_RHS2] = total[0];
+        s[S_RZ] = total[1];
         s[S_ACTIVE] = 1.0;
         s[S_ITER] = 0.0;
         s[S_RESID] = 0.0;
@@ -674,16 +728,21 @@ __global__ void __launch_bounds__(THREADS) k_cg_matvec(Planes P, Red R)
         R.partial[blockIdx.x] = v[0];
 }
 
-__global__ void k_cg_alpha(Planes P, Red R)
+// alpha; block 0 also clears the count of planes that stay active, which k_cg_beta of this iteration adds up.
+__global__ void __launch_bounds__(FOLD_THREADS) k_cg_alpha(Planes P, Red R, unsigned int* active_count)
 {
     const int pl = blockIdx.x;
     double* s = R.scalars + (size_t)pl * S_COUNT;
+    if (pl == 0 && threadIdx.x == 0)
+        *active_count = 0;
     if (s[S_ACTIVE] == 0.0)
         return;
     const long long b0 = P.start[pl] / THREADS, b1 = P.start[pl + 1] / THREADS;
-    const double pap = plane_total(R.partial, R.nblocks, b0, b1, 0, 0);
+    double total[1];
+    plane_totals<1>(R.partial, R.nblocks, b0, b1, { 0 }, { 0 }, total);
     if (threadIdx.x == 0)
     {
+        const double pap = total[0];
         s[S_PAP] = pap;
         s[S_ALPHA] = pap > 0.0 ? s[S_RZ] / pap : 0.0;
     }
@@ -746,18 +805,20 @@ __global__ void __launch_bounds__(THREADS) k_cg_update(Planes P, Red R)
 }
 
 // beta, the residual, and the device-side stop: at an iteration that is a multiple of CG_PROBE a plane whose residual
-// is not at or above the tolerance leaves (the reference's host probe, src/solve_level1.cu:1288-1302).
-__global__ void k_cg_beta(Planes P, Red R, int it, unsigned int* active_count, double tol)
+// is not at or above the tolerance leaves (the reference's host probe, src/solve_level1.cu:1288-1302): its direction
+// is not updated again, which nothing reads.
+__global__ void __launch_bounds__(FOLD_THREADS) k_cg_beta(Planes P, Red R, int it, unsigned int* active_count, double tol)
 {
     const int pl = blockIdx.x;
     double* s = R.scalars + (size_t)pl * S_COUNT;
     if (s[S_ACTIVE] == 0.0)
         return;
     const long long b0 = P.start[pl] / THREADS, b1 = P.start[pl + 1] / THREADS;
-    const double rr = plane_total(R.partial, R.nblocks, b0, b1, 0, 0);
-    const double rz_new = plane_total(R.partial, R.nblocks, b0, b1, 1, 0);
+    double total[2];
+    plane_totals<2>(R.partial, R.nblocks, b0, b1, { 0, 1 }, { 0, 0 }, total);
     if (threadIdx.x == 0)
     {
+        const double rr = total[0], rz_new = total[1];
         const double rz = s[S_RZ];
         s[S_RR] = rr;
         s[S_RZ_NEW] = rz_new;
@@ -767,7 +828,7 @@ __global__ void k_cg_beta(Planes P, Red R, int it, unsigned int* active_count, d
         s[S_RESID] = rhs2 > 0.0 ? sqrt((rr > 0.0 ? rr : 0.0) / rhs2) : 0.0;
         s[S_ITER] = (double)(it + 1);
         if ((it + 1) % CG_PROBE == 0 && !(s[S_RESID] >= tol))
-            s[S_ACTIVE] = 0.5;   // leaves after this iteration's direction update (which no longer matters)
+            s[S_ACTIVE] = 0.0;
         else
             atomicAdd(active_count, 1u);
     }
@@ -791,13 +852,6 @@ __global__ void __launch_bounds__(THREADS) k_cg_direction(Planes P, Red R)
         const size_t q = (size_t)t * P.c + i;
         V.p[q] = V.z[q] + beta * V.p[q];
     }
-}
-
-__global__ void k_cg_retire(Planes P, double* scalars)
-{
-    const int pl = threadIdx.x;
-    if (pl < P.n && scalars[(size_t)pl * S_COUNT + S_ACTIVE] == 0.5)
-        scalars[(size_t)pl * S_COUNT + S_ACTIVE] = 0.0;
 }
 
 // ---- the correction and the movement probe (src/solve_level1.cu:872-979) -------------------------------------------
@@ -838,19 +892,17 @@ __global__ void __launch_bounds__(THREADS) k_correct_range(Planes P, Red R)
         }
 }
 
-__global__ void k_range_reduce(Planes P, Red R)
+// One block per plane and channel (grid.y).
+__global__ void __launch_bounds__(FOLD_THREADS) k_range_reduce(Planes P, Red R)
 {
-    const int pl = blockIdx.x;
+    const int pl = blockIdx.x, q = blockIdx.y;
     const long long b0 = P.start[pl] / THREADS, b1 = P.start[pl + 1] / THREADS;
-    for (int q = 0; q < P.c; q++)
+    double total[2];
+    plane_totals<2>(R.partial, R.nblocks, b0, b1, { 3 + q, 3 + MAX_CH + q }, { 1, 2 }, total);
+    if (threadIdx.x == 0)
     {
-        const double lo = plane_total(R.partial, R.nblocks, b0, b1, 3 + q, 1);
-        const double hi = plane_total(R.partial, R.nblocks, b0, b1, 3 + MAX_CH + q, 2);
-        if (threadIdx.x == 0)
-        {
-            R.scalars[(size_t)pl * S_COUNT + S_LO + q] = lo;
-            R.scalars[(size_t)pl * S_COUNT + S_HI + q] = hi;
-        }
+        R.scalars[(size_t)pl * S_COUNT + S_LO + q] = total[0];
+        R.scalars[(size_t)pl * S_COUNT + S_HI + q] = total[1];
     }
 }
 
@@ -883,19 +935,18 @@ __global__ void __launch_bounds__(THREADS) k_movement(Planes P, Red R, int level
             R.partial[(size_t)q * R.nblocks + blockIdx.x] = v[q];
 }
 
-__global__ void k_movement_reduce(Planes P, Red R)
+__global__ void __launch_bounds__(FOLD_THREADS) k_movement_reduce(Planes P, Red R)
 {
     const int pl = blockIdx.x;
     const long long b0 = P.start[pl] / THREADS, b1 = P.start[pl + 1] / THREADS;
-    const double moved = plane_total(R.partial, R.nblocks, b0, b1, 0, 0);
-    const double d2 = plane_total(R.partial, R.nblocks, b0, b1, 1, 0);
-    const double p2 = plane_total(R.partial, R.nblocks, b0, b1, 2, 0);
+    double total[3];
+    plane_totals<3>(R.partial, R.nblocks, b0, b1, { 0, 1, 2 }, { 0, 0, 0 }, total);
     if (threadIdx.x == 0)
     {
         double* s = R.scalars + (size_t)pl * S_COUNT;
-        s[S_MOVED] = moved;
-        s[S_DELTA2] = d2;
-        s[S_PLANE2] = p2;
+        s[S_MOVED] = total[0];
+        s[S_DELTA2] = total[1];
+        s[S_PLANE2] = total[2];
     }
 }
 
@@ -1075,7 +1126,7 @@ int assemble(nntc_b200_device* d, const nntc_b200_model* m, int k, double ridge,
     else
         k_diag<double><<<tblocks, THREADS, 0, d->stream>>>(P, R);
     NB_LAUNCHED();
-    k_diag_reduce<<<P.n, 32, 0, d->stream>>>(P, R, ridge);
+    k_diag_reduce<<<P.n, FOLD_THREADS, 0, d->stream>>>(P, R, ridge);
     NB_LAUNCHED();
     return NNTC_B200_OK;
 }
@@ -1117,13 +1168,12 @@ int solve_block(nntc_b200_device* d, const nntc_b200_model* m, int k, double rid
     else
         k_precondition_init<double><<<tblocks, THREADS, 0, d->stream>>>(P, R);
     NB_LAUNCHED();
-    k_cg_start<<<P.n, 32, 0, d->stream>>>(P, R);
+    k_cg_start<<<P.n, FOLD_THREADS, 0, d->stream>>>(P, R);
     NB_LAUNCHED();
     NB_CUDA(cudaEventRecord(d->ev[3], d->stream));
     unsigned int* active = d->counters + CNT_ACTIVE;
     for (int it = 0; it < CG_MAX_IT; it++)
     {
-        NB_CUDA(cudaMemsetAsync(active + (it % CG_PROBE), 0, sizeof(unsigned int), d->stream));
         NB_TRY(ktimer_begin(d, level0 ? NNTC_B200_K_MATVEC0 : NNTC_B200_K_MATVEC));
         if (adjoint)
             NB_TRY(matvec_free(d, P, R.partial, level0));
@@ -1149,7 +1199,7 @@ int solve_block(nntc_b200_device* d, const nntc_b200_model* m, int k, double rid
             NB_LAUNCHED();
         }
         NB_TRY(ktimer_end(d));
-        k_cg_alpha<<<P.n, 32, 0, d->stream>>>(P, R);
+        k_cg_alpha<<<P.n, FOLD_THREADS, 0, d->stream>>>(P, R, active + (it % CG_PROBE));
         NB_LAUNCHED();
         switch (P.c)
         {
@@ -1159,12 +1209,10 @@ int solve_block(nntc_b200_device* d, const nntc_b200_model* m, int k, double rid
         default: k_cg_update<4><<<tblocks, THREADS, 0, d->stream>>>(P, R); break;
         }
         NB_LAUNCHED();
-        k_cg_beta<<<P.n, 32, 0, d->stream>>>(P, R, it, active + (it % CG_PROBE),
+        k_cg_beta<<<P.n, FOLD_THREADS, 0, d->stream>>>(P, R, it, active + (it % CG_PROBE),
                                              adjoint || d->sten_f32[level0] ? CG_TOL_FP32 : CG_TOL);
         NB_LAUNCHED();
         k_cg_direction<<<tblocks, THREADS, 0, d->stream>>>(P, R);
-        NB_LAUNCHED();
-        k_cg_retire<<<1, 32, 0, d->stream>>>(P, d->scalars);
         NB_LAUNCHED();
         if ((it + 1) % CG_PROBE != 0)
             continue;
@@ -1177,12 +1225,12 @@ int solve_block(nntc_b200_device* d, const nntc_b200_model* m, int k, double rid
     }
     k_correct_range<<<tblocks, THREADS, 0, d->stream>>>(P, R);
     NB_LAUNCHED();
-    k_range_reduce<<<P.n, 32, 0, d->stream>>>(P, R);
+    k_range_reduce<<<dim3(P.n, P.c), FOLD_THREADS, 0, d->stream>>>(P, R);
     NB_LAUNCHED();
     const int levels = level0 ? 255 : (1 << m->bits1) - 1;
     k_movement<<<tblocks, THREADS, 0, d->stream>>>(P, R, levels);
     NB_LAUNCHED();
-    k_movement_reduce<<<P.n, 32, 0, d->stream>>>(P, R);
+    k_movement_reduce<<<P.n, FOLD_THREADS, 0, d->stream>>>(P, R);
     NB_LAUNCHED();
     NB_CUDA(cudaMemcpyAsync(d->host_scalars, d->scalars, (size_t)np * S_COUNT * sizeof(double),
                             cudaMemcpyDeviceToHost, d->stream));
