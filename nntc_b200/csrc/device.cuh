@@ -47,7 +47,7 @@ enum Scalar
 constexpr int RGRID = 148 * 4;
 constexpr int RROWS = 3 + 2 * MAX_CH;
 constexpr int THREADS = 256;
-constexpr int GATHER_TABLE_MAX = 8192;   // int4 entries of one visit table
+constexpr int GATHER_TABLE_MAX = 8192;   // int4 entries of one visit table (one for FP64 and one for FP32 sums)
 constexpr int LS_GRID = 148 * 4;         // normal equations: blocks per plane (four per SM at the base plane)
 constexpr int COV_GRID = 512;            // init covariance: partials per entry
 constexpr int HIST_BINS = 4096;          // init0: the percentile histogram
@@ -134,9 +134,9 @@ struct nntc_b200_device
     int site_tgt_kc = -1;                // the K site_tgt holds (-1: none yet; the source never changes)
     double* obj_tgt = nullptr;           // the fractional sites' double targets at K, nout per site (objective)
     int obj_tgt_kc = -1;                 // the K obj_tgt holds (-1: none yet)
-    void* gtab[2] = { nullptr, nullptr };// the gather's visit tables of level 1 / level 0 (GATHER_TABLE_MAX int4 each)
+    void* gtab[2] = { nullptr, nullptr };// the gather's visit tables of level 1 / level 0 (2 GATHER_TABLE_MAX int4 each)
     int gtab_kc[2] = { -1, -1 };         // the K each table was built for (-1: none yet)
-    int gtab_off[2][4][6] = {};          // each table's entry ranges per parity class and slot
+    int gtab_off[2][25][6] = {};         // each table's entry ranges per class (gather.cuh) and slot
     int reference_shaped_assembly = 0;   // 1: the per-texel gather of the reference's shape (same bits, slower)
     int mixed_gram = 0;                  // 1: block (a)'s sums on the tensor cores, BF16 hi + lo (gram_tc.cu)
     int bc_copy = 0;                     // 1 while the assembly for the BC refinement runs: also write bc_sten
