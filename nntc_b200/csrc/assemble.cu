@@ -15,8 +15,8 @@
 //   - the stencil's monomial sums need only the site's sample of the OTHER latent (a bilinear blend of four texels,
 //     which k_site_terms also stores per site) and the tap weights - a few dozen operations. They are gathered per
 //     (texel, slot): each slot's sums receive the same terms in the same site order as the reference's, so every sum,
-//     and the expansion against the monomial matrices after it, is the same bits. gather.cu gathers the planes whose
-//     visits are tabled; k_gather_walk below the others.
+//     and the expansion against the monomial matrices after it, is the same bits. gather.cu does it in tiles; k_gather_walk below
+//     takes the few planes no tile fits.
 //
 // Every plane of the chain is in each launch (nb::Planes); the per-site buffer holds every plane's sites.
 
@@ -311,8 +311,8 @@ __device__ __forceinline__ void stencil_texel(long long pos, int w, int h, int& 
     y = 2 * (int)(r / rw) + cy;
 }
 
-// The gather of a plane whose visits are not tabled (level 1 at any other ratio than a quarter of a power-of-two plane,
-// and planes one texel wide or high): one thread per (texel, slot) tests every site of the two texels' common
+// The gather of the planes no tile takes (planes one texel wide or high at level 0, level-1 planes whose tile would not
+// fit shared memory): one thread per (texel, slot) tests every site of the two texels' common
 // footprint, in site order; the self-slot thread also gathers the gradient. Blocks run in (region, colour, slot) order,
 // the slot fastest, so that the five slots of one run of texels and the four colours of one region run side by side
 // and share the region's sites in L2.
@@ -428,7 +428,7 @@ static int launch_walk(nntc_b200_device* d, int level0, const Planes& P, const T
     return NNTC_B200_OK;
 }
 
-// The gather of every plane: the tiled planes in one launch, the others in another.
+// The gather of every plane: the tabled planes in one launch, the others in one or two more.
 template <typename TS>
 static int gather_planes(nntc_b200_device* d, int level0, const Planes& P, int nmono, const double* mono, int slots)
 {
@@ -479,6 +479,25 @@ static int gather_planes(nntc_b200_device* d, int level0, const Planes& P, int n
     A.tab = (const int4*)d->gtab[level0] + (sizeof(TS) == sizeof(double) ? 0 : GATHER_TABLE_MAX);
     std::memcpy(A.off, d->gtab_off[level0], sizeof(A.off));
     auto pow2 = [](int v) { return v > 0 && (v & (v - 1)) == 0; };
+    // A level-1 plane that is not tabled goes to k_gather_any1 in tiles of the same texels, wherever a tile's sites fit
+    // shared memory: three tiles to an SM while its pixels are about four a texel (up to ANY_SHARED bytes), else, on
+    // the deep planes of an odd chain, as many as fit (up to ANY_SHARED_MAX) - in a launch of their own when the others
+    // would lose their three for it, in the same launch when there are too few tiles for that to matter.
+    constexpr size_t ANY_SHARED = 73 * 1024, ANY_SHARED_MAX = 200 * 1024;
+    constexpr int ANY_FEW = 2 * 148;
+    AnyTiles R{};
+    size_t any_bytes[MAX_PLANES] = {};
+    auto widest = [](int n, int n0, int tile) {
+        int most = 0;
+        for (int t = 0; t < n; t += tile)
+        {
+            int lo, hi, other;
+            reach(t, n0, n, lo, other);
+            reach(std::min(t + tile, n) - 1, n0, n, other, hi);
+            most = std::max(most, hi - lo + 1);
+        }
+        return most;
+    };
     WalkBlocks B{};
     long long at = 0, walk = 0;
     for (int i = 0; i < P.n; i++)
@@ -490,9 +509,17 @@ static int gather_planes(nntc_b200_device* d, int level0, const Planes& P, int n
         at += (long long)v.w0 * v.h0 * (1 + k);
         const int tw = level0 ? TILE0_W : TILE1_W, th = level0 ? TILE0_H : TILE1_H;
         A.btiles[i] = tiled ? ((v.w + tw - 1) / tw) * ((v.h + th - 1) / th) : 0;
+        if (!tiled && !level0)
+        {
+            R.px[i] = widest(v.w, v.w0, TILE1_W);
+            R.py[i] = widest(v.h, v.h0, TILE1_H);
+            const size_t bytes = any_tile_bytes(R.px[i], R.py[i], 1 + k);
+            any_bytes[i] = bytes <= ANY_SHARED_MAX && R.px[i] * (1 + k) < 1024 ? bytes : 0;
+        }
+        const bool walked = !tiled && any_bytes[i] == 0;
         B.start[i] = walk;
         const long long largest = (long long)((v.w + 1) / 2) * ((v.h + 1) / 2);   // colour 0
-        walk += tiled ? 0 : (largest + WALK_THREADS - 1) / WALK_THREADS * 4 * slots;
+        walk += walked ? (largest + WALK_THREADS - 1) / WALK_THREADS * 4 * slots : 0;
     }
     A.site0[P.n] = at;
     B.start[P.n] = walk;
@@ -501,6 +528,26 @@ static int gather_planes(nntc_b200_device* d, int level0, const Planes& P, int n
         A.bend[i] = tiles += A.btiles[i];
     if (walk > 0)
         NB_TRY(launch_walk<TS>(d, level0, P, A, B));
+    int any_tiles = 0;
+    for (int i = 0; i < P.n; i++)
+        any_tiles += any_bytes[i] ? ((P.p[i].w + TILE1_W - 1) / TILE1_W) * ((P.p[i].h + TILE1_H - 1) / TILE1_H) : 0;
+    for (int group = 0; group < 2 && any_tiles > 0; group++)   // the larger tiles, then the others
+    {
+        TileArgs<TS> G = A;
+        size_t shared = 0;
+        int blocks = 0;
+        for (int i = P.n - 1; i >= 0; i--)
+        {
+            const bool large = any_bytes[i] > ANY_SHARED || any_tiles <= ANY_FEW;
+            G.btiles[i] = any_bytes[i] && large == (group == 0)
+                              ? ((P.p[i].w + TILE1_W - 1) / TILE1_W) * ((P.p[i].h + TILE1_H - 1) / TILE1_H)
+                              : 0;
+            shared = G.btiles[i] ? std::max(shared, any_bytes[i]) : shared;
+            G.bend[i] = blocks += G.btiles[i];
+        }
+        if (blocks > 0)
+            NB_TRY(launch_gather_any(d, P, G, R, (unsigned)blocks, shared));
+    }
     if (tiles > 0)
         NB_TRY(launch_gather_tiles(d, level0, P, A, (unsigned)tiles));
     return NNTC_B200_OK;

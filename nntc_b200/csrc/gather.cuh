@@ -245,6 +245,30 @@ __device__ __forceinline__ void visit_sums(TS (&sums)[MAX_MONO], const float4& y
     }
 }
 
+// Level 1 planes whose visits are not tabled, in tiles of the same texels (k_gather_any1): the pixels a tile's texels
+// can meet on each axis, at most, per plane.
+struct AnyTiles
+{
+    int px[MAX_PLANES], py[MAX_PLANES];
+};
+
+// The entries of n pixel columns' (or rows') taps, one of padding after every four.
+__host__ __device__ inline int any_taps(int n, int per)
+{
+    return n * per * 2 + (n + 3) / 4;
+}
+
+// Shared memory of one such tile: every site's sample, then each pixel column's and row's taps.
+inline size_t any_tile_bytes(int px, int py, int per)
+{
+    return (size_t)((px + 3) / 4 * 4) * py * per * sizeof(float4) +
+           (size_t)(any_taps(px, per) + any_taps(py, per)) * 16;
+}
+
+int launch_gather_any(nntc_b200_device* d, const Planes& P, const TileArgs<double>& A, const AnyTiles& S,
+                      unsigned grid, size_t shared);
+int launch_gather_any(nntc_b200_device* d, const Planes& P, const TileArgs<float>& A, const AnyTiles& S, unsigned grid,
+                      size_t shared);
 int launch_gather_tiles(nntc_b200_device* d, int level0, const Planes& P, const TileArgs<double>& A, unsigned grid);
 int launch_gather_tiles(nntc_b200_device* d, int level0, const Planes& P, const TileArgs<float>& A, unsigned grid);
 
