@@ -105,6 +105,24 @@ __host__ __device__ __forceinline__ Tap tap_at(int px, int py, float dx, float d
     return t;
 }
 
+// tap_at where the caller knows the exact reciprocals of w0 and h0 (powers of two; 0 where one is not): the same bits.
+__device__ __forceinline__ Tap tap_scaled(int px, int py, float dx, float dy, int w0, int h0, int w, int h, float inv_w,
+                                          float inv_h)
+{
+    const float nx = ((float)px + 0.5f + dx) * (float)w, ny = ((float)py + 0.5f + dy) * (float)h;
+    const float x = w == w0 ? (float)px + dx : (inv_w > 0.0f ? nx * inv_w : nx / (float)w0) - 0.5f;
+    const float y = h == h0 ? (float)py + dy : (inv_h > 0.0f ? ny * inv_h : ny / (float)h0) - 0.5f;
+    const int xf = (int)floorf(x), yf = (int)floorf(y);
+    Tap t;
+    t.fx = x - (float)xf;
+    t.fy = y - (float)yf;
+    t.x0 = clampi(xf, w);
+    t.x1 = clampi(xf + 1, w);
+    t.y0 = clampi(yf, h);
+    t.y1 = clampi(yf + 1, h);
+    return t;
+}
+
 // The four corner weights in the order (x0,y0), (x1,y0), (x0,y1), (x1,y1).
 __host__ __device__ __forceinline__ void tap_weights(const Tap& t, float w[4])
 {
@@ -141,6 +159,48 @@ __device__ __forceinline__ void blend_u(const float* plane, int w, int c, const 
     for (int k = 0; k < MAXC; k++)
         if (k < c)
             out[k] = wt[0] * __ldg(a + k) + wt[1] * __ldg(b + k) + wt[2] * __ldg(e + k) + wt[3] * __ldg(f + k);
+}
+
+// blend_u with the channel count a constant: a tap's channels are one vector load where their size allows it.
+template <int C>
+__device__ __forceinline__ void load_channels(const float* p, float* out)
+{
+    if constexpr (C == 4)
+    {
+        const float4 v = __ldg(reinterpret_cast<const float4*>(p));
+        out[0] = v.x;
+        out[1] = v.y;
+        out[2] = v.z;
+        out[3] = v.w;
+    }
+    else if constexpr (C == 2)
+    {
+        const float2 v = __ldg(reinterpret_cast<const float2*>(p));
+        out[0] = v.x;
+        out[1] = v.y;
+    }
+    else
+    {
+#pragma unroll
+        for (int k = 0; k < C; k++)
+            out[k] = __ldg(p + k);
+    }
+}
+
+template <int C>
+__device__ __forceinline__ void blend_c(const float* plane, int w, const Tap& t, float* out)
+{
+    float a[C], b[C], e[C], f[C], wt[4];
+    // (a plane's floats are far below 2^32: 32-bit offsets)
+    const unsigned r0 = (unsigned)t.y0 * (unsigned)w, r1 = (unsigned)t.y1 * (unsigned)w;
+    load_channels<C>(plane + (r0 + (unsigned)t.x0) * C, a);
+    load_channels<C>(plane + (r0 + (unsigned)t.x1) * C, b);
+    load_channels<C>(plane + (r1 + (unsigned)t.x0) * C, e);
+    load_channels<C>(plane + (r1 + (unsigned)t.x1) * C, f);
+    tap_weights(t, wt);
+#pragma unroll
+    for (int k = 0; k < C; k++)
+        out[k] = wt[0] * a[k] + wt[1] * b[k] + wt[2] * e[k] + wt[3] * f[k];
 }
 
 // phi in the shader's order: [c_j] [s_i] [s_i c_j], i outer (src/sample.cuh:74-85).
@@ -185,6 +245,19 @@ __host__ __device__ __forceinline__ void subtexel(int kc, int j, int tx, int ty,
     }
     dx = ox;
     dy = oy;
+}
+
+// The same without a loop over the turns (selections of signs and places alone: the same offsets), for the kernels whose
+// time it is; where a kernel's site loop was left rolled because of that loop, unrolling it costs more than it saves.
+__device__ __forceinline__ void subtexel_turned(int kc, int j, int tx, int ty, float& dx, float& dy)
+{
+    subtexel(kc, j, 0, 0, dx, dy);
+    if (kc == 2)
+        return;
+    // a quarter turn is (x, y) -> (-y, x): one when tx is odd, two when ty is
+    const float ax = (tx & 1) ? -dy : dx, ay = (tx & 1) ? dx : dy;
+    dx = (ty & 1) ? -ax : ax;
+    dy = (ty & 1) ? -ay : ay;
 }
 
 // Site j of a pixel: 0 the centre, 1..K the fractional sites.
