@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "device.cuh"
+#include "row_stage.cuh"
 
 namespace nb
 {
@@ -341,6 +342,162 @@ __global__ void __launch_bounds__(OBJ_P_THREADS, 5)
                 else
                     fractional = fma(e, e, fractional);
             }
+        }
+    }
+    const double a = block_sum(weighted, red);
+    const double b = block_sum(centre, red);
+    const double c = block_sum(fractional, red);
+    if (threadIdx.x == 0)
+    {
+        const size_t nb = gridDim.x;
+        partial[blockIdx.x] = a;
+        partial[nb + blockIdx.x] = b;
+        partial[2 * nb + blockIdx.x] = c;
+    }
+}
+
+// obj_sample with a constant channel count (vector loads) and, for a power-of-two plane, the caller's division by its
+// extent done as the exact product: the same bits.
+template <int C>
+__device__ __forceinline__ void obj_sample_c(const float* plane, int w, int h, double u, double v, double* out)
+{
+    const double x = u * (double)w - 0.5, y = v * (double)h - 0.5;
+    const double xf = floor(x), yf = floor(y);
+    const double fx = x - xf, fy = y - yf;
+    const int x0 = clampi((int)xf, w), x1 = clampi((int)xf + 1, w);
+    const int y0 = clampi((int)yf, h), y1 = clampi((int)yf + 1, h);
+    float a[C], b[C], e[C], f[C];
+    const unsigned r0 = (unsigned)y0 * (unsigned)w, r1 = (unsigned)y1 * (unsigned)w;
+    load_channels<C>(plane + (r0 + (unsigned)x0) * C, a);
+    load_channels<C>(plane + (r0 + (unsigned)x1) * C, b);
+    load_channels<C>(plane + (r1 + (unsigned)x0) * C, e);
+    load_channels<C>(plane + (r1 + (unsigned)x1) * C, f);
+    const double w00 = (1.0 - fx) * (1.0 - fy), w10 = fx * (1.0 - fy), w01 = (1.0 - fx) * fy, w11 = fx * fy;
+#pragma unroll
+    for (int k = 0; k < C; k++)
+        out[k] = w00 * (double)a[k] + w10 * (double)b[k] + w01 * (double)e[k] + w11 * (double)f[k];
+}
+
+__device__ __forceinline__ void obj_sample_any(const float* plane, int w, int h, int c, double u, double v, double* out)
+{
+    if (c == 4)
+        obj_sample_c<4>(plane, w, h, u, v, out);
+    else if (c == 2)
+        obj_sample_c<2>(plane, w, h, u, v, out);
+    else
+        obj_sample<MAX_CH>(plane, w, h, c, u, v, out);
+}
+
+// k_objective_p with the targets of the next site on their way to shared memory while this one is decoded
+// (row_stage.cuh) and the features that the channel counts do not have skipped (their weights are zero). Bound by issue
+// and the FP64 pipe (about 600 operations a site): 1857 -> 1739 us at 6 x 2048 x 2048, 772 -> 630 us at 4 x 2048 x 1024.
+// With rows of one or two textures (24 or 48 bytes) the lanes' own loads are the cheaper way (163 against 201 us at 1 x
+// 1000 x 1000), and those materials keep k_objective_p.
+template <int NOUT>
+__global__ void __launch_bounds__(OBJ_P_THREADS, 5)
+    k_objective_staged(Planes P, const __grid_constant__ ObjDecoder W, double* partial, const __grid_constant__ ObjTargets T)
+{
+    using Rows = RowShape<NOUT, double>;
+    __shared__ __align__(16) char staged[2][OBJ_P_THREADS / 32][32 * Rows::STRIDE];
+    __shared__ double red[32];
+    const int c0 = P.c0, c1 = P.c1, kc = P.kc;
+    const long long base = (long long)blockIdx.x * blockDim.x;
+    const int pl = plane_of(P, base);
+    const PlaneView& V = P.p[pl];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const long long pixels = (long long)V.w0 * V.h0;
+    const long long first = base - P.start[pl] + warp * 32, local = first + lane;   // the warp's first pixel, this lane's
+    double weighted = 0.0, centre = 0.0, fractional = 0.0;
+    if (first < pixels)
+    {
+        const int rows = (int)(pixels - first < 32 ? pixels - first : 32);
+        const double* tf = T.t + (size_t)(T.site0[pl] + first * kc) * NOUT;
+        const double inv_w = (V.w0 & (V.w0 - 1)) == 0 ? 1.0 / (double)V.w0 : 0.0;
+        const double inv_h = (V.h0 & (V.h0 - 1)) == 0 ? 1.0 / (double)V.h0 : 0.0;
+        const int at = (int)(local < pixels ? local : pixels - 1), px = at % V.w0, py = at / V.w0;
+        stage_rows<NOUT, float>(staged[0][warp], V.src + (size_t)first * NOUT, NOUT, rows, lane);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+#pragma unroll 1
+        for (int j = 0; j <= kc; j++)
+        {
+            if (j < kc)
+                stage_rows<NOUT, double>(staged[(j + 1) & 1][warp], tf + (size_t)j * NOUT, kc * NOUT, rows, lane);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            float dx = 0.0f, dy = 0.0f;
+            if (j > 0)
+                subtexel_turned(kc, j - 1, px, py, dx, dy);
+            const double nu = (double)px + 0.5 + (double)dx, nv = (double)py + 0.5 + (double)dy;
+            const double u = inv_w > 0.0 ? nu * inv_w : nu / (double)V.w0;
+            const double v = inv_h > 0.0 ? nv * inv_h : nv / (double)V.h0;
+            double s[MAX_CH] = { 0.0, 0.0, 0.0, 0.0 }, c[MAX_CH] = { 0.0, 0.0, 0.0, 0.0 };
+            obj_sample_any(V.v1, V.w1, V.h1, c1, u, v, c);
+            if (j == 0)
+            {
+#pragma unroll
+                for (int i = 0; i < MAX_CH; i++)
+                    if (i < c0)
+                        s[i] = (double)V.v0[(size_t)at * c0 + i];
+            }
+            else
+                obj_sample_any(V.v0, V.w0, V.h0, c0, u, v, s);
+            // every row's dot product advanced together, feature by feature (each row's own sum keeps phi's order),
+            // so that NOUT independent chains of DFMAs are in flight at once; a product feature s_i c_q is formed
+            // once, when its turn comes, instead of being held for the whole site
+            double acc[NOUT];
+#pragma unroll
+            for (int r = 0; r < NOUT; r++)
+                acc[r] = W.b[r];
+#pragma unroll
+            for (int h = 0; h < 4; h++)
+                if (h < c1)
+                {
+#pragma unroll
+                    for (int r = 0; r < NOUT; r++)
+                        acc[r] = fma(W.w[r * 24 + h], c[h], acc[r]);
+                }
+#pragma unroll
+            for (int h = 0; h < 4; h++)
+                if (h < c0)
+                {
+#pragma unroll
+                    for (int r = 0; r < NOUT; r++)
+                        acc[r] = fma(W.w[r * 24 + 4 + h], s[h], acc[r]);
+                }
+#pragma unroll
+            for (int h = 0; h < 16; h++)
+                if (h / 4 < c0 && h % 4 < c1)
+                {
+                    const double sc = s[h / 4] * c[h % 4];
+#pragma unroll
+                    for (int r = 0; r < NOUT; r++)
+                        acc[r] = fma(W.w[r * 24 + 8 + h], sc, acc[r]);
+                }
+            asm volatile("cp.async.wait_group 1;" ::: "memory");   // this site's rows; the next one's stay in flight
+            __syncwarp();
+            // the pixel's own source at the centre site, else the fractional site's sample from k_objective_targets
+            auto add = [&](auto zero) {
+                using TT = decltype(zero);
+                TT t[NOUT];
+                read_row<NOUT, TT>(staged[j & 1][warp], lane, t);
+#pragma unroll
+                for (int r = 0; r < NOUT; r++)
+                {
+                    const double e = acc[r] - (double)t[r];
+                    weighted = fma(W.cw[r] * e, e, weighted);
+                    if (sizeof(TT) == sizeof(float))
+                        centre = fma(e, e, centre);
+                    else
+                        fractional = fma(e, e, fractional);
+                }
+            };
+            if (local < pixels)
+            {
+                if (j == 0)
+                    add(0.0f);
+                else
+                    add(0.0);
+            }
+            __syncwarp();   // the buffer is read before the copies of the site after next
         }
     }
     const double a = block_sum(weighted, red);
@@ -699,10 +856,10 @@ int objective_sums(nntc_b200_device* d, int k, std::vector<double>& acc, double*
     {
     case 3: k_objective_p<3><<<nblocks, OBJ_P_THREADS, 0, d->stream>>>(P, W, d->obj_partial, T); break;
     case 6: k_objective_p<6><<<nblocks, OBJ_P_THREADS, 0, d->stream>>>(P, W, d->obj_partial, T); break;
-    case 9: k_objective_p<9><<<nblocks, OBJ_P_THREADS, 0, d->stream>>>(P, W, d->obj_partial, T); break;
-    case 12: k_objective_p<12><<<nblocks, OBJ_P_THREADS, 0, d->stream>>>(P, W, d->obj_partial, T); break;
-    case 15: k_objective_p<15><<<nblocks, OBJ_P_THREADS, 0, d->stream>>>(P, W, d->obj_partial, T); break;
-    case 18: k_objective_p<18><<<nblocks, OBJ_P_THREADS, 0, d->stream>>>(P, W, d->obj_partial, T); break;
+    case 9: k_objective_staged<9><<<nblocks, OBJ_P_THREADS, 0, d->stream>>>(P, W, d->obj_partial, T); break;
+    case 12: k_objective_staged<12><<<nblocks, OBJ_P_THREADS, 0, d->stream>>>(P, W, d->obj_partial, T); break;
+    case 15: k_objective_staged<15><<<nblocks, OBJ_P_THREADS, 0, d->stream>>>(P, W, d->obj_partial, T); break;
+    case 18: k_objective_staged<18><<<nblocks, OBJ_P_THREADS, 0, d->stream>>>(P, W, d->obj_partial, T); break;
     default:
         k_objective<<<nblocks, OBJ_THREADS, 0, d->stream>>>(P, ObjArgs{ d->weights, d->bias, d->cw, d->obj_partial });
     }
