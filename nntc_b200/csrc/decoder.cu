@@ -54,6 +54,12 @@ constexpr int NE_STRIDE = 57;    // floats per staged site: 48 columns; an odd s
 constexpr int NE_TILES = 18;     // block pairs I <= J of six blocks with I <= 3: the rows a < 32 the system reads
                                  // (pairs of two target blocks are never needed)
 
+// After the staged rows (and the warps' tiles, which take their place): each warp's 32 target rows.
+constexpr size_t NE_TILE_BYTES = (size_t)NE_WARPS * NE_TILES * 64 * sizeof(double);
+constexpr size_t NE_STAGE_BYTES = (size_t)NE_THREADS * NE_STRIDE * sizeof(float);
+constexpr size_t NE_ROWS_OFFSET = ((NE_TILE_BYTES > NE_STAGE_BYTES ? NE_TILE_BYTES : NE_STAGE_BYTES) + 15) / 16 * 16;
+constexpr size_t NE_SHARED = NE_ROWS_OFFSET + (size_t)NE_THREADS * RowShape<MAX_NOUT, float>::STRIDE;
+
 __device__ __forceinline__ void dmma_8x8x4(double& d0, double& d1, double a, double b)
 {
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
@@ -90,6 +96,17 @@ __global__ void __launch_bounds__(NE_THREADS, 4) k_ls_accumulate_mma(Planes P, c
         acc[t][1] = 0.0;
     }
 
+    if ((long long)blockIdx.x >= chunks)
+    {
+        // no texels left for this block: its partials are zero
+        for (int e = tid; e < A.entries; e += NE_THREADS)
+            A.partial[((size_t)pl * A.entries + e) * LS_GRID + blockIdx.x] = 0.0;
+        return;
+    }
+    // the targets of this warp's next 32 sites are on their way while it multiplies the current ones
+    char* target_rows = reinterpret_cast<char*>(ne_sh) + NE_ROWS_OFFSET + warp * 32 * RowShape<NOUT, float>::STRIDE;
+    stage_targets<NOUT>(target_rows, V, tgt, kc, (long long)blockIdx.x * NE_THREADS + warp * 32, texels, 0, lane);
+    const bool wide = P.c0 > 2;   // slots 16..23, the products of channels two and three, are in use
     for (long long chunk = blockIdx.x; chunk < chunks; chunk += gridDim.x)
     {
         const long long pixel = chunk * NE_THREADS + tid;
@@ -98,8 +115,15 @@ __global__ void __launch_bounds__(NE_THREADS, 4) k_ls_accumulate_mma(Planes P, c
         for (int j = 0; j <= kc; j++)
         {
             float z[ZS_WIDTH];
+            float t[NOUT];
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncwarp();
+            read_row<NOUT, float>(target_rows, lane, t);
+            __syncwarp();
+            const long long next = j < kc ? chunk : chunk + gridDim.x;
+            stage_targets<NOUT>(target_rows, V, tgt, kc, next * NE_THREADS + warp * 32, texels, j < kc ? j + 1 : 0, lane);
             if (valid)
-                site_z<NOUT>(P, V, tgt, pixel, px, py, j, z);
+                site_z_staged<NOUT>(P, V, t, pixel, px, py, j, z);
             else
             {
 #pragma unroll
@@ -121,10 +145,19 @@ __global__ void __launch_bounds__(NE_THREADS, 4) k_ls_accumulate_mma(Planes P, c
                 double frag[6];
 #pragma unroll
                 for (int b = 0; b < 6; b++)
-                    frag[b] = (double)f[8 * b];
+                    if (8 * b < ZS_T + NOUT)
+                        frag[b] = (double)f[8 * b];
 #pragma unroll
                 for (int t = 0; t < NE_TILES; t++)
-                    dmma_8x8x4(acc[t][0], acc[t][1], frag[tile_i(t)], frag[tile_j(t)]);
+                    if (8 * tile_j(t) < ZS_T + NOUT && tile_i(t) != 2 && tile_j(t) != 2)
+                        dmma_8x8x4(acc[t][0], acc[t][1], frag[tile_i(t)], frag[tile_j(t)]);
+                if (wide)
+                {
+#pragma unroll
+                    for (int t = 0; t < NE_TILES; t++)
+                        if (8 * tile_j(t) < ZS_T + NOUT && (tile_i(t) == 2 || tile_j(t) == 2))
+                            dmma_8x8x4(acc[t][0], acc[t][1], frag[tile_i(t)], frag[tile_j(t)]);
+                }
             }
         }
     }
@@ -260,8 +293,7 @@ int normal_equations(nntc_b200_device* d, int k, const double* per_site, double*
     }
     else
     {
-        const size_t shared = std::max((size_t)NE_THREADS * NE_STRIDE * sizeof(float),
-                                       (size_t)NE_WARPS * NE_TILES * 64 * sizeof(double));
+        const size_t shared = NE_SHARED;
         NB_TRY(ktimer_begin(d, NNTC_B200_K_NORMAL_EQ));
 #define NB_NE(NO)                                                                                                     \
     case NO:                                                                                                          \

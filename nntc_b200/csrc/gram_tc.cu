@@ -72,7 +72,9 @@ constexpr uint32_t TG_WAIT_LIMIT = 1u << 26;
 // shared memory is at least this long.
 constexpr uint32_t TG_MAX_STRIDE = TG_MN > TG_KG ? TG_MN : TG_KG;
 constexpr uint32_t TG_REACH = (TG_BUFFERS - 1) * TG_BUF + (TG_KSTEPS - 1) * TG_STEP + 16 * TG_MAX_STRIDE + 16;
-constexpr uint32_t TG_SHARED = TG_ACC_OFFSET + TG_ACC_BYTES > TG_REACH ? TG_ACC_OFFSET + TG_ACC_BYTES : TG_REACH;
+constexpr uint32_t TG_ROWS_OFFSET = (TG_ACC_OFFSET + TG_ACC_BYTES + 15) / 16 * 16;   // each warp's 32 staged target rows
+constexpr uint32_t TG_ROWS_BYTES = TG_THREADS * RowShape<MAX_NOUT, float>::STRIDE;
+constexpr uint32_t TG_SHARED = TG_ROWS_OFFSET + TG_ROWS_BYTES > TG_REACH ? TG_ROWS_OFFSET + TG_ROWS_BYTES : TG_REACH;
 static_assert(TG_SHARED <= 56 * 1024, "four CTAs per SM");
 static_assert(TG_ACC_OFFSET % 16 == 0 && TG_BUF % 16 == 0, "16-byte aligned operand and accumulator regions");
 
@@ -279,6 +281,9 @@ __global__ void __launch_bounds__(TG_THREADS, 4) k_ls_accumulate_tc(Planes P, co
         int in_batch = 0, stage = 0;
         bool stop = false;
 
+        // the targets of this warp's next 32 sites are on their way while it splits and stores the current ones
+        char* target_rows = reinterpret_cast<char*>(tg_sh + TG_ROWS_OFFSET) + warp * 32 * RowShape<NOUT, float>::STRIDE;
+        stage_targets<NOUT>(target_rows, V, tgt, kc, (long long)blockIdx.x * TG_THREADS + warp * 32, texels, 0, lane);
         for (long long chunk = blockIdx.x; chunk < chunks && !stop; chunk += gridDim.x)
         {
             const long long pixel = chunk * TG_THREADS + tid;
@@ -289,9 +294,20 @@ __global__ void __launch_bounds__(TG_THREADS, 4) k_ls_accumulate_tc(Planes P, co
                 const int bsel = stage % TG_BUFFERS;
                 // 1. this thread's site row, split hi + lo in registers (the previous stage's MMAs run meanwhile)
                 float z[ZS_WIDTH];
+                {
+                    float t[NOUT];
+                    asm volatile("cp.async.wait_all;" ::: "memory");
+                    __syncwarp();
+                    read_row<NOUT, float>(target_rows, lane, t);
+                    __syncwarp();
+                    const long long next = j < kc ? chunk : chunk + gridDim.x;
+                    stage_targets<NOUT>(target_rows, V, tgt, kc, next * TG_THREADS + warp * 32, texels,
+                                        j < kc ? j + 1 : 0, lane);
+                    if (valid)
+                        site_z_staged<NOUT>(P, V, t, pixel, px, py, j, z);
+                }
                 if (valid)
                 {
-                    site_z<NOUT>(P, V, tgt, pixel, px, py, j, z);
                     if constexpr (OBJ)
                     {
                         float sw = 0.0f, ss = 0.0f;

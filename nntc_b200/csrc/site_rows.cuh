@@ -10,7 +10,7 @@
 // FP64 form's sums are of the same floats as before.
 #pragma once
 
-#include "device.cuh"
+#include "row_stage.cuh"
 
 namespace nb
 {
@@ -82,6 +82,65 @@ __device__ __forceinline__ void site_z(const Planes& P, const PlaneView& V, cons
 #pragma unroll
     for (int q = ZS_T + NOUT; q < ZS_WIDTH; q++)
         z[q] = 0.0f;
+}
+
+// site_z with the targets from a row the warp staged (row_stage.cuh) and the latents' channels as vectors: the same row.
+template <int NOUT>
+__device__ __forceinline__ void site_z_staged(const Planes& P, const PlaneView& V, const float (&t)[NOUT], long long pixel,
+                                              int px, int py, int j, float (&z)[ZS_WIDTH])
+{
+    const int c0 = P.c0, c1 = P.c1;
+    float dx, dy;
+    site_offset(P.kc, j, px, py, dx, dy);
+    float s[MAX_CH] = { 0.0f, 0.0f, 0.0f, 0.0f }, c[MAX_CH] = { 0.0f, 0.0f, 0.0f, 0.0f };
+    blend_any(V.v1, V.w1, c1, tap_at(px, py, dx, dy, V.w0, V.h0, V.w1, V.h1), c);
+    if (j == 0)
+    {
+        if (c0 == 4)
+            load_channels<4>(V.v0 + pixel * 4, s);
+        else
+        {
+#pragma unroll
+            for (int i = 0; i < MAX_CH; i++)
+                if (i < c0)
+                    s[i] = __ldg(V.v0 + pixel * c0 + i);
+        }
+    }
+    else
+        blend_any(V.v0, V.w0, c0, tap_at(px, py, dx, dy, V.w0, V.h0, V.w0, V.h0), s);
+#pragma unroll
+    for (int b = 0; b < MAX_CH; b++)
+        z[ZS_C + b] = b < c1 ? c[b] : 0.0f;
+#pragma unroll
+    for (int i = 0; i < MAX_CH; i++)
+        z[ZS_S + i] = i < c0 ? s[i] : 0.0f;
+#pragma unroll
+    for (int i = 0; i < MAX_CH; i++)
+#pragma unroll
+        for (int b = 0; b < MAX_CH; b++)
+            z[ZS_SC + i * 4 + b] = i < c0 && b < c1 ? s[i] * c[b] : 0.0f;
+    z[ZS_ONE] = 1.0f;
+#pragma unroll
+    for (int r = 0; r < NOUT; r++)
+        z[ZS_T + r] = t[r];
+#pragma unroll
+    for (int q = ZS_T + NOUT; q < ZS_WIDTH; q++)
+        z[q] = 0.0f;
+}
+
+// The rows of site j of the 32 pixels from `first` (the warp's), staged asynchronously: the pixels' own source at the
+// centre, else the target cache's rows.
+template <int NOUT>
+__device__ __forceinline__ void stage_targets(char* buffer, const PlaneView& V, const float* tgt, int kc, long long first,
+                                              long long texels, int j, int lane)
+{
+    const int rows = (int)(texels - first < 32 ? texels - first : 32);
+    if (rows <= 0)
+        return;
+    if (j == 0)
+        stage_rows<NOUT, float>(buffer, V.src + (size_t)first * NOUT, NOUT, rows, lane);
+    else
+        stage_rows<NOUT, float>(buffer, tgt + ((size_t)first * kc + (j - 1)) * NOUT, kc * NOUT, rows, lane);
 }
 
 }   // namespace nb
