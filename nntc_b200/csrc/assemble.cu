@@ -674,6 +674,7 @@ static int gather_planes(nntc_b200_device* d, int level0, const Planes& P, int n
                     A.plain = A.plain && std::isfinite(v) && mat[i * c + j] == mat[j * c + i];
                 }
         }
+    d->sten_symmetric[level0] = A.plain != 0;   // symmetric matrices expand to symmetric blocks
     if (q != nmono)
     {
         set_error(NNTC_B200_ERR_STATE, "monomial layout and count disagree");

@@ -459,6 +459,44 @@ struct StenBlock
     }
 };
 
+// A texel's C consecutive doubles, as 16-byte accesses where they are whole vectors.
+template <int C>
+__device__ __forceinline__ void load_texel(const double* p, double* out)
+{
+    if constexpr (C % 2 == 0)
+    {
+#pragma unroll
+        for (int q = 0; q < C / 2; q++)
+        {
+            const double2 v = reinterpret_cast<const double2*>(p)[q];
+            out[2 * q] = v.x;
+            out[2 * q + 1] = v.y;
+        }
+    }
+    else
+    {
+#pragma unroll
+        for (int q = 0; q < C; q++)
+            out[q] = p[q];
+    }
+}
+template <int C>
+__device__ __forceinline__ void store_texel(double* p, const double* v)
+{
+    if constexpr (C % 2 == 0)
+    {
+#pragma unroll
+        for (int q = 0; q < C / 2; q++)
+            reinterpret_cast<double2*>(p)[q] = make_double2(v[2 * q], v[2 * q + 1]);
+    }
+    else
+    {
+#pragma unroll
+        for (int q = 0; q < C; q++)
+            p[q] = v[q];
+    }
+}
+
 // ---- ridge, preconditioner ----------------------------------------------------------------------------------------
 
 template <typename TS>
@@ -505,16 +543,22 @@ __global__ void __launch_bounds__(FOLD_THREADS) k_diag_reduce(Planes P, Red R, d
     }
 }
 
-// Gauss-Jordan with partial pivoting on [a | I], n <= 4, in double (src/solve_level1.cu:689-740).
-__device__ __forceinline__ bool invert(double* a, int n, double* inv)
+// Gauss-Jordan with partial pivoting on [a | I], n <= 4, in double (src/solve_level1.cu:689-740). Unrolled, a pivot row
+// swapped in by selection: a row found at run time would put both matrices in local memory.
+template <int n>
+__device__ __forceinline__ bool invert(double (&a)[n * n], double (&inv)[n * n])
 {
+#pragma unroll
     for (int i = 0; i < n; i++)
+#pragma unroll
         for (int j = 0; j < n; j++)
             inv[i * n + j] = i == j ? 1.0 : 0.0;
+#pragma unroll
     for (int k = 0; k < n; k++)
     {
         int pivot = k;
         double best = fabs(a[k * n + k]);
+#pragma unroll
         for (int i = k + 1; i < n; i++)
             if (fabs(a[i * n + k]) > best)
             {
@@ -523,22 +567,29 @@ __device__ __forceinline__ bool invert(double* a, int n, double* inv)
             }
         if (!(best > 0.0))
             return false;
-        if (pivot != k)
-            for (int j = 0; j < n; j++)
+#pragma unroll
+        for (int i = k + 1; i < n; i++)
+            if (pivot == i)
             {
-                double t = a[k * n + j];
-                a[k * n + j] = a[pivot * n + j];
-                a[pivot * n + j] = t;
-                t = inv[k * n + j];
-                inv[k * n + j] = inv[pivot * n + j];
-                inv[pivot * n + j] = t;
+#pragma unroll
+                for (int j = 0; j < n; j++)
+                {
+                    double t = a[k * n + j];
+                    a[k * n + j] = a[i * n + j];
+                    a[i * n + j] = t;
+                    t = inv[k * n + j];
+                    inv[k * n + j] = inv[i * n + j];
+                    inv[i * n + j] = t;
+                }
             }
         const double s = 1.0 / a[k * n + k];
+#pragma unroll
         for (int j = 0; j < n; j++)
         {
             a[k * n + j] *= s;
             inv[k * n + j] *= s;
         }
+#pragma unroll
         for (int i = 0; i < n; i++)
         {
             if (i == k)
@@ -546,6 +597,7 @@ __device__ __forceinline__ bool invert(double* a, int n, double* inv)
             const double f = a[i * n + k];
             if (f == 0.0)
                 continue;
+#pragma unroll
             for (int j = 0; j < n; j++)
             {
                 a[i * n + j] -= f * a[k * n + j];
@@ -567,6 +619,21 @@ __device__ __forceinline__ void apply_precond(const float* minv, const double* r
     }
 }
 
+// A neighbour's values in the product: whole vectors at four channels; at two the scalar loads measured faster (68
+// against 77 us at 4 x 1024 x 1024: the vectors leave the compiler fewer loads in flight).
+template <int C>
+__device__ __forceinline__ void load_neighbour(const double* p, double* out)
+{
+    if constexpr (C == 4)
+        load_texel<C>(p, out);
+    else
+    {
+#pragma unroll
+        for (int q = 0; q < C; q++)
+            out[q] = p[q];
+    }
+}
+
 // y_t = (H_tt + lambda I) x_t + sum of the owned slots' blocks times the forward neighbours + the transposes of the
 // backward neighbours' blocks (src/solve_level1.cu:781-828), in the reference's order of accumulation.
 template <int C, typename TS>
@@ -576,7 +643,8 @@ __device__ __forceinline__ void stencil_apply(const PlaneView& V, size_t T, long
     constexpr int cc = C * C;
     const int tx = (int)(t % V.w), ty = (int)(t / V.w);
     const size_t sp = stencil_pos(tx, ty, V.w, V.h);
-    const double* xt = x + (size_t)t * C;
+    double xt[C];
+    load_texel<C>(x + (size_t)t * C, xt);
     const StenBlock<C, TS> self(V, 0, T, sp);
 #pragma unroll
     for (int i = 0; i < C; i++)
@@ -598,7 +666,8 @@ __device__ __forceinline__ void stencil_apply(const PlaneView& V, size_t T, long
         const int fx = tx + dx, fy = ty + dy;
         const bool fwd = fx >= 0 && fx < V.w && fy >= 0 && fy < V.h;
         const int gx = fwd ? fx : tx, gy = fwd ? fy : ty;
-        const double* xn = x + ((size_t)gy * V.w + gx) * C;
+        double xn[C], xb[C];
+        load_neighbour<C>(x + ((size_t)gy * V.w + gx) * C, xn);
         const StenBlock<C, TS> blk(V, slot, T, sp);
 #pragma unroll
         for (int i = 0; i < C; i++)
@@ -612,7 +681,7 @@ __device__ __forceinline__ void stencil_apply(const PlaneView& V, size_t T, long
         const bool bwd = bx >= 0 && bx < V.w && by >= 0 && by < V.h;
         const int hx = bwd ? bx : tx, hy = bwd ? by : ty;
         const size_t nt = (size_t)hy * V.w + hx, np = stencil_pos(hx, hy, V.w, V.h);
-        const double* xb = x + nt * C;
+        load_neighbour<C>(x + nt * C, xb);
         const StenBlock<C, TS> nbk(V, slot, T, np);
 #pragma unroll
         for (int i = 0; i < C; i++)
@@ -625,7 +694,10 @@ __device__ __forceinline__ void stencil_apply(const PlaneView& V, size_t T, long
     }
 }
 
-template <typename TS>
+// The channel count as a constant and every texel's values as whole vectors: scalar stores a texel apart wrote each
+// sector of the five vectors and the preconditioner several times (5.0 GB of DRAM writes for 1.1 GB of results, 1915 us
+// at 6 x 2048 x 2048).
+template <int C, typename TS>
 __global__ void __launch_bounds__(THREADS) k_precondition_init(Planes P, Red R)
 {
     __shared__ double sh[2 * 32];
@@ -634,40 +706,60 @@ __global__ void __launch_bounds__(THREADS) k_precondition_init(Planes P, Red R)
     const PlaneView& V = P.p[pl];
     const long long t = base - P.start[pl] + threadIdx.x;
     const size_t T = (size_t)V.w * V.h;
-    const int c = P.c;
+    constexpr int c = C;
     double v[2] = { 0.0, 0.0 };
     const int kind[2] = { 0, 0 };
     if (t < (long long)T)
     {
         const double lambda = R.scalars[(size_t)pl * S_COUNT + S_LAMBDA];
-        double a[MAX_CH * MAX_CH], inv[MAX_CH * MAX_CH];
+        double a[c * c], inv[c * c];
+        const StenBlock<C, TS> self(V, 0, T, stencil_pos((int)(t % V.w), (int)(t / V.w), V.w, V.h));
+#pragma unroll
         for (int i = 0; i < c; i++)
+#pragma unroll
             for (int j = 0; j < c; j++)
-                a[i * c + j] = sten<TS>(V, sten_index<TS>(0, i * c + j, c * c, T, stencil_pos((int)(t % V.w), (int)(t / V.w), V.w, V.h))) +
-                               (i == j ? lambda : 0.0);
-        if (!invert(a, c, inv))
-            for (int i = 0; i < c; i++)
-                for (int j = 0; j < c; j++)
-                    inv[i * c + j] = i == j ? 1.0 : 0.0;
-        float minv[MAX_CH * MAX_CH];
+                a[i * c + j] = self[i * c + j] + (i == j ? lambda : 0.0);
+        const bool inverted = invert<C>(a, inv);
+#pragma unroll
+        for (int i = 0; i < c; i++)
+#pragma unroll
+            for (int j = 0; j < c; j++)
+                inv[i * c + j] = inverted ? inv[i * c + j] : (i == j ? 1.0 : 0.0);
+        float minv[c * c];
+#pragma unroll
         for (int i = 0; i < c * c; i++)
-        {
             minv[i] = (float)inv[i];
-            V.precond[(size_t)t * c * c + i] = minv[i];
+        float* out = V.precond + (size_t)t * c * c;
+        if constexpr (C % 2 == 0)
+        {
+#pragma unroll
+            for (int i = 0; i < c * c / 4; i++)
+                reinterpret_cast<float4*>(out)[i] =
+                    make_float4(minv[4 * i], minv[4 * i + 1], minv[4 * i + 2], minv[4 * i + 3]);
+        }
+        else
+        {
+#pragma unroll
+            for (int i = 0; i < c * c; i++)
+                out[i] = minv[i];
         }
         // CG from d = 0: r = -grad, z = M r, p = z.
-        double r[MAX_CH], z[MAX_CH];
+        double r[c], z[c], zero[c];
+        load_texel<C>(V.grad + (size_t)t * c, r);
+#pragma unroll
         for (int i = 0; i < c; i++)
         {
-            r[i] = -V.grad[(size_t)t * c + i];
-            V.x[(size_t)t * c + i] = 0.0;
-            V.r[(size_t)t * c + i] = r[i];
+            r[i] = -r[i];
+            zero[i] = 0.0;
         }
+        store_texel<C>(V.x + (size_t)t * c, zero);
+        store_texel<C>(V.r + (size_t)t * c, r);
         apply_precond(minv, r, c, z);
+        store_texel<C>(V.z + (size_t)t * c, z);
+        store_texel<C>(V.p + (size_t)t * c, z);
+#pragma unroll
         for (int i = 0; i < c; i++)
         {
-            V.z[(size_t)t * c + i] = z[i];
-            V.p[(size_t)t * c + i] = z[i];
             v[0] += r[i] * r[i];
             v[1] += r[i] * z[i];
         }
@@ -698,7 +790,7 @@ __global__ void __launch_bounds__(FOLD_THREADS) k_cg_start(Planes P, Red R)
 }
 
 template <int C, typename TS>
-__global__ void __launch_bounds__(THREADS) k_cg_matvec(Planes P, Red R)
+__global__ void __launch_bounds__(THREADS, 4) k_cg_matvec(Planes P, Red R)
 {
     __shared__ double sh[32];
     const long long base = (long long)blockIdx.x * blockDim.x;
@@ -714,15 +806,168 @@ __global__ void __launch_bounds__(THREADS) k_cg_matvec(Planes P, Red R)
     const int kind[1] = { 0 };
     if (t < (long long)T)
     {
-        double acc[MAX_CH];
+        double acc[C], pt[C];
         stencil_apply<C, TS>(V, T, t, s[S_LAMBDA], V.p, acc);
+        store_texel<C>(V.ap + (size_t)t * c, acc);
+        load_texel<C>(V.p + (size_t)t * c, pt);
 #pragma unroll
         for (int i = 0; i < c; i++)
+            v[0] += pt[i] * acc[i];
+    }
+    block_reduce(v, kind, sh);
+    if (threadIdx.x == 0)
+        R.partial[blockIdx.x] = v[0];
+}
+
+// The product for an FP32 stencil of two or four channels with a lane per row: C lanes share a texel, lane i forms row i
+// of the product - the same sums in the same order - and reads row i of each of the nine blocks as one vector, so that a
+// warp's reads of a slot are contiguous runs. One thread per texel read each block's rows 64 bytes apart: the L1 served
+// the same line four times, and that bound the kernel (97% of its wavefronts; 627 us at 6 x 2048 x 2048, against 330 us
+// for its bytes; by rows 549 us, bound by the loads' latency: six blocks per SM, four take 690 us). A backward neighbour's transposed block is read by rows too where the blocks are symmetric bit for bit
+// (symmetric != 0), else by columns.
+template <int C>
+__device__ __forceinline__ void load_row(const float* p, float (&r)[C])
+{
+    if constexpr (C == 4)
+    {
+        const float4 v = __ldg(reinterpret_cast<const float4*>(p));
+        r[0] = v.x;
+        r[1] = v.y;
+        r[2] = v.z;
+        r[3] = v.w;
+    }
+    else
+    {
+        const float2 v = __ldg(reinterpret_cast<const float2*>(p));
+        r[0] = v.x;
+        r[1] = v.y;
+    }
+}
+
+// A texel's place among its neighbours, in 32-bit indices: the stencil positions of a row's even and odd texels (the
+// colour-major order of stencil_pos) for its own row and the one above.
+struct TexelPlace
+{
+    int tx, ty, t;               // column, row, row-major index
+    unsigned even, odd;          // this row: position of texel x is (x & 1 ? odd : even) + x / 2
+    unsigned even_up, odd_up;    // the row above (this row where there is none)
+    __device__ __forceinline__ TexelPlace(int x, int y, int w, int h) : tx(x), ty(y), t(y * w + x)
+    {
+        const unsigned w0c = (unsigned)(w + 1) >> 1, w1c = (unsigned)w >> 1, h0c = (unsigned)(h + 1) >> 1;
+        const unsigned h1c = (unsigned)h >> 1, odd_rows = (unsigned)w * h0c;
+        auto row = [&](int r, unsigned& e, unsigned& o) {
+            const unsigned half = (unsigned)r >> 1;
+            e = (r & 1 ? odd_rows : 0u) + half * w0c;
+            o = (r & 1 ? odd_rows + w0c * h1c : w0c * h0c) + half * w1c;
+        };
+        row(y, even, odd);
+        row(y > 0 ? y - 1 : y, even_up, odd_up);
+    }
+    __device__ __forceinline__ unsigned at(int x) const { return (x & 1 ? odd : even) + ((unsigned)x >> 1); }
+    __device__ __forceinline__ unsigned above(int x) const { return (x & 1 ? odd_up : even_up) + ((unsigned)x >> 1); }
+};
+
+// Row i of the four owned blocks times the forward neighbours plus the four backward neighbours' transposed blocks,
+// added to acc in the order of stencil_apply. Every load is issued, a missing neighbour's from the texel itself, whose
+// products are replaced by -0.0.
+template <int C>
+__device__ __forceinline__ void neighbour_rows(const PlaneView& V, unsigned T, const TexelPlace& at, int i, const double* x,
+                                               int symmetric, double& acc)
+{
+    constexpr int cc = C * C;
+    const float* S = reinterpret_cast<const float*>(V.stencil);
+    const int w = V.w;
+    const bool left = at.tx > 0, right = at.tx + 1 < w, up = at.ty > 0, down = at.ty + 1 < V.h;
+    const unsigned sp = at.at(at.tx);
+    // slots 1..4: right, down-left, down, down-right; backward: left, up-right, up, up-left
+    const bool fwd[4] = { right, down && left, down, down && right }, bwd[4] = { left, up && right, up, up && left };
+    const int ahead[4] = { 1, w - 1, w, w + 1 };
+    const unsigned back[4] = { left ? at.at(at.tx - 1) : sp, up && right ? at.above(at.tx + 1) : sp,
+                               up ? at.above(at.tx) : sp, up && left ? at.above(at.tx - 1) : sp };
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+    {
+        double xn[C], xb[C];
+        float own[C], other[C];
+        load_texel<C>(x + (size_t)(at.t + (fwd[q] ? ahead[q] : 0)) * C, xn);
+        load_texel<C>(x + (size_t)(at.t - (bwd[q] ? ahead[q] : 0)) * C, xb);
+        const float* slot = S + (size_t)(q + 1) * T * cc;
+        load_row<C>(slot + (size_t)sp * cc + i * C, own);
+        const float* nb = slot + (size_t)back[q] * cc;
+        if (symmetric)
+            load_row<C>(nb + i * C, other);
+        else
         {
-            V.ap[(size_t)t * c + i] = acc[i];
-            v[0] += V.p[(size_t)t * c + i] * acc[i];
+#pragma unroll
+            for (int j = 0; j < C; j++)
+                other[j] = __ldg(nb + j * C + i);
+        }
+#pragma unroll
+        for (int j = 0; j < C; j++)
+        {
+            const double e = (double)own[j] * xn[j];
+            acc += fwd[q] ? e : -0.0;
+        }
+#pragma unroll
+        for (int j = 0; j < C; j++)
+        {
+            const double e = (double)other[j] * xb[j];
+            acc += bwd[q] ? e : -0.0;
         }
     }
+}
+
+template <int C>
+__global__ void __launch_bounds__(THREADS, 6) k_cg_matvec_rows(Planes P, Red R, int symmetric)
+{
+    __shared__ double sh[32];
+    __shared__ double dot[THREADS];
+    const long long base = (long long)blockIdx.x * blockDim.x;
+    const int pl = plane_of(P, base);
+    const double* s = R.scalars + (size_t)pl * S_COUNT;
+    if (s[S_ACTIVE] == 0.0)
+        return;
+    const PlaneView& V = P.p[pl];
+    const long long t0 = base - P.start[pl];
+    const size_t T = (size_t)V.w * V.h;
+    const double lambda = s[S_LAMBDA];
+    const int lane = threadIdx.x & 31;
+#pragma unroll 1
+    for (int q = 0; q < C; q++)
+    {
+        const int local = (q * THREADS + (int)threadIdx.x) / C, i = (int)threadIdx.x % C;
+        const long long t = t0 + local;
+        double acc = 0.0, pq = 0.0;
+        if (t < (long long)T)
+        {
+            const unsigned row = (unsigned)t / (unsigned)V.w;
+            const TexelPlace at((int)((unsigned)t - row * (unsigned)V.w), (int)row, V.w, V.h);
+            double xt[C];
+            load_texel<C>(V.p + (size_t)t * C, xt);
+            float self[C];
+            load_row<C>(reinterpret_cast<const float*>(V.stencil) + (size_t)at.at(at.tx) * C * C + i * C, self);
+#pragma unroll
+            for (int j = 0; j < C; j++)
+                pq = j == i ? xt[j] : pq;
+            acc = lambda * pq;
+#pragma unroll
+            for (int j = 0; j < C; j++)
+                acc += (double)self[j] * xt[j];
+            neighbour_rows<C>(V, (unsigned)T, at, i, V.p, symmetric, acc);
+            V.ap[(size_t)t * C + i] = acc;
+        }
+        // the texel's share of <p, Ap>, channel by channel
+        const double e = pq * acc;
+        double sum = 0.0;
+#pragma unroll
+        for (int j = 0; j < C; j++)
+            sum += __shfl_sync(0xffffffffu, e, (lane & ~(C - 1)) + j);
+        if (i == 0)
+            dot[local] = sum;
+    }
+    __syncthreads();
+    double v[1] = { dot[threadIdx.x] };
+    const int kind[1] = { 0 };
     block_reduce(v, kind, sh);
     if (threadIdx.x == 0)
         R.partial[blockIdx.x] = v[0];
@@ -804,6 +1049,73 @@ __global__ void __launch_bounds__(THREADS) k_cg_update(Planes P, Red R)
     }
 }
 
+// k_cg_update for one, two or four channels with a lane per value: every vector is read and written in whole lines and
+// lane i applies row i of the preconditioner to the texel's residuals, exchanged within the C lanes; the texels' sums go
+// through shared memory to the block's reduction of one thread per texel. One thread per texel read each vector a texel
+// apart (91% of the L1's wavefronts, 358 us at 6 x 2048 x 2048). Three channels, whose lanes would straddle warps, keep it.
+template <int C>
+__global__ void __launch_bounds__(THREADS) k_cg_update_rows(Planes P, Red R)
+{
+    __shared__ double sh[2 * 32];
+    __shared__ double sums[2][THREADS];
+    const long long base = (long long)blockIdx.x * blockDim.x;
+    const int pl = plane_of(P, base);
+    const double* s = R.scalars + (size_t)pl * S_COUNT;
+    if (s[S_ACTIVE] == 0.0)
+        return;
+    const PlaneView& V = P.p[pl];
+    const long long t0 = base - P.start[pl];
+    const size_t T = (size_t)V.w * V.h;
+    const double alpha = s[S_ALPHA];
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int q = 0; q < C; q++)
+    {
+        const int local = (q * THREADS + (int)threadIdx.x) / C, i = (int)threadIdx.x % C;
+        double r = 0.0, z = 0.0;
+        float minv[C] = {};
+        const size_t e = (size_t)t0 * C + q * THREADS + threadIdx.x;
+        const bool ok = t0 + local < (long long)T;
+        if (ok)
+        {
+            V.x[e] += 1.0 * alpha * V.p[e];
+            r = V.r[e] + -1.0 * alpha * V.ap[e];
+            V.r[e] = r;
+            if constexpr (C == 1)
+                minv[0] = V.precond[e];
+            else
+                load_row<C>(V.precond + e * C, minv);
+        }
+#pragma unroll
+        for (int j = 0; j < C; j++)
+            z += (double)minv[j] * __shfl_sync(0xffffffffu, r, (lane & ~(C - 1)) + j);
+        if (ok)
+            V.z[e] = z;
+        const double rr = r * r, rz = r * z;
+        double srr = 0.0, srz = 0.0;
+#pragma unroll
+        for (int j = 0; j < C; j++)
+        {
+            srr += __shfl_sync(0xffffffffu, rr, (lane & ~(C - 1)) + j);
+            srz += __shfl_sync(0xffffffffu, rz, (lane & ~(C - 1)) + j);
+        }
+        if (i == 0)
+        {
+            sums[0][local] = srr;
+            sums[1][local] = srz;
+        }
+    }
+    __syncthreads();
+    double v[2] = { sums[0][threadIdx.x], sums[1][threadIdx.x] };
+    const int kind[2] = { 0, 0 };
+    block_reduce(v, kind, sh);
+    if (threadIdx.x == 0)
+    {
+        R.partial[blockIdx.x] = v[0];
+        R.partial[R.nblocks + blockIdx.x] = v[1];
+    }
+}
+
 // beta, the residual, and the device-side stop: at an iteration that is a multiple of CG_PROBE a plane whose residual
 // is not at or above the tolerance leaves (the reference's host probe, src/solve_level1.cu:1288-1302): its direction
 // is not updated again, which nothing reads.
@@ -842,15 +1154,14 @@ __global__ void __launch_bounds__(THREADS) k_cg_direction(Planes P, Red R)
     if (s[S_ACTIVE] == 0.0)
         return;
     const PlaneView& V = P.p[pl];
-    const long long t = base - P.start[pl] + threadIdx.x;
-    const size_t T = (size_t)V.w * V.h;
-    if (t >= (long long)T)
-        return;
+    // the block's texels' values, a value a thread: whole lines
+    const size_t first = (size_t)(base - P.start[pl]) * P.c, end = (size_t)V.w * V.h * P.c;
     const double beta = s[S_BETA];
     for (int i = 0; i < P.c; i++)
     {
-        const size_t q = (size_t)t * P.c + i;
-        V.p[q] = V.z[q] + beta * V.p[q];
+        const size_t q = first + (size_t)i * THREADS + threadIdx.x;
+        if (q < end)
+            V.p[q] = V.z[q] + beta * V.p[q];
     }
 }
 
@@ -959,65 +1270,99 @@ struct SweepArgs
     const float* hi;
     int bits;
     int cx, cy;
+    int symmetric;         // the FP32 stencil's blocks are symmetric bit for bit
     unsigned int* moved;   // [plane]
 };
 
+// One colour of one sweep: the texels' couplings to their eight neighbours, then each texel's channels in turn. With an
+// FP32 stencil of two or four channels the couplings are formed a lane per row (neighbour_rows) and handed to the
+// texels' threads through shared memory, so that the stencil is read in whole lines; with an FP64 stencil (a plane of
+// doubles per coefficient) a thread per texel already reads whole lines. The texel's own values are whole vectors.
 template <int C, typename TS>
 __global__ void __launch_bounds__(THREADS) k_quant_sweep(Planes P, SweepArgs A)
 {
+    constexpr bool ROWS = sizeof(TS) == sizeof(float) && C % 2 == 0;
+    __shared__ __align__(16) double coupling[ROWS ? THREADS * C : 1];
     const long long base = (long long)blockIdx.x * blockDim.x;
     const int pl = plane_of(P, base);
     const PlaneView& V = P.p[pl];
-    const long long ci = base - P.start[pl] + threadIdx.x;
     const int cwn = (V.w - A.cx + 1) / 2, chn = (V.h - A.cy + 1) / 2;
-    if (ci >= (long long)cwn * chn)
-        return;
-    const int tx = A.cx + 2 * (int)(ci % cwn);
-    const int ty = A.cy + 2 * (int)(ci / cwn);
-    const size_t t = (size_t)ty * V.w + tx;
-    const size_t sp = stencil_pos(tx, ty, V.w, V.h);
+    const long long ci0 = base - P.start[pl], ci = ci0 + threadIdx.x, n = (long long)cwn * chn;
     const size_t T = (size_t)V.w * V.h;
     constexpr int c = C, cc = C * C;
-    const double lambda = A.scalars[(size_t)pl * S_COUNT + S_LAMBDA];
-    double nb[MAX_CH];
+    double nb[C];
 #pragma unroll
     for (int i = 0; i < c; i++)
         nb[i] = 0.0;
-    // as in stencil_apply: every load issued, a missing neighbour's products replaced by -0.0 (an exact no-op)
-#pragma unroll
-    for (int slot = 1; slot < SLOTS; slot++)
+    if constexpr (ROWS)
     {
-        int dx, dy;
-        slot_offset(slot, dx, dy);
-        const int fx = tx + dx, fy = ty + dy;
-        const bool fwd = fx >= 0 && fx < V.w && fy >= 0 && fy < V.h;
-        const int gx = fwd ? fx : tx, gy = fwd ? fy : ty;
-        const double* xn = V.x + ((size_t)gy * V.w + gx) * c;
-        const StenBlock<C, TS> blk(V, slot, T, sp);
-#pragma unroll
-        for (int i = 0; i < c; i++)
-#pragma unroll
-            for (int j = 0; j < c; j++)
+#pragma unroll 1
+        for (int q = 0; q < C; q++)
+        {
+            const long long at = ci0 + (q * THREADS + (int)threadIdx.x) / C;
+            double acc = 0.0;
+            if (at < n)
             {
-                const double e = blk[i * c + j] * xn[j];
-                nb[i] += fwd ? e : -0.0;
+                const unsigned row = (unsigned)at / (unsigned)cwn;
+                const TexelPlace place(A.cx + 2 * (int)((unsigned)at - row * (unsigned)cwn), A.cy + 2 * (int)row, V.w, V.h);
+                neighbour_rows<C>(V, (unsigned)T, place, (int)threadIdx.x % C, V.x, A.symmetric, acc);
             }
-        const int bx = tx - dx, by = ty - dy;
-        const bool bwd = bx >= 0 && bx < V.w && by >= 0 && by < V.h;
-        const int hx = bwd ? bx : tx, hy = bwd ? by : ty;
-        const size_t nt = (size_t)hy * V.w + hx, np = stencil_pos(hx, hy, V.w, V.h);
-        const double* xb = V.x + nt * c;
-        const StenBlock<C, TS> nbk(V, slot, T, np);
+            coupling[q * THREADS + threadIdx.x] = acc;
+        }
+        __syncthreads();
+        load_texel<C>(coupling + threadIdx.x * C, nb);
+    }
+    if (ci >= n)
+        return;
+    const int tx = A.cx + 2 * (int)((unsigned)ci % (unsigned)cwn);
+    const int ty = A.cy + 2 * (int)((unsigned)ci / (unsigned)cwn);
+    const size_t t = (size_t)ty * V.w + tx;
+    const size_t sp = stencil_pos(tx, ty, V.w, V.h);
+    const double lambda = A.scalars[(size_t)pl * S_COUNT + S_LAMBDA];
+    if constexpr (!ROWS)
+    {
+        // as in stencil_apply: every load issued, a missing neighbour's products replaced by -0.0 (an exact no-op)
 #pragma unroll
-        for (int i = 0; i < c; i++)
+        for (int slot = 1; slot < SLOTS; slot++)
+        {
+            int dx, dy;
+            slot_offset(slot, dx, dy);
+            const int fx = tx + dx, fy = ty + dy;
+            const bool fwd = fx >= 0 && fx < V.w && fy >= 0 && fy < V.h;
+            const int gx = fwd ? fx : tx, gy = fwd ? fy : ty;
+            double xn[C], xb[C];
+            load_texel<C>(V.x + ((size_t)gy * V.w + gx) * c, xn);
+            const StenBlock<C, TS> blk(V, slot, T, sp);
 #pragma unroll
-            for (int j = 0; j < c; j++)
-            {
-                const double e = nbk[j * c + i] * xb[j];
-                nb[i] += bwd ? e : -0.0;
-            }
+            for (int i = 0; i < c; i++)
+#pragma unroll
+                for (int j = 0; j < c; j++)
+                {
+                    const double e = blk[i * c + j] * xn[j];
+                    nb[i] += fwd ? e : -0.0;
+                }
+            const int bx = tx - dx, by = ty - dy;
+            const bool bwd = bx >= 0 && bx < V.w && by >= 0 && by < V.h;
+            const int hx = bwd ? bx : tx, hy = bwd ? by : ty;
+            const size_t nt = (size_t)hy * V.w + hx, np = stencil_pos(hx, hy, V.w, V.h);
+            load_texel<C>(V.x + nt * c, xb);
+            const StenBlock<C, TS> nbk(V, slot, T, np);
+#pragma unroll
+            for (int i = 0; i < c; i++)
+#pragma unroll
+                for (int j = 0; j < c; j++)
+                {
+                    const double e = nbk[j * c + i] * xb[j];
+                    nb[i] += bwd ? e : -0.0;
+                }
+        }
     }
     const StenBlock<C, TS> self(V, 0, T, sp);
+    double x[C], grad[C];
+    float prev[C];
+    load_texel<C>(V.x + t * c, x);
+    load_texel<C>(V.grad + t * c, grad);
+    load_channels<C>(V.prev + t * c, prev);
     unsigned int changed = 0;
 #pragma unroll
     for (int q = 0; q < c; q++)
@@ -1031,9 +1376,9 @@ __global__ void __launch_bounds__(THREADS) k_quant_sweep(Planes P, SweepArgs A)
 #pragma unroll
         for (int j = 0; j < c; j++)
             if (j != q)
-                rest += self[q * c + j] * V.x[t * c + j];
-        const double b = V.grad[idx] + rest;
-        const double want = (double)V.prev[idx] - b / a;
+                rest += self[q * c + j] * x[j];
+        const double b = grad[q] + rest;
+        const double want = (double)prev[q] - b / a;
         const int kk = grid_index(l, A.hi[q], A.bits, (float)want);
         const float value = grid_value(l, A.hi[q], A.bits, kk);
         if ((int)V.k[idx] != kk)
@@ -1042,8 +1387,10 @@ __global__ void __launch_bounds__(THREADS) k_quant_sweep(Planes P, SweepArgs A)
             changed++;
         }
         V.v[idx] = value;
-        V.x[idx] = (double)value - (double)V.prev[idx];
+        x[q] = (double)value - (double)prev[q];
     }
+    // a channel that stayed out of the step keeps its correction: stored as it was read
+    store_texel<C>(V.x + t * c, x);
     if (changed)
         atomicAdd(A.moved + pl, changed);
 }
@@ -1054,14 +1401,16 @@ __global__ void k_snapshot(Planes P)
     const long long base = (long long)blockIdx.x * blockDim.x;
     const int pl = plane_of(P, base);
     const PlaneView& V = P.p[pl];
-    const long long t = base - P.start[pl] + threadIdx.x;
-    if (t >= (long long)V.w * V.h)
-        return;
+    // the block's texels' values, a value a thread: whole lines
+    const size_t first = (size_t)(base - P.start[pl]) * P.c, end = (size_t)V.w * V.h * P.c;
     for (int i = 0; i < P.c; i++)
     {
-        const size_t q = (size_t)t * P.c + i;
-        V.prev[q] = V.v[q];
-        V.x[q] = 0.0;
+        const size_t q = first + (size_t)i * THREADS + threadIdx.x;
+        if (q < end)
+        {
+            V.prev[q] = V.v[q];
+            V.x[q] = 0.0;
+        }
     }
 }
 
@@ -1104,6 +1453,7 @@ int assemble(nntc_b200_device* d, const nntc_b200_model* m, int k, double ridge,
     const bool split = diag_only || (!d->reference_shaped_assembly && k <= 4);
     // the adjoint form stores the stencil in FP32 (the split form only; the reference-shaped kernel is FP64)
     d->sten_f32[level0] = split && d->mixed_stencil != 0;
+    d->sten_symmetric[level0] = false;
     if (split)
         NB_TRY(assemble_split(d, k, level0, P, nmono, mono.data(), diag_only ? 1 : SLOTS, d->sten_f32[level0]));
     else if (level0)
@@ -1148,6 +1498,26 @@ static void fill_report(const nntc_b200_device* d, int i, int channels, nntc_b20
     }
 }
 
+static int precondition_init(nntc_b200_device* d, const Planes& P, const Red& R, int tblocks, bool f32)
+{
+#define NB_PRECOND(C)                                                                                                 \
+    if (f32)                                                                                                          \
+        k_precondition_init<C, float><<<tblocks, THREADS, 0, d->stream>>>(P, R);                                      \
+    else                                                                                                              \
+        k_precondition_init<C, double><<<tblocks, THREADS, 0, d->stream>>>(P, R);                                     \
+    break;
+    switch (P.c)
+    {
+    case 1: NB_PRECOND(1)
+    case 2: NB_PRECOND(2)
+    case 3: NB_PRECOND(3)
+    default: NB_PRECOND(4)
+    }
+#undef NB_PRECOND
+    NB_LAUNCHED();
+    return NNTC_B200_OK;
+}
+
 int solve_block(nntc_b200_device* d, const nntc_b200_model* m, int k, double ridge, int level0,
                 nntc_b200_plane_report* rep, double* ms)
 {
@@ -1163,11 +1533,7 @@ int solve_block(nntc_b200_device* d, const nntc_b200_model* m, int k, double rid
     Planes P = texel_planes(d, level0, k);
     const Red R = red_for(d, P);
     const int tblocks = (int)(P.start[P.n] / THREADS);
-    if (d->sten_f32[level0])
-        k_precondition_init<float><<<tblocks, THREADS, 0, d->stream>>>(P, R);
-    else
-        k_precondition_init<double><<<tblocks, THREADS, 0, d->stream>>>(P, R);
-    NB_LAUNCHED();
+    NB_TRY(precondition_init(d, P, R, tblocks, d->sten_f32[level0]));
     k_cg_start<<<P.n, FOLD_THREADS, 0, d->stream>>>(P, R);
     NB_LAUNCHED();
     NB_CUDA(cudaEventRecord(d->ev[3], d->stream));
@@ -1187,7 +1553,12 @@ int solve_block(nntc_b200_device* d, const nntc_b200_model* m, int k, double rid
     case 3: k_cg_matvec<3, TS><<<tblocks, THREADS, 0, d->stream>>>(P, R); break;                                      \
     default: k_cg_matvec<4, TS><<<tblocks, THREADS, 0, d->stream>>>(P, R); break;                                     \
     }
-            if (d->sten_f32[level0])
+            const int symmetric = d->sten_symmetric[level0] ? 1 : 0;
+            if (d->sten_f32[level0] && P.c == 4)
+                k_cg_matvec_rows<4><<<tblocks, THREADS, 0, d->stream>>>(P, R, symmetric);
+            else if (d->sten_f32[level0] && P.c == 2)
+                k_cg_matvec_rows<2><<<tblocks, THREADS, 0, d->stream>>>(P, R, symmetric);
+            else if (d->sten_f32[level0])
             {
                 NB_MATVEC(float)
             }
@@ -1203,10 +1574,10 @@ int solve_block(nntc_b200_device* d, const nntc_b200_model* m, int k, double rid
         NB_LAUNCHED();
         switch (P.c)
         {
-        case 1: k_cg_update<1><<<tblocks, THREADS, 0, d->stream>>>(P, R); break;
-        case 2: k_cg_update<2><<<tblocks, THREADS, 0, d->stream>>>(P, R); break;
+        case 1: k_cg_update_rows<1><<<tblocks, THREADS, 0, d->stream>>>(P, R); break;
+        case 2: k_cg_update_rows<2><<<tblocks, THREADS, 0, d->stream>>>(P, R); break;
         case 3: k_cg_update<3><<<tblocks, THREADS, 0, d->stream>>>(P, R); break;
-        default: k_cg_update<4><<<tblocks, THREADS, 0, d->stream>>>(P, R); break;
+        default: k_cg_update_rows<4><<<tblocks, THREADS, 0, d->stream>>>(P, R); break;
         }
         NB_LAUNCHED();
         k_cg_beta<<<P.n, FOLD_THREADS, 0, d->stream>>>(P, R, it, active + (it % CG_PROBE),
@@ -1283,7 +1654,8 @@ int sweep_block(nntc_b200_device* d, const nntc_b200_model* m, int k, double rid
             C.kc = k;
             if (C.start[C.n] == 0)
                 continue;
-            SweepArgs A{ d->scalars, level0 ? d->lo0 : d->lo1, level0 ? d->hi0 : d->hi1, bits, cx, cy, d->counters + CNT_SWEEP };
+            SweepArgs A{ d->scalars, level0 ? d->lo0 : d->lo1, level0 ? d->hi0 : d->hi1, bits, cx, cy,
+                         d->sten_symmetric[level0] ? 1 : 0, d->counters + CNT_SWEEP };
             NB_TRY(ktimer_begin(d, NNTC_B200_K_SWEEP));
             const int sblocks = (int)(C.start[C.n] / THREADS);
 #define NB_SWEEP(TS)                                                                                                  \
@@ -1344,11 +1716,7 @@ int descent_direction(nntc_b200_device* d, const nntc_b200_model* m, int k, doub
     Planes P = texel_planes(d, level0, k);
     const Red R = red_for(d, P);
     const int tblocks = (int)(P.start[P.n] / THREADS);
-    if (d->sten_f32[level0])
-        k_precondition_init<float><<<tblocks, THREADS, 0, d->stream>>>(P, R);
-    else
-        k_precondition_init<double><<<tblocks, THREADS, 0, d->stream>>>(P, R);
-    NB_LAUNCHED();
+    NB_TRY(precondition_init(d, P, R, tblocks, d->sten_f32[level0]));
     k_snapshot<<<tblocks, THREADS, 0, d->stream>>>(P);
     NB_LAUNCHED();
     return NNTC_B200_OK;
