@@ -152,28 +152,40 @@ __global__ void k_bc_decode(BcPlanes P, const float* lo0, const float* hi0)
 // The layout of one warp's block in shared memory, per level-0 channel count.
 //
 // A2 couples a texel only with itself and its eight neighbours (the 9-point stencil), so it is held as the sixteen
-// texels' five OWNED stencil blocks, S[texel][slot][i][j] (the texel stride padded to an odd number of doubles), and
+// texels' OWNED stencil blocks whose partner lies in the 4x4 block too (58 of 80, block_at; each padded to an odd number
+// of doubles), and
 // an entry A2[(t, i)][(u, j)] is read from t's block when u sits at one of t's owned offsets, else from u's block,
 // transposed. Every sum over a row of A2 visits only the entries that can be nonzero, in column order: such a sum
 // starts at +0.0 and so never holds -0.0, and adding the product of a structural zero would leave it bit-for-bit
-// unchanged. The vector u = A2 d lives in registers, R rows per lane.
+// unchanged. The vector u = A2 d is kept beside it, each lane updating R of its rows.
 template <int C0>
 struct RefineShape
 {
-    static constexpr int N = 16 * C0;              // unknowns of the block: (texel, channel), texel-major
-    static constexpr int R = (N + 31) / 32;        // rows of u per lane: row r = lane + 32 q
+    static constexpr int N = 16 * C0;              // unknowns of the block: row r is channel r / 16 of texel r % 16
+    static constexpr int R = (N + 31) / 32;        // rows of u a lane updates: row r = lane + 32 q
     static constexpr int CC = C0 * C0;
-    static constexpr int TS = (5 * CC) | 1;        // doubles per texel of S
-    static constexpr int PER_WARP = 16 * TS + 2 * N + 16 + 8 + 16;   // S, a1, d, dlt, the weights, ep and sel
+    static constexpr int BS = CC | 1;              // doubles per stored block of S
+    static constexpr int BLOCKS = 16 + 12 + 9 + 12 + 9;   // the owned blocks whose partner lies in the 4x4 block
+    static constexpr int FOLD = 17;                // doubles per row of the fold scratch: 16 terms, padded
+    // S, a1, d (then u), dlt, the weights, the candidates, five rows of fold scratch, ep and sel
+    static constexpr int PER_WARP = BLOCKS * BS + 2 * N + 16 + 8 + 8 + 5 * FOLD + 1 + 16;
 };
+
+// Where the owned block of texel t towards slot `slot`'s neighbour starts in S, for a neighbour inside the 4x4 block: the
+// sixteen self blocks, then right (3 a row), down-left (3 a row, three rows), down (4 a row) and down-right.
+template <int C0>
+__device__ __forceinline__ int block_at(int t, int slot)
+{
+    const int base = slot == 0 ? 0 : (slot == 1 ? 16 : (slot == 2 ? 27 : (slot == 3 ? 37 : 49)));
+    return (base + t - (slot == 0 || slot == 3 ? 0 : t >> 2)) * RefineShape<C0>::BS;
+}
 
 // The entry of A2 at row (t, i), column (u, j), where u is t's neighbour number k (k = (dy + 1) 3 + (dx + 1), the
 // neighbours' order by texel index).
 template <int C0>
 __device__ __forceinline__ double a2_entry(const double* S, int t, int i, int u, int j, int k)
 {
-    using Sh = RefineShape<C0>;
-    return k >= 4 ? S[t * Sh::TS + (k - 4) * Sh::CC + i * C0 + j] : S[u * Sh::TS + (4 - k) * Sh::CC + j * C0 + i];
+    return k >= 4 ? S[block_at<C0>(t, k - 4) + i * C0 + j] : S[block_at<C0>(u, 4 - k) + j * C0 + i];
 }
 
 // Neighbour k of in-block texel t, or -1 outside the block.
@@ -190,27 +202,13 @@ __device__ __forceinline__ int neighbour_index(int t, int u)
     return dx >= -1 && dx <= 1 && dy >= -1 && dy <= 1 ? (dy + 1) * 3 + (dx + 1) : -1;
 }
 
-// Row idx of u, from the lane that holds it (every lane takes part; the value is meaningful on every lane).
-template <int R>
-__device__ __forceinline__ double row_of(const double (&uv)[R], int idx)
-{
-    double v = 0.0;
-#pragma unroll
-    for (int q = 0; q < R; q++)
-    {
-        const double x = __shfl_sync(0xffffffffu, uv[q], idx & 31);
-        if ((idx >> 5) == q)
-            v = x;
-    }
-    return v;
-}
-
-// The sixteen lanes' terms folded serially in texel order, the same on every lane.
-__device__ __forceinline__ double fold16(double v)
+// The sixteen terms of a row of the fold scratch added serially in texel order.
+__device__ __forceinline__ double fold16(const double* row)
 {
     double s = 0.0;
+#pragma unroll
     for (int t = 0; t < 16; t++)
-        s += __shfl_sync(0xffffffffu, v, t);
+        s += row[t];
     return s;
 }
 
@@ -225,18 +223,21 @@ struct RefineArgs
 // One warp per 4x4 block of the colour; the blocks of every plane of the chain in one launch (start[] counts blocks
 // of the colour per plane).
 template <int C0>
-__global__ void __launch_bounds__(32 * REFINE_WARPS, 8) k_bc_refine(BcPlanes P, RefineArgs R)
+__global__ void __launch_bounds__(32 * REFINE_WARPS, 10) k_bc_refine(BcPlanes P, RefineArgs R)
 {
     using Sh = RefineShape<C0>;
-    constexpr int N = Sh::N, RR = Sh::R, TS = Sh::TS, CC = Sh::CC;
+    constexpr int N = Sh::N, RR = Sh::R, CC = Sh::CC;
     extern __shared__ double smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     double* S = smem + warp * Sh::PER_WARP;
-    double* a1 = S + 16 * TS;
+    double* a1 = S + Sh::BLOCKS * Sh::BS;
     double* dv = a1 + N;
+    double* us = dv;   // d is spent once u = A2 d is formed
     double* dlt = dv + N;
     double* w8 = dlt + 16;
-    int* s_ep = (int*)(w8 + 8);                          // 8 ints
+    double* cand = w8 + 8;                               // a channel's eight candidate values
+    double* fold = cand + 8;                             // five rows of FOLD doubles
+    int* s_ep = (int*)(fold + 5 * Sh::FOLD + 1);         // 8 ints
     unsigned char* s_sel = (unsigned char*)(s_ep + 8);   // 64 bytes
 
     const long long bi = (long long)blockIdx.x * REFINE_WARPS + warp;
@@ -267,7 +268,7 @@ __global__ void __launch_bounds__(32 * REFINE_WARPS, 8) k_bc_refine(BcPlanes P, 
         const int r = lane + 32 * q;
         if (r >= N)
             continue;
-        const int t = r / C0, i = r % C0;
+        const int t = r & 15, i = r >> 4;
         const int px = gx * 4 + (t & 3), py = gy * 4 + (t >> 2);
         const bool in = px < w0 && py < h0;
         const size_t ti = in ? (size_t)py * w0 + px : 0;
@@ -282,16 +283,23 @@ __global__ void __launch_bounds__(32 * REFINE_WARPS, 8) k_bc_refine(BcPlanes P, 
             const int lx = fx - gx * 4, ly = fy - gy * 4;
             const bool f_blk = lx >= 0 && lx < 4 && ly >= 0 && ly < 4;
             const double* row = own + (size_t)(slot * CC + i * C0) * 16 + t;   // coefficient j at row[16 j]
-            double* s_row = S + t * TS + slot * CC + i * C0;
+            double own_row[C0];
 #pragma unroll
             for (int j = 0; j < C0; j++)
-                s_row[j] = f_img && f_blk ? row[16 * j] : 0.0;
-            if (f_img && !f_blk)
+                own_row[j] = f_img ? row[16 * j] : 0.0;
+            if (f_blk)
+            {
+                double* s_row = S + block_at<C0>(t, slot) + i * C0;
+#pragma unroll
+                for (int j = 0; j < C0; j++)
+                    s_row[j] = own_row[j];
+            }
+            else if (f_img)
             {
                 const double* xn = B.delta + ((size_t)fy * w0 + fx) * C0;
 #pragma unroll
                 for (int j = 0; j < C0; j++)
-                    acc += row[16 * j] * xn[j];
+                    acc += own_row[j] * xn[j];
             }
             if (slot == 0 || !in)
                 continue;
@@ -326,11 +334,10 @@ __global__ void __launch_bounds__(32 * REFINE_WARPS, 8) k_bc_refine(BcPlanes P, 
 #pragma unroll
     for (int q = 0; q < RR; q++)
     {
-        uv[q] = 0.0;
         const int r = lane + 32 * q;
         if (r >= N)
             continue;
-        const int t = r / C0, i = r % C0;
+        const int t = r & 15, i = r >> 4;
         double s = 0.0;
 #pragma unroll
         for (int k = 0; k < 9; k++)
@@ -340,10 +347,16 @@ __global__ void __launch_bounds__(32 * REFINE_WARPS, 8) k_bc_refine(BcPlanes P, 
                 continue;
 #pragma unroll
             for (int j = 0; j < C0; j++)
-                s += a2_entry<C0>(S, t, i, u, j, k) * dv[u * C0 + j];
+                s += a2_entry<C0>(S, t, i, u, j, k) * dv[j * 16 + u];
         }
         uv[q] = s;
     }
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < RR; q++)
+        if (lane + 32 * q < N)
+            us[lane + 32 * q] = uv[q];
+    __syncwarp();
 
     double taken = 0.0;
     const int t16 = lane & 15;
@@ -351,9 +364,10 @@ __global__ void __launch_bounds__(32 * REFINE_WARPS, 8) k_bc_refine(BcPlanes P, 
     for (int c = 0; c < C0; c++)
     {
         const double step = ((double)R.hi0[c] - (double)R.lo0[c]) / 255.0;
-        const int idx = t16 * C0 + c;
-        const double u_idx = row_of(uv, idx);
-        double tbp = 0.0, tbq = 0.0, tpap = 0.0, tpaq = 0.0, tqaq = 0.0;
+        const int idx = c * 16 + t16;
+        const double u_idx = us[idx];
+        // the five sums' terms, one texel a lane, then a sum a lane: a fold by shuffles on every lane was 48 instructions
+        // a sum
         if (lane < 16)
         {
             const double a = w8[s_sel[c * 16 + lane]];
@@ -372,14 +386,17 @@ __global__ void __launch_bounds__(32 * REFINE_WARPS, 8) k_bc_refine(BcPlanes P, 
                 ap += e * step * aj;
                 aq += e * step * (1.0 - aj);
             }
-            tbp = b * p;
-            tbq = b * q;
-            tpap = p * ap;
-            tpaq = p * aq;
-            tqaq = q * aq;
+            fold[lane] = b * p;
+            fold[Sh::FOLD + lane] = b * q;
+            fold[2 * Sh::FOLD + lane] = p * ap;
+            fold[3 * Sh::FOLD + lane] = p * aq;
+            fold[4 * Sh::FOLD + lane] = q * aq;
         }
-        const double bp = fold16(tbp), bq = fold16(tbq), pap = fold16(tpap), paq = fold16(tpaq),
-                     qaq = fold16(tqaq);
+        __syncwarp();
+        const double folded = fold16(fold + (lane < 5 ? lane : 0) * Sh::FOLD);
+        const double bp = __shfl_sync(0xffffffffu, folded, 0), bq = __shfl_sync(0xffffffffu, folded, 1),
+                     pap = __shfl_sync(0xffffffffu, folded, 2), paq = __shfl_sync(0xffffffffu, folded, 3),
+                     qaq = __shfl_sync(0xffffffffu, folded, 4);
         const int r0 = s_ep[2 * c], r1 = s_ep[2 * c + 1];
         const double det = pap * qaq - paq * paq;
         double d0 = 0.0, d1 = 0.0;
@@ -390,24 +407,29 @@ __global__ void __launch_bounds__(32 * REFINE_WARPS, 8) k_bc_refine(BcPlanes P, 
         }
         const double v0r = (double)r0 + d0, v1r = (double)r1 + d1;
         const int c0r = (int)floor(v0r + 0.5), c1r = (int)floor(v1r + 0.5);
-        double best = 0.0;
+        // the nine rounded candidates, one a lane; the lowest change wins, ties to the earlier candidate: the one an
+        // in-order scan with a strict `<` from zero keeps
         int best0 = r0, best1 = r1;
-        for (int e0 = -1; e0 <= 1; e0++)
-            for (int e1 = -1; e1 <= 1; e1++)
+        {
+            const int n = lane < 9 ? lane : 8;
+            const int e0 = n / 3 - 1, e1 = n % 3 - 1;
+            const int a0 = c0r + e0 < 0 ? 0 : (c0r + e0 > 255 ? 255 : c0r + e0);
+            const int a1i = c1r + e1 < 0 ? 0 : (c1r + e1 > 255 ? 255 : c1r + e1);
+            const double f0 = (double)(a0 - r0), f1 = (double)(a1i - r1);
+            const double de = 2.0 * (bp * f0 + bq * f1) + pap * f0 * f0 + 2.0 * paq * f0 * f1 + qaq * f1 * f1;
+            const double mine = lane < 9 && a0 > a1i && de < 0.0 ? de : 0.0;
+            double v = mine;
+#pragma unroll
+            for (int o = 1; o < 16; o <<= 1)
+                v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
+            v = __shfl_sync(0xffffffffu, v, 0);
+            if (v < 0.0)
             {
-                const int a0 = c0r + e0 < 0 ? 0 : (c0r + e0 > 255 ? 255 : c0r + e0);
-                const int a1i = c1r + e1 < 0 ? 0 : (c1r + e1 > 255 ? 255 : c1r + e1);
-                if (a0 <= a1i)
-                    continue;
-                const double f0 = (double)(a0 - r0), f1 = (double)(a1i - r1);
-                const double de = 2.0 * (bp * f0 + bq * f1) + pap * f0 * f0 + 2.0 * paq * f0 * f1 + qaq * f1 * f1;
-                if (de < best)
-                {
-                    best = de;
-                    best0 = a0;
-                    best1 = a1i;
-                }
+                const int win = __ffs(__ballot_sync(0xffffffffu, lane < 9 && mine == v)) - 1;
+                best0 = __shfl_sync(0xffffffffu, a0, win);
+                best1 = __shfl_sync(0xffffffffu, a1i, win);
             }
+        }
         if (best0 == r0 && best1 == r1)
             continue;
         if (lane < 16)
@@ -417,7 +439,6 @@ __global__ void __launch_bounds__(32 * REFINE_WARPS, 8) k_bc_refine(BcPlanes P, 
             dlt[lane] = (double)next - (double)now;
         }
         __syncwarp();
-        double term = 0.0;
         if (lane < 16)
         {
             double quad = 0.0;
@@ -428,9 +449,10 @@ __global__ void __launch_bounds__(32 * REFINE_WARPS, 8) k_bc_refine(BcPlanes P, 
                 if (u >= 0)
                     quad += a2_entry<C0>(S, lane, c, u, c, k) * dlt[u];
             }
-            term = dlt[lane] * (2.0 * (a1[idx] + u_idx) + quad);
+            fold[lane] = dlt[lane] * (2.0 * (a1[idx] + u_idx) + quad);
         }
-        const double exact = fold16(term);
+        __syncwarp();
+        const double exact = fold16(fold);
         if (exact < 0.0)
         {
 #pragma unroll
@@ -439,7 +461,7 @@ __global__ void __launch_bounds__(32 * REFINE_WARPS, 8) k_bc_refine(BcPlanes P, 
                 const int r = lane + 32 * q;
                 if (r >= N)
                     continue;
-                const int t = r / C0, i = r % C0;
+                const int t = r & 15, i = r >> 4;
                 double add = 0.0;
 #pragma unroll
                 for (int k = 0; k < 9; k++)
@@ -448,7 +470,7 @@ __global__ void __launch_bounds__(32 * REFINE_WARPS, 8) k_bc_refine(BcPlanes P, 
                     if (u >= 0)
                         add += a2_entry<C0>(S, t, i, u, c, k) * dlt[u];
                 }
-                uv[q] += add;
+                us[r] += add;
             }
             if (lane == 0)
             {
@@ -461,70 +483,84 @@ __global__ void __launch_bounds__(32 * REFINE_WARPS, 8) k_bc_refine(BcPlanes P, 
     }
 
     // ---- (ii) the selectors: two Gauss-Seidel passes of exact 8-way argmins (src/cpu/cpu_refine_bc.cpp:314-345).
-    // Every group of eight lanes evaluates the eight candidates, one per lane, and takes the lowest change in three
-    // butterfly rounds, ties to the lower candidate: the candidate the reference's in-order scan with a strict `<`
-    // keeps, and no candidate when none lowers E.
-    //
-    // The four groups of eight lanes take four consecutive texels' steps at once, each against the current u. A step's
-    // inputs are the sequential scan's as long as no earlier step of the four moved a selector; so the first step of
-    // the four that lowers E is taken, the steps before it stand (none of them lowered E), and the scan resumes after
-    // it. Steps that lower nothing, the common case once the selectors settle, cost a quarter of an iteration each.
-    const int k8 = lane & 7, grp = lane >> 3;
+    // All sixteen texels' steps are evaluated at once against the current u, a texel on two lanes of four candidates
+    // each, with the tie rule of an in-order scan with a strict `<` (the lower candidate, and none when none lowers E).
+    // A step's inputs are the sequential scan's as long as no earlier texel's selector moved; so the first texel at or
+    // after the scan's place that lowers E is taken, the steps before it stand (none of them lowered E), and the scan
+    // resumes after it with every step evaluated again. A pass that moves k selectors costs k + 1 evaluations, where a
+    // group of eight lanes per texel, four texels at a time, took k + 4 with three rounds of exchanges in each.
+    const int half = lane >> 4;
     for (int pass = 0; pass < 2; pass++)
         for (int c = 0; c < C0; c++)
         {
-            const int r0 = s_ep[2 * c], r1 = s_ep[2 * c + 1];
-            const double cand = (double)bc0_value(R.lo0[c], R.hi0[c], bc4_entry(r0, r1, k8));
-            int t0 = 0;
-            while (t0 < 16)
-            {
-                const int t = t0 + grp < 16 ? t0 + grp : 15;   // past the last texel a group repeats it, unused
-                const int i = t * C0 + c;
-                const double b = a1[i] + row_of(uv, i);
-                const double a = S[t * TS + c * C0 + c];
-                const int cur = s_sel[c * 16 + t];
-                const double now = __shfl_sync(0xffffffffu, cand, cur);
-                const double d = cand - now;
-                const double de = 2.0 * b * d + a * d * d;
-                // the lowest change of the group's eight candidates (a candidate that does not lower E counts as 0),
-                // then the first candidate that reaches it: the one the reference's in-order scan with a strict `<`
-                // keeps
-                const double mine = de < 0.0 ? de : 0.0;
-                double v = mine;
+            if (lane < 8)
+                cand[lane] = (double)bc0_value(R.lo0[c], R.hi0[c], bc4_entry(s_ep[2 * c], s_ep[2 * c + 1], lane));
+            __syncwarp();
+            double cv[4];
 #pragma unroll
-                for (int o = 1; o < 8; o <<= 1)
-                    v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
-                const unsigned hits = __ballot_sync(0xffffffffu, mine == v);
-                const int id = __ffs((hits >> (grp * 8)) & 0xffu) - 1;
-                const unsigned lowers = __ballot_sync(0xffffffffu, k8 == 0 && t0 + grp < 16 && v < 0.0);
-                if (lowers == 0u)
+            for (int k = 0; k < 4; k++)
+                cv[k] = cand[half * 4 + k];
+            const int idx = c * 16 + t16;
+            const double a = S[block_at<C0>(t16, 0) + c * C0 + c], a1_idx = a1[idx];
+            int cur = s_sel[c * 16 + t16], t0 = 0;
+            while (true)
+            {
+                const double b = a1_idx + us[idx], now = cand[cur];
+                double v = 0.0;
+                int id = 0;
+#pragma unroll
+                for (int k = 0; k < 4; k++)
                 {
-                    t0 += 4;
-                    continue;
+                    const double d = cv[k] - now;
+                    const double de = 2.0 * b * d + a * d * d;
+                    if (de < v)
+                    {
+                        v = de;
+                        id = half * 4 + k;
+                    }
                 }
-                // the first group whose step lowers E: its texel, change, candidate and new value on every lane
-                const int g = (__ffs(lowers) - 1) >> 3;
-                const int tf = t0 + g;
-                const double vf = __shfl_sync(0xffffffffu, v, g * 8);
-                const int idf = __shfl_sync(0xffffffffu, id, g * 8);
-                const double mv = __shfl_sync(0xffffffffu, d, g * 8 + idf);
+                // the texel's lower half of candidates wins a tie
+                const double ov = __shfl_xor_sync(0xffffffffu, v, 16);
+                const int oid = __shfl_xor_sync(0xffffffffu, id, 16);
+                if (half == 0 ? ov < v : ov <= v)
+                {
+                    v = ov;
+                    id = oid;
+                }
+                const unsigned lowers = __ballot_sync(0xffffffffu, half == 0 && t16 >= t0 && v < 0.0);
+                if (lowers == 0u)
+                    break;
+                // the first texel whose step lowers E: its change, candidate and new value on every lane
+                const int tf = __ffs(lowers) - 1, near = neighbour_index(t16, tf);
+                const double vf = __shfl_sync(0xffffffffu, v, tf);
+                const int idf = __shfl_sync(0xffffffffu, id, tf);
+                const double mv = cand[idf] - __shfl_sync(0xffffffffu, now, tf);
+                __syncwarp();   // every lane has read its us
+                // the block that couples the lane's texel with tf, the texel's own or tf's transposed
+                const bool own_block = near >= 4;
+                const int slot = own_block ? near - 4 : 4 - near, owner = own_block ? t16 : tf;
+                const int first = (int)((0x31251b1000ull >> (8 * (slot & 7))) & 0xff) + owner -
+                                  ((0x16 >> (slot & 7)) & 1 ? owner >> 2 : 0);   // block_at
+                const double* coupling = S + first * Sh::BS + (own_block ? c : c * C0);
+                const int step = own_block ? C0 : 1;
 #pragma unroll
                 for (int q = 0; q < RR; q++)
                 {
                     const int r = lane + 32 * q;
                     if (r >= N)
                         continue;
-                    const int rt = r / C0, ri = r % C0;
-                    const int k = neighbour_index(rt, tf);
-                    if (k >= 0)
-                        uv[q] += a2_entry<C0>(S, rt, ri, tf, c, k) * mv;
+                    if (near >= 0)   // every row of a lane is of its own texel
+                        us[r] += coupling[(r >> 4) * step] * mv;
                 }
-                if (lane == 0)
-                    s_sel[c * 16 + tf] = (unsigned char)idf;
+                if (t16 == tf)
+                    cur = idf;
                 taken += vf;
-                __syncwarp();
                 t0 = tf + 1;
+                __syncwarp();
             }
+            if (half == 0)
+                s_sel[c * 16 + t16] = (unsigned char)cur;
+            __syncwarp();
         }
 
     // ---- what the block leaves behind
