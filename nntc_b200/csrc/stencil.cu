@@ -1263,7 +1263,49 @@ __global__ void __launch_bounds__(FOLD_THREADS) k_movement_reduce(Planes P, Red 
 
 // ---- the quantised phase (src/solve_level1.cu:1023-1098) ----------------------------------------------------------
 
-struct SweepArgs
+// The fractions rep(k) / 255 of a grid's values, formed once per block: grid_index and grid_value divide by 255 for each
+// of the values they look at, four divisions a channel that nothing but the index decides.
+constexpr int GRID_FRACTIONS = 256;
+__device__ __forceinline__ void grid_fractions(double* frac, int bits)
+{
+    for (int k = threadIdx.x; k < (1 << bits); k += blockDim.x)
+        frac[k] = (double)rep_index(k, bits) / 255.0;
+}
+
+// grid_index and the value of the index it finds, from the block's fractions: the same bits.
+__device__ __forceinline__ int grid_nearest(float lo, float hi, int bits, float value, const double* frac, float& nearest)
+{
+    const double span = (double)hi - (double)lo;
+    const int levels = (1 << bits) - 1;
+    auto at = [&](int k) { return (float)__dadd_rn((double)lo, __dmul_rn(frac[k], span)); };
+    int best = 0;
+    if (span > 0.0)
+    {
+        double x = ((double)value - (double)lo) / span * (double)levels;
+        x = x < 0.0 ? 0.0 : (x > (double)levels ? (double)levels : x);
+        int k = (int)(x + 0.5);
+        k = k < 0 ? 0 : (k > levels ? levels : k);
+        best = k;
+        double best_d = fabs((double)value - (double)at(k));
+#pragma unroll
+        for (int d = -1; d <= 1; d += 2)
+        {
+            const int n = k + d;
+            if (n < 0 || n > levels)
+                continue;
+            const double dist = fabs((double)value - (double)at(n));
+            if (dist < best_d || (dist == best_d && n < best))
+            {
+                best_d = dist;
+                best = n;
+            }
+        }
+    }
+    nearest = at(best);
+    return best;
+}
+
+struct ColourArgs
 {
     const double* scalars;
     const float* lo;
@@ -1279,10 +1321,14 @@ struct SweepArgs
 // texels' threads through shared memory, so that the stencil is read in whole lines; with an FP64 stencil (a plane of
 // doubles per coefficient) a thread per texel already reads whole lines. The texel's own values are whole vectors.
 template <int C, typename TS>
-__global__ void __launch_bounds__(THREADS) k_quant_sweep(Planes P, SweepArgs A)
+__global__ void __launch_bounds__(THREADS) k_quant_colour(Planes P, ColourArgs A)
 {
     constexpr bool ROWS = sizeof(TS) == sizeof(float) && C % 2 == 0;
     __shared__ __align__(16) double coupling[ROWS ? THREADS * C : 1];
+    // (an FP64 stencil's kernel has no barrier to hide the fractions' set-up behind: with it 183 -> 201 us a colour)
+    __shared__ double frac[ROWS ? GRID_FRACTIONS : 1];
+    if (ROWS)
+        grid_fractions(frac, A.bits);
     const long long base = (long long)blockIdx.x * blockDim.x;
     const int pl = plane_of(P, base);
     const PlaneView& V = P.p[pl];
@@ -1309,7 +1355,7 @@ __global__ void __launch_bounds__(THREADS) k_quant_sweep(Planes P, SweepArgs A)
             }
             coupling[q * THREADS + threadIdx.x] = acc;
         }
-        __syncthreads();
+        __syncthreads();   // the fractions and the couplings
         load_texel<C>(coupling + threadIdx.x * C, nb);
     }
     if (ci >= n)
@@ -1379,8 +1425,15 @@ __global__ void __launch_bounds__(THREADS) k_quant_sweep(Planes P, SweepArgs A)
                 rest += self[q * c + j] * x[j];
         const double b = grad[q] + rest;
         const double want = (double)prev[q] - b / a;
-        const int kk = grid_index(l, A.hi[q], A.bits, (float)want);
-        const float value = grid_value(l, A.hi[q], A.bits, kk);
+        float value;
+        int kk;
+        if constexpr (ROWS)
+            kk = grid_nearest(l, A.hi[q], A.bits, (float)want, frac, value);
+        else
+        {
+            kk = grid_index(l, A.hi[q], A.bits, (float)want);
+            value = grid_value(l, A.hi[q], A.bits, kk);
+        }
         if ((int)V.k[idx] != kk)
         {
             V.k[idx] = (uint8_t)kk;
@@ -1393,6 +1446,286 @@ __global__ void __launch_bounds__(THREADS) k_quant_sweep(Planes P, SweepArgs A)
     store_texel<C>(V.x + t * c, x);
     if (changed)
         atomicAdd(A.moved + pl, changed);
+}
+
+// A whole sweep, its four colours in order, in one launch, for planes of at most a tile an SM. A block takes a tile of
+// SWEEP_W x SWEEP_H texels, holds the corrections of the tile and a margin in shared memory, and takes the colours one
+// after another; what a later colour of the tile needs of the texels outside it is computed by the block itself - colour 0
+// three texels out (two up and down), colour 1 two, colour 2 one - from the corrections before the sweep, so that every
+// texel's step has exactly the inputs it has in four launches of one colour each, and blocks need not wait on one another.
+// The corrections are read from one vector and written to another (x and r in turn), and a tile's own texels alone are
+// written.
+//
+// Where the line lies: a colour of few texels is a launch whose threads each wait out the same loads and divisions, so four
+// of them in one launch save three rounds of that (1 x 256 x 256, level 1: 49 -> 32 us a sweep, level 0: 26 -> 17 us; 1 x
+// 100 x 76: 58 -> 26 us). With more tiles than SMs the tiles' second wave costs as much again (175 k level-1 texels: 71
+// against 35 us), and at level 0 of 4 x 2048 x 1024 the colours side by side, at four blocks an SM, read a quarter less from
+// DRAM and still took 675 against 560 us (FP64: 1314 against 732 us), waiting at the colours' barriers.
+constexpr int SWEEP_W = 32, SWEEP_H = 28, SWEEP_MARGIN = 4;
+constexpr int SWEEP_COLS = (SWEEP_W + 2 * SWEEP_MARGIN) / 2, SWEEP_ROWS = (SWEEP_H + 2 * SWEEP_MARGIN) / 2;   // a colour's
+constexpr int SWEEP_CELLS = SWEEP_COLS * SWEEP_ROWS;
+constexpr int SWEEP_TILES = 148;
+// Threads: a colour's texels in one pass (FP64), or its rows in two or three (FP32).
+template <typename TS>
+constexpr int SWEEP_THREADS = sizeof(TS) == sizeof(float) ? 512 : 320;
+
+struct SweepArgs
+{
+    const double* scalars;
+    const float* lo;
+    const float* hi;
+    int bits;
+    int symmetric;         // the FP32 stencil's blocks are symmetric bit for bit
+    int first;             // the first sweep: the corrections are zero
+    int to_r;              // the corrections go to r and come from x, else the other way round
+    int bend[MAX_PLANES];  // one past each plane's last block, the planes in descending order
+    int btiles[MAX_PLANES];
+    unsigned int* moved;   // [plane]
+};
+
+// The corrections of the tile and its margin: [pair of channels][colour][row][column].
+template <int C>
+struct TileX
+{
+    static constexpr int PAIRS = (C + 1) / 2;
+    double2* cells;
+    __device__ __forceinline__ int at(int rx, int ry) const
+    {
+        return ((rx & 1) + 2 * (ry & 1)) * SWEEP_CELLS + (ry >> 1) * SWEEP_COLS + (rx >> 1);
+    }
+    __device__ __forceinline__ void get(int rx, int ry, double* out) const
+    {
+        const int i = at(rx, ry);
+#pragma unroll
+        for (int q = 0; q < PAIRS; q++)
+        {
+            const double2 v = cells[q * 4 * SWEEP_CELLS + i];
+            out[2 * q] = v.x;
+            if (2 * q + 1 < C)
+                out[2 * q + 1] = v.y;
+        }
+    }
+    __device__ __forceinline__ void set(int rx, int ry, const double* v) const
+    {
+        const int i = at(rx, ry);
+#pragma unroll
+        for (int q = 0; q < PAIRS; q++)
+            cells[q * 4 * SWEEP_CELLS + i] = make_double2(v[2 * q], 2 * q + 1 < C ? v[2 * q + 1] : 0.0);
+    }
+};
+
+template <int C, typename TS, int COLOUR>
+__device__ __forceinline__ unsigned sweep_colour(const PlaneView& V, const SweepArgs& A, double lambda, int x0, int y0,
+                                                 const TileX<C>& X, const double* frac, double* coupling, double* xout)
+{
+    constexpr bool ROWS = sizeof(TS) == sizeof(float) && C % 2 == 0;
+    constexpr int cx = COLOUR & 1, cy = COLOUR >> 1, cc = C * C;
+    // this colour's texels of the tile and as far outside it as the later colours read
+    constexpr int hx = COLOUR == 0 ? 3 : (COLOUR == 1 ? 2 : (COLOUR == 2 ? 1 : 0));
+    constexpr int hy = COLOUR <= 1 ? 2 : (COLOUR == 2 ? 1 : 0);
+    constexpr int rx0 = SWEEP_MARGIN - hx + ((SWEEP_MARGIN - hx) % 2 != cx), ry0 = SWEEP_MARGIN - hy + ((SWEEP_MARGIN - hy) % 2 != cy);
+    constexpr int nx = (SWEEP_MARGIN + SWEEP_W - 1 + hx - rx0) / 2 + 1, ny = (SWEEP_MARGIN + SWEEP_H - 1 + hy - ry0) / 2 + 1;
+    constexpr int TASKS = nx * ny;
+    const int w = V.w, h = V.h;
+    const size_t T = (size_t)w * h;
+    unsigned changed = 0;
+#pragma unroll 1
+    for (int batch = 0; batch < TASKS; batch += SWEEP_THREADS<TS>)
+    {
+        if constexpr (ROWS)
+        {
+            const float* S = reinterpret_cast<const float*>(V.stencil);
+#pragma unroll 1
+            for (int q = 0; q < C; q++)
+            {
+                const int task = batch + (q * SWEEP_THREADS<TS> + (int)threadIdx.x) / C, i = (int)threadIdx.x % C;
+                const int rx = rx0 + 2 * (task % nx), ry = ry0 + 2 * (task / nx);
+                const int gx = x0 - SWEEP_MARGIN + rx, gy = y0 - SWEEP_MARGIN + ry;
+                double acc = 0.0;
+                if (task < TASKS && gx >= 0 && gx < w && gy >= 0 && gy < h)
+                {
+                    const TexelPlace at(gx, gy, w, h);
+                    const bool left = gx > 0, right = gx + 1 < w, up = gy > 0, down = gy + 1 < h;
+                    const unsigned sp = at.at(gx);
+                    // slots 1..4: right, down-left, down, down-right; backward: left, up-right, up, up-left
+                    const bool fwd[4] = { right, down && left, down, down && right };
+                    const bool bwd[4] = { left, up && right, up, up && left };
+                    const unsigned back[4] = { left ? at.at(gx - 1) : sp, up && right ? at.above(gx + 1) : sp,
+                                               up ? at.above(gx) : sp, up && left ? at.above(gx - 1) : sp };
+#pragma unroll
+                    for (int d = 0; d < 4; d++)
+                    {
+                        int dx, dy;
+                        slot_offset(d + 1, dx, dy);
+                        float own[C], other[C];
+                        const float* slot = S + (size_t)(d + 1) * T * cc;
+                        load_row<C>(slot + (size_t)sp * cc + i * C, own);
+                        const float* nb = slot + (size_t)back[d] * cc;
+                        if (A.symmetric)
+                            load_row<C>(nb + i * C, other);
+                        else
+                        {
+#pragma unroll
+                            for (int j = 0; j < C; j++)
+                                other[j] = __ldg(nb + j * C + i);
+                        }
+                        double xn[C], xb[C];
+                        X.get(rx + dx, ry + dy, xn);
+                        X.get(rx - dx, ry - dy, xb);
+#pragma unroll
+                        for (int j = 0; j < C; j++)
+                        {
+                            const double e = (double)own[j] * xn[j];
+                            acc += fwd[d] ? e : -0.0;
+                        }
+#pragma unroll
+                        for (int j = 0; j < C; j++)
+                        {
+                            const double e = (double)other[j] * xb[j];
+                            acc += bwd[d] ? e : -0.0;
+                        }
+                    }
+                }
+                coupling[q * SWEEP_THREADS<TS> + threadIdx.x] = acc;
+            }
+            __syncthreads();
+        }
+        const int task = batch + (int)threadIdx.x;
+        const int rx = rx0 + 2 * (task % nx), ry = ry0 + 2 * (task / nx);
+        const int gx = x0 - SWEEP_MARGIN + rx, gy = y0 - SWEEP_MARGIN + ry;
+        if (task < TASKS && gx >= 0 && gx < w && gy >= 0 && gy < h)
+        {
+            const size_t t = (size_t)gy * w + gx, sp = stencil_pos(gx, gy, w, h);
+            const bool own = rx >= SWEEP_MARGIN && rx < SWEEP_MARGIN + SWEEP_W && ry >= SWEEP_MARGIN &&
+                             ry < SWEEP_MARGIN + SWEEP_H;
+            double nb[C];
+            if constexpr (ROWS)
+                load_texel<C>(coupling + threadIdx.x * C, nb);
+            else
+            {
+#pragma unroll
+                for (int i = 0; i < C; i++)
+                    nb[i] = 0.0;
+                // as in stencil_apply: every load issued, a missing neighbour's products replaced by -0.0 (an exact no-op)
+#pragma unroll
+                for (int slot = 1; slot < SLOTS; slot++)
+                {
+                    int dx, dy;
+                    slot_offset(slot, dx, dy);
+                    const bool fwd = gx + dx >= 0 && gx + dx < w && gy + dy < h;
+                    const bool bwd = gx - dx >= 0 && gx - dx < w && gy - dy >= 0;
+                    double xn[C], xb[C];
+                    X.get(rx + dx, ry + dy, xn);
+                    X.get(rx - dx, ry - dy, xb);
+                    const StenBlock<C, TS> blk(V, slot, T, sp);
+#pragma unroll
+                    for (int i = 0; i < C; i++)
+#pragma unroll
+                        for (int j = 0; j < C; j++)
+                        {
+                            const double e = blk[i * C + j] * xn[j];
+                            nb[i] += fwd ? e : -0.0;
+                        }
+                    const StenBlock<C, TS> nbk(V, slot, T, bwd ? stencil_pos(gx - dx, gy - dy, w, h) : sp);
+#pragma unroll
+                    for (int i = 0; i < C; i++)
+#pragma unroll
+                        for (int j = 0; j < C; j++)
+                        {
+                            const double e = nbk[j * C + i] * xb[j];
+                            nb[i] += bwd ? e : -0.0;
+                        }
+                }
+            }
+            const StenBlock<C, TS> self(V, 0, T, sp);
+            double x[2 * TileX<C>::PAIRS], grad[C];
+            float prev[C];
+            X.get(rx, ry, x);
+            load_texel<C>(V.grad + t * C, grad);
+            load_channels<C>(V.prev + t * C, prev);
+#pragma unroll
+            for (int q = 0; q < C; q++)
+            {
+                const float l = A.lo[q], span = A.hi[q] - A.lo[q];
+                const double a = self[q * C + q] + lambda;
+                if (!(a > 0.0) || !(span > 0.0f))
+                    continue;
+                double rest = nb[q];
+#pragma unroll
+                for (int j = 0; j < C; j++)
+                    if (j != q)
+                        rest += self[q * C + j] * x[j];
+                const double b = grad[q] + rest;
+                const double want = (double)prev[q] - b / a;
+                float value;
+                const int kk = grid_nearest(l, A.hi[q], A.bits, (float)want, frac, value);
+                if (own)
+                {
+                    const size_t idx = t * C + q;
+                    if ((int)V.k[idx] != kk)
+                    {
+                        V.k[idx] = (uint8_t)kk;
+                        changed++;
+                    }
+                    V.v[idx] = value;
+                }
+                x[q] = (double)value - (double)prev[q];
+            }
+            X.set(rx, ry, x);
+            if (own)
+                store_texel<C>(xout + t * C, x);
+        }
+        __syncthreads();   // the couplings are spent; after the last batch, the colour is done
+    }
+    return changed;
+}
+
+template <int C, typename TS>
+__global__ void __launch_bounds__(SWEEP_THREADS<TS>, 1) k_quant_sweep(Planes P, const __grid_constant__ SweepArgs A)
+{
+    extern __shared__ double2 sweep_sh[];
+    __shared__ double frac[GRID_FRACTIONS];
+    grid_fractions(frac, A.bits);
+    const TileX<C> X{ sweep_sh };
+    double* coupling = reinterpret_cast<double*>(sweep_sh + TileX<C>::PAIRS * 4 * SWEEP_CELLS);
+    int pl = P.n - 1;
+    while ((int)blockIdx.x >= A.bend[pl])
+        pl--;
+    const int tile = (int)blockIdx.x - (A.bend[pl] - A.btiles[pl]);
+    const PlaneView& V = P.p[pl];
+    const int tiles_x = (V.w + SWEEP_W - 1) / SWEEP_W;
+    const int x0 = tile % tiles_x * SWEEP_W, y0 = tile / tiles_x * SWEEP_H;
+    const double* xin = A.to_r ? V.x : V.r;
+    double* xout = A.to_r ? V.r : V.x;
+    for (int i = threadIdx.x; i < 4 * SWEEP_CELLS; i += SWEEP_THREADS<TS>)
+    {
+        const int rx = i % (2 * SWEEP_COLS), ry = i / (2 * SWEEP_COLS);
+        const int gx = x0 - SWEEP_MARGIN + rx, gy = y0 - SWEEP_MARGIN + ry;
+        double x[2 * TileX<C>::PAIRS] = {};
+        if (!A.first && gx >= 0 && gx < V.w && gy >= 0 && gy < V.h)
+            load_texel<C>(xin + ((size_t)gy * V.w + gx) * C, x);
+        X.set(rx, ry, x);
+    }
+    __syncthreads();
+    const double lambda = A.scalars[(size_t)pl * S_COUNT + S_LAMBDA];
+    unsigned changed = sweep_colour<C, TS, 0>(V, A, lambda, x0, y0, X, frac, coupling, xout);
+    changed += sweep_colour<C, TS, 1>(V, A, lambda, x0, y0, X, frac, coupling, xout);
+    changed += sweep_colour<C, TS, 2>(V, A, lambda, x0, y0, X, frac, coupling, xout);
+    changed += sweep_colour<C, TS, 3>(V, A, lambda, x0, y0, X, frac, coupling, xout);
+    if (changed)
+        atomicAdd(A.moved + pl, changed);
+}
+
+template <int C, typename TS>
+static int launch_sweep(nntc_b200_device* d, const Planes& P, const SweepArgs& A, int tiles)
+{
+    constexpr bool ROWS = sizeof(TS) == sizeof(float) && C % 2 == 0;
+    const int shared =
+        TileX<C>::PAIRS * 4 * SWEEP_CELLS * (int)sizeof(double2) + (ROWS ? SWEEP_THREADS<TS> * C * (int)sizeof(double) : 0);
+    NB_CUDA(cudaFuncSetAttribute(k_quant_sweep<C, TS>, cudaFuncAttributeMaxDynamicSharedMemorySize, shared));
+    k_quant_sweep<C, TS><<<tiles, SWEEP_THREADS<TS>, shared, d->stream>>>(P, A);
+    NB_LAUNCHED();
+    return NNTC_B200_OK;
 }
 
 // prev = v, x = 0 (the quantised path and the refinement measure the correction from the plane as assembled).
@@ -1643,7 +1976,36 @@ int sweep_block(nntc_b200_device* d, const nntc_b200_model* m, int k, double rid
     NB_LAUNCHED();
     NB_CUDA(cudaMemsetAsync(d->counters + CNT_SWEEP, 0, MAX_PLANES * sizeof(unsigned int), d->stream));
     const int bits = level0 ? 8 : m->bits1;
-    for (int s = 0; s < sweeps; s++)
+    SweepArgs S{ d->scalars, level0 ? d->lo0 : d->lo1, level0 ? d->hi0 : d->hi1, bits, d->sten_symmetric[level0] ? 1 : 0 };
+    S.moved = d->counters + CNT_SWEEP;
+    int tiles = 0;
+    for (int i = P.n - 1; i >= 0; i--)
+    {
+        S.btiles[i] = ((P.p[i].w + SWEEP_W - 1) / SWEEP_W) * ((P.p[i].h + SWEEP_H - 1) / SWEEP_H);
+        S.bend[i] = tiles += S.btiles[i];
+    }
+    for (int s = 0; s < sweeps && tiles <= SWEEP_TILES; s++)
+    {
+        S.first = s == 0;
+        S.to_r = (sweeps - 1 - s) & 1;   // the last sweep leaves the corrections in x
+        NB_TRY(ktimer_begin(d, NNTC_B200_K_SWEEP));
+#define NB_SWEEP(C)                                                                                                   \
+    if (d->sten_f32[level0])                                                                                          \
+        NB_TRY((launch_sweep<C, float>(d, P, S, tiles)));                                                             \
+    else                                                                                                              \
+        NB_TRY((launch_sweep<C, double>(d, P, S, tiles)));                                                            \
+    break;
+        switch (P.c)
+        {
+        case 1: NB_SWEEP(1)
+        case 2: NB_SWEEP(2)
+        case 3: NB_SWEEP(3)
+        default: NB_SWEEP(4)
+        }
+#undef NB_SWEEP
+        NB_TRY(ktimer_end(d));
+    }
+    for (int s = 0; s < sweeps && tiles > SWEEP_TILES; s++)
         for (int colour = 0; colour < 4; colour++)
         {
             const int cx = colour & 1, cy = colour >> 1;
@@ -1654,17 +2016,17 @@ int sweep_block(nntc_b200_device* d, const nntc_b200_model* m, int k, double rid
             C.kc = k;
             if (C.start[C.n] == 0)
                 continue;
-            SweepArgs A{ d->scalars, level0 ? d->lo0 : d->lo1, level0 ? d->hi0 : d->hi1, bits, cx, cy,
+            ColourArgs A{ d->scalars, level0 ? d->lo0 : d->lo1, level0 ? d->hi0 : d->hi1, bits, cx, cy,
                          d->sten_symmetric[level0] ? 1 : 0, d->counters + CNT_SWEEP };
             NB_TRY(ktimer_begin(d, NNTC_B200_K_SWEEP));
             const int sblocks = (int)(C.start[C.n] / THREADS);
 #define NB_SWEEP(TS)                                                                                                  \
     switch (C.c)                                                                                                      \
     {                                                                                                                 \
-    case 1: k_quant_sweep<1, TS><<<sblocks, THREADS, 0, d->stream>>>(C, A); break;                                    \
-    case 2: k_quant_sweep<2, TS><<<sblocks, THREADS, 0, d->stream>>>(C, A); break;                                    \
-    case 3: k_quant_sweep<3, TS><<<sblocks, THREADS, 0, d->stream>>>(C, A); break;                                    \
-    default: k_quant_sweep<4, TS><<<sblocks, THREADS, 0, d->stream>>>(C, A); break;                                   \
+    case 1: k_quant_colour<1, TS><<<sblocks, THREADS, 0, d->stream>>>(C, A); break;                                    \
+    case 2: k_quant_colour<2, TS><<<sblocks, THREADS, 0, d->stream>>>(C, A); break;                                    \
+    case 3: k_quant_colour<3, TS><<<sblocks, THREADS, 0, d->stream>>>(C, A); break;                                    \
+    default: k_quant_colour<4, TS><<<sblocks, THREADS, 0, d->stream>>>(C, A); break;                                   \
     }
             if (d->sten_f32[level0])
             {
