@@ -262,14 +262,19 @@ __global__ void __launch_bounds__(LR_THREADS) k_ls_obj_reduce(const double* part
     }
 }
 
-// obj_sums (the mixed-precision Gram only): also the objective's three raw sums per plane of the decoder on the device,
-// at the same sites, into host memory (3 per plane).
-int normal_equations(nntc_b200_device* d, int k, const double* per_site, double* ms, std::vector<double>* obj_sums)
+// The normal equations queued, up to the end of their span. with_obj (the mixed-precision Gram only): also the
+// objective's three raw sums per plane of the decoder on the device, at the same sites, fetched.
+static int queue_normal_equations(nntc_b200_device* d, int k, const double* per_site, bool with_obj)
 {
+    if (with_obj && !d->mixed_gram)
+    {
+        set_error(NNTC_B200_ERR_STATE, "the objective rides only on the tensor-core normal equations");
+        return NNTC_B200_ERR_STATE;
+    }
     const int mm = d->nin + 1;
     const int entries = mm * (mm + 1) / 2 + d->nout * mm;
     double* omega = d->ls_partial + (size_t)d->planes.size() * entries * LS_GRID;
-    NB_CUDA(cudaMemcpyAsync(omega, per_site, d->planes.size() * sizeof(double), cudaMemcpyHostToDevice, d->stream));
+    NB_TRY(upload_small(d, omega, per_site, d->planes.size() * sizeof(double)));
     Planes P = planes_for(d, 0, [&](int) { return (size_t)0; });
     P.kc = k;
     NB_TRY(block_begin(d));
@@ -288,7 +293,7 @@ int normal_equations(nntc_b200_device* d, int k, const double* per_site, double*
     {
         NB_CUDA(cudaMemsetAsync(d->counters + CNT_STATUS, 0, sizeof(unsigned int), d->stream));
         NB_TRY(ktimer_begin(d, NNTC_B200_K_NORMAL_EQ));
-        NB_TRY(launch_ls_accumulate_tc(d, P, d->ls_partial, entries, A.tgt, d->stream, obj_sums ? d->ls_obj : nullptr));
+        NB_TRY(launch_ls_accumulate_tc(d, P, d->ls_partial, entries, A.tgt, d->stream, with_obj ? d->ls_obj : nullptr));
         NB_TRY(ktimer_end(d));
     }
     else
@@ -321,33 +326,41 @@ int normal_equations(nntc_b200_device* d, int k, const double* per_site, double*
     NB_CUDA(cudaFuncSetAttribute(k_ls_reduce, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lr_shared));
     k_ls_reduce<<<entries, LR_THREADS, lr_shared, d->stream>>>(d->ls_partial, entries, P.n, omega, d->reduction);
     NB_LAUNCHED();
-    const bool with_obj = obj_sums && d->mixed_gram;
     double* obj_out = d->ls_obj + (size_t)P.n * 3 * LS_GRID;
     if (with_obj)
     {
         k_ls_obj_reduce<<<P.n, LR_THREADS, 0, d->stream>>>(d->ls_obj, P.n, obj_out);
         NB_LAUNCHED();
     }
-    NB_TRY(block_end(d, ms));
+    NB_TRY(block_mark(d));
     if (with_obj)
-    {
-        obj_sums->assign((size_t)3 * P.n, 0.0);
-        NB_TRY(download(d, obj_sums->data(), obj_out, obj_sums->size() * sizeof(double)));
-    }
-    else if (obj_sums)
-    {
-        set_error(NNTC_B200_ERR_STATE, "the objective rides only on the tensor-core normal equations");
-        return NNTC_B200_ERR_STATE;
-    }
+        NB_TRY(fetch(d, FETCH_OBJECTIVE, obj_out, (size_t)3 * P.n * sizeof(double)));
     if (d->mixed_gram)
+        NB_TRY(fetch(d, FETCH_STATUS, d->counters + CNT_STATUS, sizeof(unsigned int)));
+    return NNTC_B200_OK;
+}
+
+// The wait for queue_normal_equations (and whatever was queued after it), its span and its status.
+static int finish_normal_equations(nntc_b200_device* d, double* ms)
+{
+    NB_TRY(block_finish(d, ms));
+    if (d->mixed_gram && *fetched<unsigned int>(d, FETCH_STATUS))
     {
-        unsigned int status = 0;
-        NB_TRY(download(d, &status, d->counters + CNT_STATUS, sizeof(status)));
-        if (status)
-        {
-            set_error(NNTC_B200_ERR_TIMEOUT, "the tensor-core normal equations gave up waiting on their MMAs");
-            return NNTC_B200_ERR_TIMEOUT;
-        }
+        set_error(NNTC_B200_ERR_TIMEOUT, "the tensor-core normal equations gave up waiting on their MMAs");
+        return NNTC_B200_ERR_TIMEOUT;
+    }
+    return NNTC_B200_OK;
+}
+
+// obj_sums: the objective's sums too, 3 per plane (queue_normal_equations' with_obj).
+int normal_equations(nntc_b200_device* d, int k, const double* per_site, double* ms, std::vector<double>* obj_sums)
+{
+    NB_TRY(queue_normal_equations(d, k, per_site, obj_sums != nullptr));
+    NB_TRY(finish_normal_equations(d, ms));
+    if (obj_sums)
+    {
+        const double* sums = fetched<double>(d, FETCH_OBJECTIVE);
+        obj_sums->assign(sums, sums + (size_t)3 * d->planes.size());
     }
     return NNTC_B200_OK;
 }
@@ -597,14 +610,15 @@ __global__ void __launch_bounds__(DS_THREADS) k_decoder_solve(const double* __re
         out->rung = 4;
 }
 
-static_assert(sizeof(DecoderSolveOut) <= 2048, "the arena's dec_solve slice holds one DecoderSolveOut");
+static_assert(sizeof(DecoderSolveOut) <= 2048, "the arena's dec_solve slice and the fetch place hold one");
 
 static long long g_rung_tally[4] = { 0, 0, 0, 0 };
 
 void objective_from_sums(const nntc_b200_model& m, int k, const double* per_site, const std::vector<double>& acc,
                          nntc_b200_objective* r);
 
-int solve_decoder_on_device(nntc_b200_device* d, nntc_b200_model& m, int k, const double* per_site)
+// The solve queued on the normal equations on the device, its answer fetched.
+static int queue_decoder_solve(nntc_b200_device* d, const nntc_b200_model& m, int k, const double* per_site)
 {
     DecoderSolveArgs a{};
     a.nin = m.nin;
@@ -626,8 +640,13 @@ int solve_decoder_on_device(nntc_b200_device* d, nntc_b200_model& m, int k, cons
     DecoderSolveOut* dev_out = reinterpret_cast<DecoderSolveOut*>(d->dec_solve);
     k_decoder_solve<<<1, DS_THREADS, 0, d->stream>>>(d->reduction, a, dev_out);
     NB_LAUNCHED();
-    DecoderSolveOut o;
-    NB_TRY(download(d, &o, dev_out, sizeof(o)));
+    return fetch(d, FETCH_DECODER, dev_out, sizeof(DecoderSolveOut));
+}
+
+// The fetched answer into the model and onto the device.
+static int take_decoder(nntc_b200_device* d, nntc_b200_model& m)
+{
+    const DecoderSolveOut& o = *fetched<DecoderSolveOut>(d, FETCH_DECODER);
     const int mm = m.nin + 1;
     g_rung_tally[o.rung < 3 ? o.rung : 3]++;
     if (o.rung <= 3)
@@ -640,7 +659,7 @@ int solve_decoder_on_device(nntc_b200_device* d, nntc_b200_model& m, int k, cons
         }
         m.has_decoder = 1;
     }
-    return NNTC_B200_OK;
+    return upload_decoder(d, &m);
 }
 
 }   // namespace nb
@@ -653,9 +672,11 @@ extern "C"
 int nntc_b200_solve_decoder(nntc_b200_device* d, nntc_b200_model* m, int k, const double* per_site, double* ms)
 {
     double t = 0.0;
-    NB_TRY(normal_equations(d, k, per_site, &t, nullptr));
-    NB_TRY(solve_decoder_on_device(d, *m, k, per_site));
-    NB_TRY(upload_decoder(d, m));
+    // one wait for both: the solve needs nothing of the host
+    NB_TRY(queue_normal_equations(d, k, per_site, false));
+    NB_TRY(queue_decoder_solve(d, *m, k, per_site));
+    NB_TRY(finish_normal_equations(d, &t));
+    NB_TRY(take_decoder(d, *m));
     if (ms)
         *ms = t;
     return NNTC_B200_OK;
@@ -682,8 +703,9 @@ int normal_equations_and_objective(nntc_b200_device* d, const nntc_b200_model* m
 // Block (a) from the normal equations already on the device (normal_equations_and_objective at the same latents).
 int solve_decoder_prepared(nntc_b200_device* d, nntc_b200_model* m, int k, const double* per_site)
 {
-    NB_TRY(solve_decoder_on_device(d, *m, k, per_site));
-    return upload_decoder(d, m);
+    NB_TRY(queue_decoder_solve(d, *m, k, per_site));
+    NB_CUDA(cudaStreamSynchronize(d->stream));
+    return take_decoder(d, *m);
 }
 
 }   // namespace nb

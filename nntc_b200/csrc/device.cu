@@ -108,9 +108,20 @@ int block_begin(nntc_b200_device* d)
     return NNTC_B200_OK;
 }
 
-int block_end(nntc_b200_device* d, double* ms)
+int block_mark(nntc_b200_device* d)
 {
     NB_CUDA(cudaEventRecord(d->ev[1], d->stream));
+    return NNTC_B200_OK;
+}
+
+int block_end(nntc_b200_device* d, double* ms)
+{
+    NB_TRY(block_mark(d));
+    return block_finish(d, ms);
+}
+
+int block_finish(nntc_b200_device* d, double* ms)
+{
     NB_CUDA(cudaStreamSynchronize(d->stream));
     float t = 0.0f;
     NB_CUDA(cudaEventElapsedTime(&t, d->ev[0], d->ev[1]));
@@ -125,6 +136,31 @@ int upload(nntc_b200_device* d, void* dst, const void* src, size_t bytes)
         return NNTC_B200_OK;
     NB_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, d->stream));
     NB_CUDA(cudaStreamSynchronize(d->stream));
+    return NNTC_B200_OK;
+}
+
+int upload_small(nntc_b200_device* d, void* dst, const void* src, size_t bytes)
+{
+    if (bytes == 0)
+        return NNTC_B200_OK;
+    if (bytes > STAGE_RING / 2)
+        return upload(d, dst, src, bytes);
+    if (d->stage_at + bytes > STAGE_RING)
+    {
+        // the ring starts over: what it still carries has to be on the device first
+        NB_CUDA(cudaStreamSynchronize(d->stream));
+        d->stage_at = 0;
+    }
+    unsigned char* slot = d->host_stage + d->stage_at;
+    d->stage_at += (bytes + 63) / 64 * 64;
+    std::memcpy(slot, src, bytes);
+    NB_CUDA(cudaMemcpyAsync(dst, slot, bytes, cudaMemcpyHostToDevice, d->stream));
+    return NNTC_B200_OK;
+}
+
+int fetch(nntc_b200_device* d, Fetched place, const void* src, size_t bytes)
+{
+    NB_CUDA(cudaMemcpyAsync(d->host_stage + STAGE_RING + place, src, bytes, cudaMemcpyDeviceToHost, d->stream));
     return NNTC_B200_OK;
 }
 
@@ -156,8 +192,8 @@ int upload_decoder(nntc_b200_device* d, const nntc_b200_model* m)
     // what it had (src/device.cuh:472-478 with zero bytes).
     if (!m->has_decoder)
         return NNTC_B200_OK;
-    NB_TRY(upload(d, d->weights, m->dec_w, (size_t)d->nout * d->nin * sizeof(float)));
-    NB_TRY(upload(d, d->bias, m->dec_b, (size_t)d->nout * sizeof(float)));
+    NB_TRY(upload_small(d, d->weights, m->dec_w, (size_t)d->nout * d->nin * sizeof(float)));
+    NB_TRY(upload_small(d, d->bias, m->dec_b, (size_t)d->nout * sizeof(float)));
     std::memcpy(d->host_weights, m->dec_w, (size_t)d->nout * d->nin * sizeof(float));
     std::memcpy(d->host_bias, m->dec_b, (size_t)d->nout * sizeof(float));
     return NNTC_B200_OK;
@@ -169,7 +205,7 @@ int upload_grids(nntc_b200_device* d, const nntc_b200_model* m)
     for (int c = 0; c < d->c0; c++)
         for (int k = 0; k < m->palette0_len[c] && k < 16; k++)
             pal[(size_t)c * 16 + k] = m->palette0[c][k];
-    NB_TRY(upload(d, d->palette, pal.data(), pal.size() * sizeof(float)));
+    NB_TRY(upload_small(d, d->palette, pal.data(), pal.size() * sizeof(float)));
     float lo[MAX_CH] = {}, hi[MAX_CH] = {};
     if (m->has_lo1)
         for (int c = 0; c < d->c1; c++)
@@ -177,8 +213,8 @@ int upload_grids(nntc_b200_device* d, const nntc_b200_model* m)
             lo[c] = m->lo1[c];
             hi[c] = m->hi1[c];
         }
-    NB_TRY(upload(d, d->lo1, lo, sizeof(lo)));
-    NB_TRY(upload(d, d->hi1, hi, sizeof(hi)));
+    NB_TRY(upload_small(d, d->lo1, lo, sizeof(lo)));
+    NB_TRY(upload_small(d, d->hi1, hi, sizeof(hi)));
     if (d->lo0)
     {
         float l0[MAX_CH] = {}, h0[MAX_CH] = {};
@@ -188,8 +224,8 @@ int upload_grids(nntc_b200_device* d, const nntc_b200_model* m)
                 l0[c] = m->lo0[c];
                 h0[c] = m->hi0[c];
             }
-        NB_TRY(upload(d, d->lo0, l0, sizeof(l0)));
-        NB_TRY(upload(d, d->hi0, h0, sizeof(h0)));
+        NB_TRY(upload_small(d, d->lo0, l0, sizeof(l0)));
+        NB_TRY(upload_small(d, d->hi0, h0, sizeof(h0)));
     }
     d->m.has_lo0 = m->has_lo0;
     d->m.has_lo1 = m->has_lo1;
@@ -641,6 +677,7 @@ static int device_create_impl(const nntc_b200_model* m, const float* const* chai
     }
     NB_CK(cudaMallocHost(&d->host_scalars, (size_t)MAX_PLANES * S_COUNT * sizeof(double)));
     NB_CK(cudaMallocHost(&d->host_counters, (size_t)COUNTERS * sizeof(unsigned int)));
+    NB_CK(cudaMallocHost(&d->host_stage, HOST_STAGE));
     // the set-up's copies and clears went to the legacy stream; the model's own stream does not wait for it
     NB_CK(cudaDeviceSynchronize());
     d->m.has_decoder = 0;
@@ -692,6 +729,7 @@ void nntc_b200_device_destroy(nntc_b200_device* d)
     cudaFree(d->arena);
     cudaFreeHost(d->host_scalars);
     cudaFreeHost(d->host_counters);
+    cudaFreeHost(d->host_stage);
     for (const nntc_b200_device::Pending& p : d->kpending)
     {
         cudaEventDestroy(p.a);

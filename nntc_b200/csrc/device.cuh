@@ -157,6 +157,11 @@ struct nntc_b200_device
     cudaEvent_t ev[4] = {};
     double* host_scalars = nullptr;      // pinned, MAX_PLANES * S_COUNT
     unsigned int* host_counters = nullptr;
+    // Pinned staging of this handle's small transfers (one allocation, HOST_STAGE bytes): a ring that small uploads are
+    // copied through without waiting for them, then fixed places that small results are fetched to and read after the
+    // wait that ends their block.
+    unsigned char* host_stage = nullptr;
+    size_t stage_at = 0;                 // the ring's next byte
     void* arena = nullptr;               // the one device allocation every buffer above is a slice of
     void* keep = nullptr;                // bc8: the outer repack loop's copy of both latents and the BC state
     size_t bytes = 0;                    // the arena's size
@@ -260,6 +265,32 @@ int ktimer_harvest(nntc_b200_device* d);
 
 // Planes 1.. of the source chain from plane 0, on the device: each level the 2x2 box of the one above.
 int build_source_chain(nntc_b200_device* d);
+
+// block_end in two halves, for results fetched between them: the span's end recorded; then the wait.
+int block_mark(nntc_b200_device* d);
+int block_finish(nntc_b200_device* d, double* ms);
+
+// A small upload on the model's stream without a wait: the bytes go through the handle's pinned ring, so the caller's
+// buffer is free on return and everything queued later sees them. Larger ones are upload()s.
+int upload_small(nntc_b200_device* d, void* dst, const void* src, size_t bytes);
+
+// A small result into its place in pinned memory, queued on the model's stream: to be read after the next wait.
+enum Fetched
+{
+    FETCH_OBJECTIVE = 0,     // 3 doubles per plane
+    FETCH_DECODER = 1024,    // a DecoderSolveOut
+    FETCH_STATUS = 3072,     // the device status word
+    FETCH_ACTIVE = 3136,     // the conjugate gradients' active planes
+    FETCH_BC_STATS = 3200,   // 2 doubles per plane
+    FETCH_BYTES = 4096
+};
+constexpr size_t STAGE_RING = 60 * 1024, HOST_STAGE = STAGE_RING + FETCH_BYTES;
+int fetch(nntc_b200_device* d, Fetched place, const void* src, size_t bytes);
+template <typename T>
+inline const T* fetched(const nntc_b200_device* d, Fetched place)
+{
+    return reinterpret_cast<const T*>(d->host_stage + STAGE_RING + place);
+}
 
 // Upload on the model's stream and wait (the staging buffer is the caller's).
 int upload(nntc_b200_device* d, void* dst, const void* src, size_t bytes);

@@ -785,6 +785,15 @@ int objective_sums(nntc_b200_device* d, int k, std::vector<double>& acc, double*
         W.b[r] = (double)d->host_bias[r];
         W.cw[r] = (double)d->m.cw[r];
     }
+    // the planes' sums with the wait that ends the pass
+    auto fetch_sums = [&]() {
+        acc.assign((size_t)3 * P.n, 0.0);
+        NB_TRY(block_mark(d));
+        NB_TRY(fetch(d, FETCH_OBJECTIVE, sums, acc.size() * sizeof(double)));
+        NB_TRY(block_finish(d, ms));
+        std::copy_n(fetched<double>(d, FETCH_OBJECTIVE), acc.size(), acc.begin());
+        return (int)NNTC_B200_OK;
+    };
     NB_TRY(block_begin(d));
     // the fractional sites' targets, formed on the first pass at this K
     ObjTargets T{};
@@ -847,9 +856,7 @@ int objective_sums(nntc_b200_device* d, int k, std::vector<double>& acc, double*
         NB_LAUNCHED();
         k_objective_reduce<<<dim3(P.n, 3), 256, 0, d->stream>>>(P, d->obj_partial, nblocks, sums, bthreads);
         NB_LAUNCHED();
-        NB_TRY(block_end(d, ms));
-        acc.assign((size_t)3 * P.n, 0.0);
-        return download(d, acc.data(), sums, acc.size() * sizeof(double));
+        return fetch_sums();
     }
     NB_TRY(ktimer_begin(d, NNTC_B200_K_OBJECTIVE));
     switch (nout)
@@ -867,9 +874,7 @@ int objective_sums(nntc_b200_device* d, int k, std::vector<double>& acc, double*
     NB_LAUNCHED();
     k_objective_reduce<<<dim3(P.n, 3), 256, 0, d->stream>>>(P, d->obj_partial, nblocks, sums, bthreads);
     NB_LAUNCHED();
-    NB_TRY(block_end(d, ms));
-    acc.assign((size_t)3 * P.n, 0.0);
-    return download(d, acc.data(), sums, acc.size() * sizeof(double));
+    return fetch_sums();
 }
 
 }   // namespace nb

@@ -710,10 +710,11 @@ int bc_refine_passes(nntc_b200_device* d, const nntc_b200_model* m, int passes, 
             NB_LAUNCHED();
         }
         double t = 0.0;
-        NB_TRY(block_end(d, &t));
+        NB_TRY(block_mark(d));
+        NB_TRY(fetch(d, FETCH_BC_STATS, d->bc_stats, (size_t)MAX_PLANES * 2 * sizeof(double)));
+        NB_TRY(block_finish(d, &t));
         total += t;
-        std::vector<double> stats((size_t)MAX_PLANES * 2);
-        NB_TRY(download(d, stats.data(), d->bc_stats, stats.size() * sizeof(double)));
+        const double* stats = fetched<double>(d, FETCH_BC_STATS);
         nntc_b200_bc_report r{};
         r.pass = pass + 1;
         r.ms = t;

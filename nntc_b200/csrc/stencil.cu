@@ -1776,7 +1776,7 @@ int assemble(nntc_b200_device* d, const nntc_b200_model* m, int k, double ridge,
     }
     std::vector<double> mono;
     build_monomials(*m, level0, mono);
-    NB_TRY(upload(d, d->mono[level0], mono.data(), mono.size() * sizeof(double)));
+    NB_TRY(upload_small(d, d->mono[level0], mono.data(), mono.size() * sizeof(double)));
     Planes P = texel_planes(d, level0, k);
     const int nmono = monomial_count(level0 ? d->c1 : d->c0);
     const int blocks = (int)(P.start[P.n] / ASM_THREADS);
@@ -1920,11 +1920,9 @@ int solve_block(nntc_b200_device* d, const nntc_b200_model* m, int k, double rid
         NB_LAUNCHED();
         if ((it + 1) % CG_PROBE != 0)
             continue;
-        unsigned int still = 0;
-        NB_CUDA(cudaMemcpyAsync(&still, active + (it % CG_PROBE), sizeof(unsigned int), cudaMemcpyDeviceToHost,
-                                d->stream));
+        NB_TRY(fetch(d, FETCH_ACTIVE, active + (it % CG_PROBE), sizeof(unsigned int)));
         NB_CUDA(cudaStreamSynchronize(d->stream));
-        if (still == 0)
+        if (*fetched<unsigned int>(d, FETCH_ACTIVE) == 0)
             break;
     }
     k_correct_range<<<tblocks, THREADS, 0, d->stream>>>(P, R);
