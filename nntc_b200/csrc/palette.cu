@@ -10,12 +10,17 @@
 // strict decrease to move. Four colour passes ((x & 1, y & 1) classes) make the texels of one pass independent.
 //
 // Shape on the B200: ONE WARP PER TEXEL. The texel's candidate sites (9 pixels x (K + 1) site slots, at most 45) are
-// spread over the lanes, each lane forming its site's residual and slope columns and the site's contributions to the
-// quadratic; the contributions are then folded one coefficient per lane, in site order, through shared memory; and the
-// palette states (at most 256 in a joint enumeration, one channel's alphabet in a sweep) are spread over the lanes and
-// reduced by a warp argmin whose tie rule (lowest energy, then first state in enumeration order, the current state
+// spread over the lanes, which first only ask whether a tap reaches the texel; the sites that do (17 of 45 away from
+// the edges) are packed in site order, so that forming a site's residual, slope columns and contributions is one turn
+// of the warp. The contributions are then folded one coefficient per lane, in site order, through shared memory; and
+// the palette states (at most 256 in a joint enumeration, one channel's alphabet in a sweep) are spread over the lanes
+// and reduced by a warp argmin whose tie rule (lowest energy, then first state in enumeration order, the current state
 // before all) is the sequential scan's. The warp design keeps each lane's state to one site, where a thread-per-texel
 // kernel carries the whole 37-site walk and a 256-state loop in one thread.
+//
+// A small texture's colour is one wave of warps, so the time is one warp's chain of dependent steps. The channel
+// counts are template arguments: with them at run time every per-channel array lay in local memory and each state of
+// the enumeration cost a pair of integer divisions: 66.0 us a colour of a 100 x 76 texture (c0 = 2, c1 = 4), 13.3 now.
 //
 // What has to match the reference bit for bit, and why: the moved texels are bytes (level 0's indices), and a state's
 // energy can tie another's to the last bit, so the float arithmetic of a site (sample, decode slope and residual, in
@@ -36,7 +41,6 @@ namespace nb
 
 constexpr int PS_WARPS = 2;                      // texels (warps) per block
 constexpr int PS_CANDIDATES = 9 * 5;             // 3x3 pixels x (K + 1) site slots at K = 4
-constexpr int PS_COEFFS = MAX_CH + MAX_CH * MAX_CH;   // a1 then a2, row-major
 
 struct SearchArgs
 {
@@ -50,26 +54,31 @@ struct SearchArgs
     int colour;
 };
 
-// One warp's staging: per candidate site, whether it contributes, its a0 terms (one per output, added one by one in
-// output order) and its a1 / a2 contributions (alpha g_i, alpha^2 s_ij).
+// One warp's staging, rows over the live sites in order: their candidate numbers, their a0 terms (one per output, added
+// one by one in output order) and their a1 / a2 contributions (alpha g_i, alpha^2 s_ij). Site-contiguous rows, an odd
+// number of doubles apart: the lanes write a row side by side and the fold's lanes read a column without conflicts.
+template <int C0>
 struct SearchStage
 {
-    double a0t[PS_CANDIDATES][MAX_NOUT];
-    double coef[PS_CANDIDATES][PS_COEFFS];
-    int live[PS_CANDIDATES];
-    double q[1 + PS_COEFFS];   // the folded quadratic: a0, a1, a2
+    double a0t[MAX_NOUT][PS_CANDIDATES];
+    double coef[C0 + C0 * C0][PS_CANDIDATES];
+    double q[1 + C0 + C0 * C0];   // the folded quadratic: a0, a1, a2 (row-major)
+    unsigned char site[PS_CANDIDATES];
 };
 
 // The energy of a state x: a0, then channel by channel the linear term and the channel's row of the quadratic term.
-__device__ __forceinline__ double state_energy(const double* q, const float* x, int c0)
+template <int C0>
+__device__ __forceinline__ double state_energy(const double (&q)[1 + C0 + C0 * C0], const float (&x)[C0])
 {
     double e = q[0];
-    for (int i = 0; i < c0; i++)
+#pragma unroll
+    for (int i = 0; i < C0; i++)
     {
         const double xi = (double)x[i];
         e += 2.0 * xi * q[1 + i];
-        for (int j = 0; j < c0; j++)
-            e += xi * (double)x[j] * q[1 + MAX_CH + i * MAX_CH + j];
+#pragma unroll
+        for (int j = 0; j < C0; j++)
+            e += xi * (double)x[j] * q[1 + C0 + i * C0 + j];
     }
     return e;
 }
@@ -91,98 +100,151 @@ __device__ __forceinline__ void warp_argmin(double& e, int& n)
 }
 
 // Candidate `cand` of texel (tx, ty): pixel (tx + ox, ty + oy) with ox, oy in -1..1 and site slot j; only the texel's
-// own pixel has a centre site (j = 0). Writes the candidate's staging row; `live` says whether it contributes.
-__device__ void search_site(const Planes& P, const PlaneView& V, const SearchArgs& A, int tx, int ty, int cand,
-                            SearchStage& S)
+// own pixel has a centre site (j = 0).
+struct SearchSite
 {
-    const int c0 = P.c0, c1 = P.c1, nin = P.nin, nout = P.nout, kc = P.kc, w0 = V.w0, h0 = V.h0;
-    const int slot = cand % (kc + 1), pix = cand / (kc + 1);
-    const int px = tx + pix % 3 - 1, py = ty + pix / 3 - 1;
-    const bool own = pix == 4;
-    int live = pix < 9 && px >= 0 && py >= 0 && px < w0 && py < h0 && (slot > 0 || own);
-    float alpha = 0.0f, beta[MAX_CH] = { 0.0f, 0.0f, 0.0f, 0.0f }, cbar[MAX_CH], target[MAX_NOUT];
-    if (live)
+    int px, py, slot;
+    float dx, dy;
+};
+
+__device__ __forceinline__ SearchSite search_site(int kc, int tx, int ty, int cand)
+{
+    SearchSite s;
+    const int pix = cand / (kc + 1);
+    s.slot = cand % (kc + 1);
+    s.px = tx + pix % 3 - 1;
+    s.py = ty + pix / 3 - 1;
+    site_offset(kc, s.slot, s.px, s.py, s.dx, s.dy);
+    return s;
+}
+
+// The weight with which a fractional site's level-0 taps reach the texel: a tap the clamp folded onto it adds its own.
+__device__ __forceinline__ float tap_reach(const Tap& t, const float (&wt)[4], int tx, int ty)
+{
+    float alpha = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+        if (((q & 1) ? t.x1 : t.x0) == tx && ((q & 2) ? t.y1 : t.y0) == ty)
+            alpha += wt[q];
+    return alpha;
+}
+
+// Whether the candidate contributes.
+__device__ __forceinline__ bool search_live(const PlaneView& V, int kc, int tx, int ty, int cand)
+{
+    const SearchSite s = search_site(kc, tx, ty, cand);
+    if (s.px < 0 || s.py < 0 || s.px >= V.w0 || s.py >= V.h0)
+        return false;
+    if (s.slot == 0)
+        return s.px == tx && s.py == ty;
+    const Tap t = tap_at(s.px, s.py, s.dx, s.dy, V.w0, V.h0, V.w0, V.h0);
+    float wt[4];
+    tap_weights(t, wt);
+    return tap_reach(t, wt, tx, ty) > 0.0f;
+}
+
+// Live candidate `cand`'s staging column `at`.
+template <int C0, int C1>
+__device__ __forceinline__ void search_terms(const PlaneView& V, const SearchArgs& A, int kc, int nout, int tx, int ty,
+                                             int cand, int at, SearchStage<C0>& S)
+{
+    constexpr int NIN = C1 + C0 + C0 * C1;
+    const int w0 = V.w0, h0 = V.h0;
+    const SearchSite s = search_site(kc, tx, ty, cand);
+    float alpha = 1.0f, beta[C0], cbar[C1], wt[4] = { 1.0f, 0.0f, 0.0f, 0.0f };
+#pragma unroll
+    for (int i = 0; i < C0; i++)
+        beta[i] = 0.0f;
+    blend_c<C1>(V.v1, V.w1, tap_at(s.px, s.py, s.dx, s.dy, w0, h0, V.w1, V.h1), cbar);
+    // slot 0 reads level 0 nearest: its sample is the texel itself
+    size_t tap[4];
+    if (s.slot == 0)
     {
-        float dx, dy;
-        site_offset(kc, slot, px, py, dx, dy);
-        blend<MAX_CH>(V.v1, V.w1, c1, tap_at(px, py, dx, dy, w0, h0, V.w1, V.h1), cbar);
-        if (slot == 0)
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            tap[q] = (size_t)ty * w0 + tx;
+    }
+    else
+    {
+        const Tap t = tap_at(s.px, s.py, s.dx, s.dy, w0, h0, w0, h0);
+        tap_weights(t, wt);
+        alpha = tap_reach(t, wt, tx, ty);
+#pragma unroll
+        for (int q = 0; q < 4; q++)
         {
-            // level 0 read nearest: the site's sample is the texel itself
-            alpha = 1.0f;
-            const float* s = V.src + ((size_t)ty * w0 + tx) * nout;
-            for (int r = 0; r < nout; r++)
-                target[r] = s[r];
-        }
-        else
-        {
-            const Tap t0 = tap_at(px, py, dx, dy, w0, h0, w0, h0);
-            blend<MAX_NOUT>(V.src, w0, nout, t0, target);
-            float wt[4];
-            tap_weights(t0, wt);
-            for (int q = 0; q < 4; q++)
+            const int qx = (q & 1) ? t.x1 : t.x0, qy = (q & 2) ? t.y1 : t.y0;
+            tap[q] = (size_t)qy * w0 + qx;
+            if (qx != tx || qy != ty)
             {
-                const int qx = (q & 1) ? t0.x1 : t0.x0, qy = (q & 2) ? t0.y1 : t0.y0;
-                if (qx == tx && qy == ty)
-                    alpha += wt[q];   // a tap the clamp folded onto the texel adds its weight
-                else
-                {
-                    const float* nv = V.v0 + ((size_t)qy * w0 + qx) * c0;
-                    for (int i = 0; i < c0; i++)
-                        beta[i] += wt[q] * nv[i];
-                }
+                const float* nv = V.v0 + tap[q] * C0;
+#pragma unroll
+                for (int i = 0; i < C0; i++)
+                    beta[i] += wt[q] * nv[i];
             }
-            live = alpha > 0.0f;
         }
     }
-    S.live[cand] = live;
-    if (!live)
-        return;
     // output by output: the decode's slope in each channel of the texel at this site (the s-columns of W plus the
     // sc-columns weighted by cbar), the decode with the texel at zero, the residual, and the double products
-    double g[MAX_CH] = { 0.0, 0.0, 0.0, 0.0 }, s2[MAX_CH * MAX_CH];
-    for (int e = 0; e < MAX_CH * MAX_CH; e++)
+    double g[C0], s2[C0 * C0];
+#pragma unroll
+    for (int i = 0; i < C0; i++)
+        g[i] = 0.0;
+#pragma unroll
+    for (int e = 0; e < C0 * C0; e++)
         s2[e] = 0.0;
+#pragma unroll 3
     for (int r = 0; r < nout; r++)
     {
-        const float* wr = A.weights + (size_t)r * nin;
-        float dec = A.bias[r];
-        for (int q = 0; q < c1; q++)
-            dec += wr[q] * cbar[q];
-        float slope[MAX_CH];
-        for (int i = 0; i < c0; i++)
+        float target = __ldg(V.src + tap[0] * nout + r);
+        if (s.slot != 0)
+            target = wt[0] * target + wt[1] * __ldg(V.src + tap[1] * nout + r) + wt[2] * __ldg(V.src + tap[2] * nout + r) +
+                     wt[3] * __ldg(V.src + tap[3] * nout + r);
+        const float* wr = A.weights + r * NIN;
+        float dec = __ldg(A.bias + r);
+#pragma unroll
+        for (int q = 0; q < C1; q++)
+            dec += __ldg(wr + q) * cbar[q];
+        float slope[C0];
+#pragma unroll
+        for (int i = 0; i < C0; i++)
         {
-            float sl = wr[c1 + i];
-            for (int q = 0; q < c1; q++)
-                sl += wr[c1 + c0 + i * c1 + q] * cbar[q];
+            float sl = __ldg(wr + C1 + i);
+#pragma unroll
+            for (int q = 0; q < C1; q++)
+                sl += __ldg(wr + C1 + C0 + i * C1 + q) * cbar[q];
             slope[i] = sl;
             dec += sl * beta[i];
         }
-        const double res = (double)(dec - target[r]);
-        const double wgt = (double)A.cw[r];
-        S.a0t[cand][r] = wgt * res * res;
-        for (int i = 0; i < c0; i++)
+        const double res = (double)(dec - target);
+        const double wgt = (double)__ldg(A.cw + r);
+        S.a0t[r][at] = wgt * res * res;
+#pragma unroll
+        for (int i = 0; i < C0; i++)
         {
             const double wq = wgt * (double)slope[i];
             g[i] += wq * res;
-            for (int j = 0; j < c0; j++)
-                s2[i * MAX_CH + j] += wq * (double)slope[j];
+#pragma unroll
+            for (int j = 0; j < C0; j++)
+                s2[i * C0 + j] += wq * (double)slope[j];
         }
     }
     const double al = (double)alpha;
-    for (int i = 0; i < c0; i++)
+#pragma unroll
+    for (int i = 0; i < C0; i++)
     {
-        S.coef[cand][i] = al * g[i];
-        for (int j = 0; j < c0; j++)
-            S.coef[cand][MAX_CH + i * MAX_CH + j] = al * al * s2[i * MAX_CH + j];
+        S.coef[i][at] = al * g[i];
+#pragma unroll
+        for (int j = 0; j < C0; j++)
+            S.coef[C0 + i * C0 + j][at] = al * al * s2[i * C0 + j];
     }
 }
 
+template <int C0, int C1>
 __global__ void __launch_bounds__(32 * PS_WARPS) k_palette_search(Planes P, SearchArgs A)
 {
-    __shared__ SearchStage stage[PS_WARPS];
+    __shared__ SearchStage<C0> stage[PS_WARPS];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    SearchStage& S = stage[wid];
+    SearchStage<C0>& S = stage[wid];
     const long long item = (long long)blockIdx.x * PS_WARPS + wid;   // the texel of this pass, over every plane
     const int pl = plane_of(P, item);
     const PlaneView& V = P.p[pl];
@@ -190,71 +252,83 @@ __global__ void __launch_bounds__(32 * PS_WARPS) k_palette_search(Planes P, Sear
     const int cw0 = (V.w0 - A.cx + 1) / 2, ch0 = (V.h0 - A.cy + 1) / 2;
     if (ci >= (long long)cw0 * ch0)
         return;   // the whole warp leaves together
-    const int c0 = P.c0;
-    const int tx = A.cx + 2 * (int)(ci % cw0), ty = A.cy + 2 * (int)(ci / cw0);
+    const int row = (int)(ci / cw0);
+    const int tx = A.cx + 2 * (int)(ci - (long long)row * cw0), ty = A.cy + 2 * row;
     const size_t t = (size_t)ty * V.w0 + tx;
-    const int ncand = 9 * (P.kc + 1);
+    const int ncand = 9 * (P.kc + 1), nout = P.nout;
 
-    for (int cand = lane; cand < ncand; cand += 32)
-        search_site(P, V, A, tx, ty, cand, S);
+    int nlive = 0;
+    for (int first = 0; first < ncand; first += 32)
+    {
+        const int cand = first + lane;
+        const bool live = cand < ncand && search_live(V, P.kc, tx, ty, cand);
+        const unsigned mask = __ballot_sync(0xffffffffu, live);
+        if (live)
+            S.site[nlive + __popc(mask & ((1u << lane) - 1u))] = (unsigned char)cand;
+        nlive += __popc(mask);
+    }
+    __syncwarp();
+    for (int at = lane; at < nlive; at += 32)
+        search_terms<C0, C1>(V, A, P.kc, nout, tx, ty, S.site[at], at, S);
     __syncwarp();
     // the fold: one coefficient per lane over the live sites in order; the last lane walks a0's terms
-    if (lane < PS_COEFFS)
+    if (lane < C0 + C0 * C0)
     {
-        const int i = lane < MAX_CH ? lane : (lane - MAX_CH) / MAX_CH, j = lane < MAX_CH ? 0 : (lane - MAX_CH) % MAX_CH;
-        if (i < c0 && j < c0)
-        {
-            double acc = 0.0;
-            for (int cand = 0; cand < ncand; cand++)
-                if (S.live[cand])
-                    acc += S.coef[cand][lane];
-            S.q[1 + lane] = acc;
-        }
+        double acc = 0.0;
+#pragma unroll 4
+        for (int at = 0; at < nlive; at++)
+            acc += S.coef[lane][at];
+        S.q[1 + lane] = acc;
     }
     else if (lane == 31)
     {
         double acc = 0.0;
-        for (int cand = 0; cand < ncand; cand++)
-            if (S.live[cand])
-                for (int r = 0; r < P.nout; r++)
-                    acc += S.a0t[cand][r];
+        for (int at = 0; at < nlive; at++)
+#pragma unroll 3
+            for (int r = 0; r < nout; r++)
+                acc += S.a0t[r][at];
         S.q[0] = acc;
     }
     __syncwarp();
 
-    int levels[MAX_CH], cur[MAX_CH], best[MAX_CH];
-    float x[MAX_CH];
-    for (int i = 0; i < c0; i++)
+    double q[1 + C0 + C0 * C0];
+#pragma unroll
+    for (int e = 0; e < 1 + C0 + C0 * C0; e++)
+        q[e] = S.q[e];
+    int cur[C0], best[C0];
+    float x[C0];
+#pragma unroll
+    for (int i = 0; i < C0; i++)
     {
-        levels[i] = (1 << A.bits[i]) - 1;
-        cur[i] = best[i] = (int)V.k0[t * c0 + i];
+        cur[i] = best[i] = (int)V.k0[t * C0 + i];
         x[i] = A.palette[i * 16 + cur[i]];
     }
-    double best_e = state_energy(S.q, x, c0);
+    double best_e = state_energy<C0>(q, x);
     if (A.joint)
     {
-        // mixed radix, channel 0 fastest; the current state stays unless something is strictly lower
-        int total = 1, cur_n = 0, stride = 1;
-        for (int i = 0; i < c0; i++)
+        // mixed radix of powers of two, channel 0 fastest; the current state stays unless something is strictly lower
+        int cur_n = 0, bits = 0;
+#pragma unroll
+        for (int i = 0; i < C0; i++)
         {
-            cur_n += cur[i] * stride;
-            stride *= levels[i] + 1;
+            cur_n += cur[i] << bits;
+            bits += A.bits[i];
         }
-        total = stride;
+        const int total = 1 << bits;
         double e_min = DBL_MAX;
         int n_min = INT_MAX;
+#pragma unroll 2
         for (int n = lane; n < total; n += 32)
         {
-            if (n == cur_n)
-                continue;
             int rest = n;
-            for (int i = 0; i < c0; i++)
+#pragma unroll
+            for (int i = 0; i < C0; i++)
             {
-                x[i] = A.palette[i * 16 + rest % (levels[i] + 1)];
-                rest /= levels[i] + 1;
+                x[i] = __ldg(A.palette + i * 16 + (rest & ((1 << A.bits[i]) - 1)));
+                rest >>= A.bits[i];
             }
-            const double e = state_energy(S.q, x, c0);
-            if (e < e_min)
+            const double e = state_energy<C0>(q, x);
+            if (n != cur_n && e < e_min)
             {
                 e_min = e;
                 n_min = n;
@@ -264,10 +338,11 @@ __global__ void __launch_bounds__(32 * PS_WARPS) k_palette_search(Planes P, Sear
         if (n_min != INT_MAX && e_min < best_e)
         {
             int rest = n_min;
-            for (int i = 0; i < c0; i++)
+#pragma unroll
+            for (int i = 0; i < C0; i++)
             {
-                best[i] = rest % (levels[i] + 1);
-                rest /= levels[i] + 1;
+                best[i] = rest & ((1 << A.bits[i]) - 1);
+                rest >>= A.bits[i];
             }
         }
     }
@@ -276,18 +351,20 @@ __global__ void __launch_bounds__(32 * PS_WARPS) k_palette_search(Planes P, Sear
         for (int sw = 0; sw < A.sweeps; sw++)
         {
             bool changed = false;
-            for (int i = 0; i < c0; i++)
+#pragma unroll
+            for (int i = 0; i < C0; i++)
             {
-                for (int q = 0; q < c0; q++)
-                    x[q] = A.palette[q * 16 + best[q]];
+#pragma unroll
+                for (int c = 0; c < C0; c++)
+                    x[c] = A.palette[c * 16 + best[c]];
                 double e_min = DBL_MAX;
                 int k_min = INT_MAX;
-                for (int k = lane; k <= levels[i]; k += 32)
+                for (int k = lane; k < 1 << A.bits[i]; k += 32)
                 {
                     if (k == best[i])
                         continue;
                     x[i] = A.palette[i * 16 + k];
-                    const double e = state_energy(S.q, x, c0);
+                    const double e = state_energy<C0>(q, x);
                     if (e < e_min)
                     {
                         e_min = e;
@@ -307,16 +384,32 @@ __global__ void __launch_bounds__(32 * PS_WARPS) k_palette_search(Planes P, Sear
         }
     }
     bool moved = false;
-    for (int i = 0; i < c0; i++)
+#pragma unroll
+    for (int i = 0; i < C0; i++)
         moved = moved || best[i] != cur[i];
     if (moved && lane == 0)
     {
-        for (int i = 0; i < c0; i++)
+#pragma unroll
+        for (int i = 0; i < C0; i++)
         {
-            V.v0[t * c0 + i] = A.palette[i * 16 + best[i]];
-            V.k0[t * c0 + i] = (uint8_t)best[i];
+            V.v0[t * C0 + i] = A.palette[i * 16 + best[i]];
+            V.k0[t * C0 + i] = (uint8_t)best[i];
         }
         atomicAdd(A.moved + pl * 4 + A.colour, 1u);
+    }
+}
+
+template <int C0>
+static void launch_palette_search(const Planes& P, const SearchArgs& A, cudaStream_t stream)
+{
+    // one warp per texel; planes_for pads each plane's range to THREADS texels, a multiple of PS_WARPS
+    const unsigned blocks = (unsigned)(P.start[P.n] / PS_WARPS);
+    switch (P.c1)
+    {
+    case 1: k_palette_search<C0, 1><<<blocks, 32 * PS_WARPS, 0, stream>>>(P, A); break;
+    case 2: k_palette_search<C0, 2><<<blocks, 32 * PS_WARPS, 0, stream>>>(P, A); break;
+    case 3: k_palette_search<C0, 3><<<blocks, 32 * PS_WARPS, 0, stream>>>(P, A); break;
+    default: k_palette_search<C0, 4><<<blocks, 32 * PS_WARPS, 0, stream>>>(P, A); break;
     }
 }
 
@@ -367,8 +460,13 @@ int nntc_b200_solve_level0_all(nntc_b200_device* d, const nntc_b200_model* m, in
         A.cx = cx;
         A.cy = cy;
         A.colour = colour;
-        // one warp per texel; planes_for pads each plane's range to THREADS texels, a multiple of PS_WARPS
-        k_palette_search<<<(unsigned)(P.start[P.n] / PS_WARPS), 32 * PS_WARPS, 0, d->stream>>>(P, A);
+        switch (d->c0)
+        {
+        case 1: launch_palette_search<1>(P, A, d->stream); break;
+        case 2: launch_palette_search<2>(P, A, d->stream); break;
+        case 3: launch_palette_search<3>(P, A, d->stream); break;
+        default: launch_palette_search<4>(P, A, d->stream); break;
+        }
         NB_LAUNCHED();
     }
     double t = 0.0;
