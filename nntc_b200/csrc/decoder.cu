@@ -368,7 +368,9 @@ int normal_equations(nntc_b200_device* d, int k, const double* per_site, double*
 // ---- the solve, on the device ---------------------------------------------------------------------------------------
 //
 // The system is tiny (mm <= 25 unknowns, nout <= 18 right-hand sides), so one block of 128 threads does all of it in
-// shared memory, with no host round trip between the accumulation and the decision:
+// shared memory, with no host round trip between the accumulation and the decision. Its time is its chains of dependent
+// FP64 operations: 35.4 us at 9 unknowns and 3 outputs with three barriers a column of the factor and an output's
+// quadratic on one thread, 29.5 with one barrier and a thread a row, the divisions of the substitutions what is left:
 //
 //   for each ridge r of the ladder {1e-9, 1e-12, 0} x mean(diag A), until one is accepted:
 //     L L^T = A + r I                       FP64 Cholesky, right-looking, a non-positive or non-finite pivot refuses
@@ -389,6 +391,7 @@ int normal_equations(nntc_b200_device* d, int k, const double* per_site, double*
 
 constexpr int DS_THREADS = 128;
 constexpr int DS_MM = MAX_NIN + 1;
+static_assert(DS_MM <= 32, "a row of the factor a lane");
 
 struct DecoderSolveArgs
 {
@@ -411,24 +414,35 @@ struct DecoderSolveOut
 };
 
 // The quadratic and its rounding bound at the solution rows X (shared), in E's units for the bound. Every thread
-// calls it; thread c < nout forms output c's terms, thread 0 adds the outputs in index order.
+// calls it: a thread an (output, row) forms the row's two sums into T and U, thread c < nout adds output c's rows,
+// thread 0 the outputs, each in index order.
 __device__ void ds_quadratic(const double (*A)[DS_MM + 1], const double (*R)[DS_MM], const double (*X)[DS_MM],
-                             const DecoderSolveArgs& a, int mm, double* qc, double* ec, double& q, double& err)
+                             double (*T)[DS_MM], double (*U)[DS_MM], const DecoderSolveArgs& a, int mm, double* qc,
+                             double* ec, double& q, double& err)
 {
-    const int c = threadIdx.x;
-    if (c < a.nout)
+    for (int e = threadIdx.x; e < a.nout * mm; e += DS_THREADS)
     {
+        const int c = e / mm, i = e % mm;
+        double ax = 0.0, aax = 0.0;
+#pragma unroll 8
+        for (int j = 0; j < mm; j++)
+        {
+            ax = fma(A[i][j], X[c][j], ax);
+            aax = fma(fabs(A[i][j]), fabs(X[c][j]), aax);
+        }
+        T[c][i] = ax - 2.0 * R[c][i];
+        U[c][i] = aax + 2.0 * fabs(R[c][i]);
+    }
+    __syncthreads();
+    if (threadIdx.x < a.nout)
+    {
+        const int c = threadIdx.x;
         double qs = 0.0, es = 0.0;
+#pragma unroll 8
         for (int i = 0; i < mm; i++)
         {
-            double ax = 0.0, aax = 0.0;
-            for (int j = 0; j < mm; j++)
-            {
-                ax = fma(A[i][j], X[c][j], ax);
-                aax = fma(fabs(A[i][j]), fabs(X[c][j]), aax);
-            }
-            qs = fma(X[c][i], ax - 2.0 * R[c][i], qs);
-            es = fma(fabs(X[c][i]), aax + 2.0 * fabs(R[c][i]), es);
+            qs = fma(X[c][i], T[c][i], qs);
+            es = fma(fabs(X[c][i]), U[c][i], es);
         }
         qc[c] = qs;
         ec[c] = es;
@@ -437,6 +451,7 @@ __device__ void ds_quadratic(const double (*A)[DS_MM + 1], const double (*R)[DS_
     if (threadIdx.x == 0)
     {
         double qt = 0.0, et = 0.0;
+#pragma unroll 6
         for (int o = 0; o < a.nout; o++)
         {
             qt += (double)a.cw[o] * qc[o];
@@ -448,19 +463,23 @@ __device__ void ds_quadratic(const double (*A)[DS_MM + 1], const double (*R)[DS_
     __syncthreads();
 }
 
-// Solve (L L^T) y = rhs in place for output row c (one thread).
+// Solve (L L^T) y = rhs in place for output row c (one thread). Both take a row's terms in ascending order: forward, a
+// solved unknown leaves every later row at once (independent sums); backward, that order is one chain, its operands
+// loaded ahead of it.
 __device__ void ds_substitute(const double (*L)[DS_MM + 1], double* y, int mm)
 {
-    for (int i = 0; i < mm; i++)
+    for (int j = 0; j < mm; j++)
     {
-        double s = y[i];
-        for (int j = 0; j < i; j++)
-            s = fma(-L[i][j], y[j], s);
-        y[i] = s / L[i][i];
+        const double v = y[j] / L[j][j];
+        y[j] = v;
+#pragma unroll 8
+        for (int i = j + 1; i < mm; i++)
+            y[i] = fma(-L[i][j], v, y[i]);
     }
     for (int i = mm - 1; i >= 0; i--)
     {
         double s = y[i];
+#pragma unroll 8
         for (int j = i + 1; j < mm; j++)
             s = fma(-L[j][i], y[j], s);
         y[i] = s / L[i][i];
@@ -471,10 +490,11 @@ __global__ void __launch_bounds__(DS_THREADS) k_decoder_solve(const double* __re
                                                                DecoderSolveOut* out)
 {
     __shared__ double A[DS_MM][DS_MM + 1], L[DS_MM][DS_MM + 1];
-    __shared__ double R[MAX_NOUT][DS_MM], X[MAX_NOUT][DS_MM], D[MAX_NOUT][DS_MM];
+    __shared__ double F[DS_MM][DS_MM + 1];   // the factor: L is what is left to eliminate
+    __shared__ double R[MAX_NOUT][DS_MM], X[MAX_NOUT][DS_MM], D[MAX_NOUT][DS_MM], U[MAX_NOUT][DS_MM];
     __shared__ double qc[MAX_NOUT], ec[MAX_NOUT];
     __shared__ double q_prev, err_prev, q_new, err_new, mean_diag;
-    __shared__ int refused, accepted;
+    __shared__ int accepted;
     const int tid = threadIdx.x, nin = a.nin, nout = a.nout, mm = nin + 1;
     const int tri = mm * (mm + 1) / 2;
 
@@ -503,7 +523,7 @@ __global__ void __launch_bounds__(DS_THREADS) k_decoder_solve(const double* __re
     }
     __syncthreads();
     if (a.had_previous)
-        ds_quadratic(A, R, X, a, mm, qc, ec, q_prev, err_prev);
+        ds_quadratic(A, R, X, D, U, a, mm, qc, ec, q_prev, err_prev);
 
     const double ladder[3] = { 1e-9, 1e-12, 0.0 };
     for (int rung = 0; rung < 3; rung++)
@@ -514,43 +534,48 @@ __global__ void __launch_bounds__(DS_THREADS) k_decoder_solve(const double* __re
             const int i = e / mm, j = e % mm;
             L[i][j] = i == j ? A[i][j] + ridge : A[i][j];
         }
-        if (tid == 0)
-            refused = 0;
         __syncthreads();
-        // right-looking Cholesky on the lower triangle
+        // right-looking Cholesky on the lower triangle, one barrier a column: every warp takes the pivot's root and the
+        // column's quotients for itself (a row a lane), then updates its own rows
+        bool refused = false;
         for (int k = 0; k < mm; k++)
         {
-            if (tid == 0)
+            const double p = L[k][k];
+            if (!(p > 0.0 && isfinite(p)))
             {
-                const double p = L[k][k];
-                if (p > 0.0 && isfinite(p))
-                    L[k][k] = sqrt(p);
-                else
-                    refused = 1;
-            }
-            __syncthreads();
-            if (refused)
+                refused = true;   // (every thread alike)
                 break;
-            for (int i = k + 1 + tid; i < mm; i += DS_THREADS)
-                L[i][k] /= L[k][k];
-            __syncthreads();
-            const int n = mm - k - 1;
-            for (int e = tid; e < n * n; e += DS_THREADS)
+            }
+            const double root = sqrt(p);
+            const int lane = tid & 31, warp = tid >> 5, n = mm - k - 1;
+            const double l = lane < n ? L[k + 1 + lane][k] / root : 0.0;
+            if (warp == 0)
             {
-                const int i = k + 1 + e / n, j = k + 1 + e % n;
-                if (j <= i)
-                    L[i][j] = fma(-L[i][k], L[j][k], L[i][j]);
+                if (lane < n)
+                    F[k + 1 + lane][k] = l;
+                else if (lane == n)
+                    F[k][k] = root;
+            }
+#pragma unroll 4
+            for (int i = warp; i < n; i += DS_THREADS / 32)
+            {
+                const double li = __shfl_sync(0xffffffffu, l, i);
+                if (lane <= i)
+                    L[k + 1 + i][k + 1 + lane] = fma(-li, l, L[k + 1 + i][k + 1 + lane]);
             }
             __syncthreads();
         }
         if (refused)
+        {
+            __syncthreads();   // the pivot read before the next rung writes L
             continue;
+        }
         // solve, then one refinement step against A + ridge I
         if (tid < nout)
         {
             for (int i = 0; i < mm; i++)
                 D[tid][i] = R[tid][i];
-            ds_substitute(L, D[tid], mm);
+            ds_substitute(F, D[tid], mm);
         }
         __syncthreads();
         for (int e = tid; e < nout * mm; e += DS_THREADS)
@@ -566,7 +591,7 @@ __global__ void __launch_bounds__(DS_THREADS) k_decoder_solve(const double* __re
         }
         __syncthreads();
         if (tid < nout)
-            ds_substitute(L, D[tid], mm);
+            ds_substitute(F, D[tid], mm);
         __syncthreads();
         int finite = 1;
         for (int e = tid; e < nout * mm; e += DS_THREADS)
@@ -578,7 +603,7 @@ __global__ void __launch_bounds__(DS_THREADS) k_decoder_solve(const double* __re
         }
         if (!__syncthreads_and(finite))
             continue;
-        ds_quadratic(A, R, X, a, mm, qc, ec, q_new, err_new);
+        ds_quadratic(A, R, X, D, U, a, mm, qc, ec, q_new, err_new);
         if (tid == 0 && (!a.had_previous ||
                          (a.norm_ok && (q_new - q_prev) * a.inv_norm + err_prev + err_new <= 1e-12)))
             accepted = rung;
