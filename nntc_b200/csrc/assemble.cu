@@ -15,8 +15,8 @@
 //   - the stencil's monomial sums need only the site's sample of the OTHER latent (a bilinear blend of four texels,
 //     which k_site_terms also stores per site) and the tap weights - a few dozen operations. They are gathered per
 //     (texel, slot): each slot's sums receive the same terms in the same site order as the reference's, so every sum,
-//     and the expansion against the monomial matrices after it, is the same bits. gather.cu does it in tiles; k_gather_walk below
-//     takes the few planes no tile fits.
+//     and the expansion against the monomial matrices after it, is the same bits. gather.cu does it in tiles;
+//     k_gather_walk below takes the few planes no tile fits.
 //
 // Every plane of the chain is in each launch (nb::Planes); the per-site buffer holds every plane's sites.
 

@@ -12,11 +12,13 @@
 // reference's. What differs is the B200 shape:
 //
 // - every plane of the chain in ONE launch (nb::Planes), one stream, no per-plane fan-out;
-// - the stencil stored structure-of-arrays [slot][i][j][texel], coalesced for a warp of consecutive texels;
-// - the gather's 5 x nmono monomial sums live in shared memory (registers spill at C = 4);
+// - the FP64 stencil stored structure-of-arrays [slot][i][j][texel], coalesced for a warp of consecutive texels, the FP32
+//   one by texel, whose kernels take a lane per row of a block;
+// - the assembly is assemble.cu's and gather.cu's; the reference-shaped one here, behind an option, keeps its 5 x nmono
+//   monomial sums in shared memory (registers spill at C = 4);
 // - the conjugate-gradient iteration is 5 launches (matvec + <p,Ap>, alpha, update + preconditioner + <r,r> +
-//   <r,z>, beta, direction) and nothing else instead of 13, all planes in lockstep, and the stop is decided ON THE DEVICE with the
-//   reference's rule (a plane leaves at an iteration that is a multiple of CG_PROBE once its residual is below the
+//   <r,z>, beta, direction) and nothing else instead of 13, all planes in lockstep, and the stop is decided ON THE
+//   DEVICE with the reference's rule (a plane leaves at an iteration that is a multiple of CG_PROBE once its residual is below the
 //   tolerance); the host reads one active-plane count every CG_PROBE iterations, the reference's probe cadence.
 // - every dot product is a fixed-order two-stage reduction: one partial per 256-texel block, added per plane in
 //   block order.
@@ -819,12 +821,13 @@ __global__ void __launch_bounds__(THREADS, 4) k_cg_matvec(Planes P, Red R)
         R.partial[blockIdx.x] = v[0];
 }
 
-// The product for an FP32 stencil of two or four channels with a lane per row: C lanes share a texel, lane i forms row i
-// of the product - the same sums in the same order - and reads row i of each of the nine blocks as one vector, so that a
-// warp's reads of a slot are contiguous runs. One thread per texel read each block's rows 64 bytes apart: the L1 served
-// the same line four times, and that bound the kernel (97% of its wavefronts; 627 us at 6 x 2048 x 2048, against 330 us
-// for its bytes; by rows 549 us, bound by the loads' latency: six blocks per SM, four take 690 us). A backward neighbour's transposed block is read by rows too where the blocks are symmetric bit for bit
-// (symmetric != 0), else by columns.
+// The product for an FP32 stencil of two or four channels with a lane per row (k_cg_matvec_rows): C lanes share a texel,
+// lane i forms row i of the product - the same sums in the same order - and reads row i of each of the nine blocks as one
+// vector, so that a warp's reads of a slot are contiguous runs. One thread per texel read each block's rows 64 bytes
+// apart: the L1 served the same line four times, and that bound the kernel (97% of its wavefronts; 627 us at 6 x 2048 x
+// 2048, against 330 us for its bytes; by rows 549 us, bound by the loads' latency: six blocks per SM, four take 690 us).
+// A backward neighbour's transposed block is read by rows too where the blocks are symmetric bit for bit (symmetric
+// != 0), else by columns. The FP64 stencil has a run per coefficient, which a thread per texel reads whole as it is.
 template <int C>
 __device__ __forceinline__ void load_row(const float* p, float (&r)[C])
 {
@@ -1878,28 +1881,35 @@ int solve_block(nntc_b200_device* d, const nntc_b200_model* m, int k, double rid
             NB_TRY(matvec_free(d, P, R.partial, level0));
         else
         {
-#define NB_MATVEC(TS)                                                                                                 \
-    switch (P.c)                                                                                                      \
-    {                                                                                                                 \
-    case 1: k_cg_matvec<1, TS><<<tblocks, THREADS, 0, d->stream>>>(P, R); break;                                      \
-    case 2: k_cg_matvec<2, TS><<<tblocks, THREADS, 0, d->stream>>>(P, R); break;                                      \
-    case 3: k_cg_matvec<3, TS><<<tblocks, THREADS, 0, d->stream>>>(P, R); break;                                      \
-    default: k_cg_matvec<4, TS><<<tblocks, THREADS, 0, d->stream>>>(P, R); break;                                     \
-    }
             const int symmetric = d->sten_symmetric[level0] ? 1 : 0;
-            if (d->sten_f32[level0] && P.c == 4)
-                k_cg_matvec_rows<4><<<tblocks, THREADS, 0, d->stream>>>(P, R, symmetric);
-            else if (d->sten_f32[level0] && P.c == 2)
-                k_cg_matvec_rows<2><<<tblocks, THREADS, 0, d->stream>>>(P, R, symmetric);
-            else if (d->sten_f32[level0])
+            const bool f32 = d->sten_f32[level0];
+            switch (P.c)
             {
-                NB_MATVEC(float)
+            case 1:
+                if (f32)
+                    k_cg_matvec<1, float><<<tblocks, THREADS, 0, d->stream>>>(P, R);
+                else
+                    k_cg_matvec<1, double><<<tblocks, THREADS, 0, d->stream>>>(P, R);
+                break;
+            case 2:
+                if (f32)
+                    k_cg_matvec_rows<2><<<tblocks, THREADS, 0, d->stream>>>(P, R, symmetric);
+                else
+                    k_cg_matvec<2, double><<<tblocks, THREADS, 0, d->stream>>>(P, R);
+                break;
+            case 3:
+                if (f32)
+                    k_cg_matvec<3, float><<<tblocks, THREADS, 0, d->stream>>>(P, R);
+                else
+                    k_cg_matvec<3, double><<<tblocks, THREADS, 0, d->stream>>>(P, R);
+                break;
+            default:
+                if (f32)
+                    k_cg_matvec_rows<4><<<tblocks, THREADS, 0, d->stream>>>(P, R, symmetric);
+                else
+                    k_cg_matvec<4, double><<<tblocks, THREADS, 0, d->stream>>>(P, R);
+                break;
             }
-            else
-            {
-                NB_MATVEC(double)
-            }
-#undef NB_MATVEC
             NB_LAUNCHED();
         }
         NB_TRY(ktimer_end(d));
