@@ -1323,8 +1323,20 @@ struct ColourArgs
 // FP32 stencil of two or four channels the couplings are formed a lane per row (neighbour_rows) and handed to the
 // texels' threads through shared memory, so that the stencil is read in whole lines; with an FP64 stencil (a plane of
 // doubles per coefficient) a thread per texel already reads whole lines. The texel's own values are whole vectors.
-template <int C, typename TS>
-__global__ void __launch_bounds__(THREADS) k_quant_colour(Planes P, ColourArgs A)
+// PER_SM: the blocks an SM is to hold, 0 for as many as the compiler's own choice of registers leaves (an explicit 1 lets
+// it take 202 in FP64 where it takes 64: 6.2 -> 8.1 ms for the sweeps of 4 x 2048 x 1024). Each block waits out the same chain of loads, so a launch takes its waves of blocks
+// times that: with an FP32 stencil of four channels about 21 us a wave at three blocks an SM (76 registers) and 27 at
+// four (64, 48 bytes spilled). colour_per_sm takes the one whose waves hold fewer blocks (us a launch, three against four:
+// 426 blocks 23.0 / 24.7, 583 blocks 41.7 / 30.7, 699 blocks 45.5 / 50.2, 984 blocks 65.8 / 57.7, 1365 blocks 83.0 / 79.4,
+// 1930 blocks 111.3 / 109.6, 2730 blocks 147.2 / 138.2; the line misses two in a hundred at 1930).
+constexpr int colour_per_sm(int blocks)
+{
+    constexpr int SMS = 148;
+    return 4 * ((blocks + 4 * SMS - 1) / (4 * SMS)) <= 3 * ((blocks + 3 * SMS - 1) / (3 * SMS)) ? 4 : 3;
+}
+
+template <int C, typename TS, int PER_SM = 0>
+__global__ void __launch_bounds__(THREADS, PER_SM) k_quant_colour(Planes P, ColourArgs A)
 {
     constexpr bool ROWS = sizeof(TS) == sizeof(float) && C % 2 == 0;
     __shared__ __align__(16) double coupling[ROWS ? THREADS * C : 1];
@@ -2034,7 +2046,12 @@ int sweep_block(nntc_b200_device* d, const nntc_b200_model* m, int k, double rid
     case 1: k_quant_colour<1, TS><<<sblocks, THREADS, 0, d->stream>>>(C, A); break;                                    \
     case 2: k_quant_colour<2, TS><<<sblocks, THREADS, 0, d->stream>>>(C, A); break;                                    \
     case 3: k_quant_colour<3, TS><<<sblocks, THREADS, 0, d->stream>>>(C, A); break;                                    \
-    default: k_quant_colour<4, TS><<<sblocks, THREADS, 0, d->stream>>>(C, A); break;                                   \
+    default:                                                                                                           \
+        if (sizeof(TS) == sizeof(float) && colour_per_sm(sblocks) == 4)                                                \
+            k_quant_colour<4, TS, sizeof(TS) == sizeof(float) ? 4 : 0><<<sblocks, THREADS, 0, d->stream>>>(C, A);      \
+        else                                                                                                           \
+            k_quant_colour<4, TS><<<sblocks, THREADS, 0, d->stream>>>(C, A);                                           \
+        break;                                                                                                         \
     }
             if (d->sten_f32[level0])
             {

@@ -87,6 +87,25 @@ def test_sweep_in_one_launch(c0, c1, w, h, mip_min, f32, sweeps):
                 assert np.array_equal(ws["x"], want), (level0, i)
 
 
+@pytest.mark.parametrize("w,h,weights", [(601, 611, "one"), (512, 750, "mixed"), (896, 600, "one")])
+def test_colour_launches_of_either_residency(w, h, weights):
+    """A colour of an FP32 stencil of four channels at about 480 and 500 blocks (four to an SM) and 700 (three), with symmetric
+    blocks and blocks that are not, against the same walk, bit for bit."""
+    mat = materials.small(w + h, w, h, textures=1, c0=4, c1=1)
+    rng = np.random.default_rng(w * h)
+    cw = None if weights == "one" else list(0.3 + rng.random(3))
+    with Session(mat, model=abi.make_model(mat, cw=cw)) as s:
+        check(lib().nntc_b200_set_option(s.d, abi.OPT_FP32_STENCIL, 1), "option")
+        for i, p in enumerate(mat.planes):
+            s.set_planes(i, rng.random(p[0] * p[1] * 4) * 2 - 1, rng.random(p[2] * p[3]) * 2 - 1)
+        s.set_decoder(rng.standard_normal((3, s.m.nin)) * 0.3, rng.random(3))
+        s.set_grids(np.full(4, -1.0), np.full(4, 1.0), np.full(1, -1.0), np.full(1, 1.0))
+        rep, _ = s.block(True, sweeps=1)
+        for i, p in enumerate(mat.planes):
+            ws = s.workspace(i, True)
+            assert np.array_equal(ws["x"], walk_sweeps(ws, p[0], p[1], 4, rep[i].lambda_, -1.0, 1.0, 1)), i
+
+
 def walk_sweeps(ws, w, h, c, lam, lo, hi, sweeps):
     S, g = ws["stencil"].reshape(h, w, 5, c, c), ws["grad"].reshape(h, w, c)
     prev = ws["prev"].reshape(h, w, c).astype(np.float64)
