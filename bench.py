@@ -475,42 +475,47 @@ def crop_gpu_mpix(L, crop, ea):
 _PIX3 = 2796160
 TRAFFIC_PER_UNIT = {
     "adjoint": {
-        "normal_equations": (723597056 + 8700928) / _PIX3,                    # k_ls_accumulate_tc<12>
-        "objective": (718641152 + 4395008) / _PIX3,                           # k_objective_f32<12>
-        "assemble_level0": (718829056 + 627887616 + 671188992 + 944002048) / _PIX3,
-        "assemble_level1": (718788608 + 627927552 + 885506560 + 71808000) / _PIX3,
-        "quant_sweep": (610947328 + 42693888) / _PIX3,                        # a level-0 colour launch
-        "bc_refine": (1279862000 + 43057664) / _PIX3,                         # one colour
+        "normal_equations": (719051776 + 6578688) / _PIX3,                    # k_ls_accumulate_tc<12>
+        "objective": (718720000 + 3744256) / _PIX3,                           # k_objective_f32<12>
+        "assemble_level0": (718749696 + 409025024 + 447635712 + 926419200) / _PIX3,
+        "assemble_level1": (718750976 + 409468672 + 447994880 + 54923520) / _PIX3,
+        "quant_sweep": (588385536 + 42799104) / _PIX3,                        # a level-0 colour launch
+        "bc_refine": (1288049408 + 55825920) / _PIX3,                         # one colour
     },
     "plain": {
-        "normal_equations": (722979328 + 8198656) / _PIX3,                    # k_ls_accumulate_mma<12>
-        "objective": (1255526000 + 4267264) / _PIX3,                          # k_objective_p<12>
-        "assemble_level0": (718652928 + 626347520 + 671268096 + 1827433000) / _PIX3,
-        "quant_sweep": (1030932000 + 46642944) / _PIX3,
-        "bc_refine": (1279862000 + 43057664) / _PIX3,
+        "normal_equations": (724286464 + 7217920) / _PIX3,                    # k_ls_accumulate_mma<12>
+        "objective": (1255532288 + 3693568) / _PIX3,                          # k_objective_staged<12>
+        "assemble_level0": (718845696 + 626082816 + 671227648 + 1820426752) / _PIX3,
+        "assemble_level1": (718744064 + 628377344 + 671327232 + 108557056) / _PIX3,
+        "quant_sweep": (1030621696 + 47152896) / _PIX3,
+        "bc_refine": (1288049408 + 55825920) / _PIX3,
     },
 }
 
 # What bounds each group, from the same captures: the roofline the HBM fraction alone does not show.
 BINDING = {
     "adjoint": {
-        "assemble_level0": "issue: the fused FP32 site terms at ~88% issue; the gather's L2 latency (one visit ahead)",
-        "assemble_level1": "issue: the fused FP32 site terms at ~88% issue; the gather at ~50% issue (cp.async ring)",
-        "objective": "issue: FP32 decode with fused multiply-adds, ~72% issue, FP32 pipe ~36%",
-        "normal_equations": "latency of the site rows' loads at 16 warps per SM; the tensor pipe (tcgen05) ~14% busy",
-        "bc_refine": "latency: the set-up (block-major stencil copy, coalesced), then the ordered selector steps",
-        "quant_sweep": "HBM (FP32 per-block stencil, a level-0 colour at ~67% of the copy bandwidth)",
+        "assemble_level0": "issue: the fused FP32 site terms at ~63% issue, the tiled gather at ~68% (48% of the L1's "
+                           "wavefronts)",
+        "assemble_level1": "issue: the fused FP32 site terms at ~65% issue; the tiled gather at ~53% issue and 15 warps per "
+                           "SM",
+        "objective": "the L1's wavefronts (~97%: a site's targets a pixel apart), ~64% issue",
+        "normal_equations": "latency and issue of forming the site rows at 16 warps per SM: ~52% issue, ~52% of the L1's "
+                            "wavefronts",
+        "bc_refine": "the L1's wavefronts (~56%) and issue (~55%): the ordered selector steps, 16 at a time",
+        "quant_sweep": "latency at 24 to 32 warps per SM (FP32 per-block stencil read by rows, a level-0 colour at ~70% of "
+                       "the copy bandwidth)",
         "cg_product_level0": "HBM (FP32 stencil)",
         "cg_product_level1": "DRAM latency (small launches)",
     },
     "plain": {
-        "assemble_level0": "FP32/ALU issue (site terms, the reference's unfused arithmetic) and FP64 issue plus stencil "
-                           "stores (gather)",
-        "assemble_level1": "FP32/ALU issue (site terms) and L2 latency (gather)",
-        "objective": "FP64 pipe (~50% of peak)",
-        "normal_equations": "the FP64 tensor pipe (mma.sync m8n8k4, ~76% busy)",
-        "bc_refine": "latency: the set-up (block-major stencil copy, coalesced), then the ordered selector steps",
-        "quant_sweep": "HBM (FP64 stencil, a level-0 colour at ~78% of the copy bandwidth)",
+        "assemble_level0": "FP32/ALU issue (site terms, the reference's unfused arithmetic, ~86%) and the FP64 pipe (gather, "
+                           "~50%)",
+        "assemble_level1": "FP32/ALU issue (site terms, ~87%) and the FP64 pipe (gather, ~43%)",
+        "objective": "issue (~75%) and the FP64 pipe (~55%)",
+        "normal_equations": "the FP64 tensor pipe (mma.sync m8n8k4)",
+        "bc_refine": "the L1's wavefronts (~56%) and issue (~55%): the ordered selector steps, 16 at a time",
+        "quant_sweep": "HBM (FP64 stencil, a level-0 colour at ~89% of the copy bandwidth)",
         "cg_product_level0": "HBM (FP64 stencil)",
         "cg_product_level1": "DRAM latency (small launches)",
     },

@@ -10,10 +10,10 @@
 // block-major copy of the FP64 stencil that the refinement's own assembly writes (a block's coefficients contiguous,
 // so the warp's reads are whole lines instead of scattered doubles of the colour-major stencil). Every value is
 // computed with the arithmetic of the reference's CPU transcription (src/cpu/cpu_refine_bc.cpp:134-400), including
-// its order of summation: each block sum is a SERIAL fold over the sixteen texels in increasing order, which a warp
-// reproduces exactly by shuffling the sixteen per-lane terms to every lane and folding them in texel order. The
-// selector argmin evaluates its eight candidates on eight lanes and scans them in candidate order. Given the same
-// stencil, gradient and planes the endpoints and selectors are therefore the same bytes as the reference's.
+// its order of summation: each block sum is a SERIAL fold over the sixteen texels in increasing order, a sum a lane over
+// terms in shared memory. The selector argmin weighs its eight candidates on two lanes in candidate order, sixteen
+// texels at once. Given the same stencil, gradient and planes the endpoints and selectors are therefore the same bytes as
+// the reference's.
 //
 // The seed pack (src/export.cpp:294-328 over shared/bc_pack.h:95-188) runs here on the device as well: one thread
 // per block-channel, integer arithmetic and the same float palette distances.
