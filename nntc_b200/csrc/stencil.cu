@@ -791,8 +791,14 @@ __global__ void __launch_bounds__(FOLD_THREADS) k_cg_start(Planes P, Red R)
     }
 }
 
-template <int C, typename TS>
-__global__ void __launch_bounds__(THREADS, 4) k_cg_matvec(Planes P, Red R)
+// The product with a thread per texel. PER_SM, the blocks an SM is to hold, weighs the loads a thread has in flight against
+// the threads: an FP64 block of four channels needs the registers of three blocks an SM (four against three, us: 256 x 256
+// 13.8 / 13.2, 1000 x 756 167 / 139, 2048 x 1024 428 / 355; two 524), two channels do with those of six (four against six:
+// 256 x 256 6.06 / 5.92, 512 x 512 18.3 / 16.2, 2048 x 2048 236 / 211), three channels stay at four (1024 x 1024: three 133,
+// four 106, five 117). A launch of at most a block an SM has nothing to hold more blocks with: two channels at 96 x 80 take
+// 4.24 us at four and 4.57 at six.
+template <int C, typename TS, int PER_SM = C == 4 ? 3 : 4>
+__global__ void __launch_bounds__(THREADS, PER_SM) k_cg_matvec(Planes P, Red R)
 {
     __shared__ double sh[32];
     const long long base = (long long)blockIdx.x * blockDim.x;
@@ -1906,8 +1912,10 @@ int solve_block(nntc_b200_device* d, const nntc_b200_model* m, int k, double rid
             case 2:
                 if (f32)
                     k_cg_matvec_rows<2><<<tblocks, THREADS, 0, d->stream>>>(P, R, symmetric);
-                else
+                else if (tblocks <= 148)
                     k_cg_matvec<2, double><<<tblocks, THREADS, 0, d->stream>>>(P, R);
+                else
+                    k_cg_matvec<2, double, 6><<<tblocks, THREADS, 0, d->stream>>>(P, R);
                 break;
             case 3:
                 if (f32)

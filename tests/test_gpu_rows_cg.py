@@ -87,6 +87,25 @@ def test_sweep_in_one_launch(c0, c1, w, h, mip_min, f32, sweeps):
                 assert np.array_equal(ws["x"], want), (level0, i)
 
 
+@pytest.mark.parametrize("c0,w,h", [(2, 171, 160), (2, 231, 180), (4, 171, 160), (3, 171, 160)])
+def test_fp64_solve_residual(c0, w, h):
+    """Block (c') on the FP64 stencil at two channels on either side of a block of texels per SM (148 blocks of 256), and at
+    three and four: the solution against the downloaded stencil. The recursive residual is below 1e-10 of the right-hand
+    side when the iterations stop, and FP64 recurrences over at most 200 of them leave the true one within 1e-9 of it."""
+    mat = materials.small(w + h, w, h, textures=2, c0=c0, c1=2)
+    rng = np.random.default_rng(w * h + c0)
+    with Session(mat) as s:
+        for i, p in enumerate(mat.planes):
+            s.set_planes(i, rng.random(p[0] * p[1] * c0) * 2 - 1, rng.random(p[2] * p[3] * 2) * 2 - 1)
+        s.set_decoder(rng.standard_normal((6, s.m.nin)) * 0.3, rng.random(6))
+        s.set_grids(np.full(c0, -1.0), np.full(c0, 1.0), np.full(2, -1.0), np.full(2, 1.0))
+        rep, _ = s.block(True, ridge=1e-3)
+        for i, p in enumerate(mat.planes):
+            ws = s.workspace(i, True)
+            ax = stencil_product(ws["stencil"], ws["x"], p[0], p[1], c0) + rep[i].lambda_ * ws["x"]
+            assert np.linalg.norm(ax + ws["grad"]) <= 1.1e-9 * np.linalg.norm(ws["grad"]), i
+
+
 @pytest.mark.parametrize("w,h,weights", [(601, 611, "one"), (512, 750, "mixed"), (896, 600, "one")])
 def test_colour_launches_of_either_residency(w, h, weights):
     """A colour of an FP32 stencil of four channels at about 480 and 500 blocks (four to an SM) and 700 (three), with symmetric
