@@ -705,7 +705,7 @@ static int gather_planes(nntc_b200_device* d, int level0, const Planes& P, int n
     // shared memory: three tiles to an SM while its pixels are about four a texel (up to ANY_SHARED bytes), else, on
     // the deep planes of an odd chain, as many as fit (up to ANY_SHARED_MAX) - in a launch of their own when the others
     // would lose their three for it, in the same launch when there are too few tiles for that to matter.
-    constexpr size_t ANY_SHARED = 73 * 1024, ANY_SHARED_MAX = 200 * 1024;
+    constexpr size_t ANY_SHARED = 73 * 1024;
     constexpr int ANY_FEW = 2 * 148;
     AnyTiles R{};
     size_t any_bytes[MAX_PLANES] = {};

@@ -69,6 +69,12 @@ void count_launch();
         NB_CUDA(cudaGetLastError());                                                                                  \
     } while (0)
 
+// The most dynamic shared memory a kernel's launches may ask for. The limit is the function's, of every host thread that
+// launches it: each call sets the same `most`, never what its own launch takes, or a handle on another thread could lower
+// it between this call and the launch.
+#define NB_SHARED_LIMIT(kernel, most) \
+    NB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(most)))
+
 inline int grid_for(size_t n, int threads)
 {
     return (int)((n + (size_t)threads - 1) / (size_t)threads);

@@ -302,8 +302,7 @@ static int queue_normal_equations(nntc_b200_device* d, int k, const double* per_
         NB_TRY(ktimer_begin(d, NNTC_B200_K_NORMAL_EQ));
 #define NB_NE(NO)                                                                                                     \
     case NO:                                                                                                          \
-        NB_CUDA(cudaFuncSetAttribute(k_ls_accumulate_mma<NO>, cudaFuncAttributeMaxDynamicSharedMemorySize,           \
-                                     (int)shared));                                                                   \
+        NB_SHARED_LIMIT(k_ls_accumulate_mma<NO>, NE_SHARED);                                                           \
         k_ls_accumulate_mma<NO><<<grid, NE_THREADS, shared, d->stream>>>(P, A);                                       \
         break;
         switch (d->nout)
@@ -323,7 +322,7 @@ static int queue_normal_equations(nntc_b200_device* d, int k, const double* per_
         NB_LAUNCHED();
     }
     const size_t lr_shared = (size_t)P.n * (LS_GRID + 1) * sizeof(double);
-    NB_CUDA(cudaFuncSetAttribute(k_ls_reduce, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lr_shared));
+    NB_SHARED_LIMIT(k_ls_reduce, (size_t)MAX_PLANES * (LS_GRID + 1) * sizeof(double));
     k_ls_reduce<<<entries, LR_THREADS, lr_shared, d->stream>>>(d->ls_partial, entries, P.n, omega, d->reduction);
     NB_LAUNCHED();
     double* obj_out = d->ls_obj + (size_t)P.n * 3 * LS_GRID;

@@ -400,8 +400,6 @@ __global__ void __launch_bounds__(TILE1_THREADS, 3) k_gather_tile1(Planes P, con
 // on the pixel row's parity alone, and the other way round - so a block forms each column's and row's once, with
 // tap_at's arithmetic, next to the staged samples; and a pixel's sites are taken side by side, one that misses the texel
 // entering the sums with weight, sample and term zero, whose exact zeros leave them as they were (a sum is never -0).
-constexpr int MAX_SITES = 5;   // sites of a pixel at the largest K the split assembly takes
-
 struct __align__(16) AxisTap
 {
     int a, b;        // the two texels, clamped
@@ -647,7 +645,7 @@ static int launch_any(nntc_b200_device* d, const Planes& P, const TileArgs<TS>& 
     default: kernel = P.kc == 4 ? k_gather_any1<TS, 4, 5> : k_gather_any1<TS, 4, 0>; break;
     }
 #undef NB_ANY
-    NB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared));
+    NB_SHARED_LIMIT(kernel, ANY_SHARED_MAX);
     kernel<<<grid, TILE1_THREADS, shared, d->stream>>>(P, A, S);
     NB_LAUNCHED();
     return NNTC_B200_OK;
@@ -669,7 +667,7 @@ template <typename TS>
 static int launch_tiles(nntc_b200_device* d, int level0, const Planes& P, const TileArgs<TS>& A, unsigned grid)
 {
     const int per = 1 + P.kc, ny = level0 ? d->c1 : d->c0;
-    const int shared = (level0 ? TILE0_PX * TILE0_PY : TILE1_PX * TILE1_PY) * per * (int)sizeof(float4);
+    const int site = (level0 ? TILE0_PX * TILE0_PY : TILE1_PX * TILE1_PY) * (int)sizeof(float4), shared = site * per;
     void (*kernel)(Planes, const TileArgs<TS>) = nullptr;
     if (level0)
         kernel = ny == 1 ? k_gather_tile0<TS, 1>
@@ -677,7 +675,7 @@ static int launch_tiles(nntc_b200_device* d, int level0, const Planes& P, const 
     else
         kernel = ny == 1 ? k_gather_tile1<TS, 1>
                          : (ny == 2 ? k_gather_tile1<TS, 2> : (ny == 3 ? k_gather_tile1<TS, 3> : k_gather_tile1<TS, 4>));
-    NB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, shared));
+    NB_SHARED_LIMIT(kernel, site * MAX_SITES);
     kernel<<<grid, level0 ? TILE0_THREADS : TILE1_THREADS, shared, d->stream>>>(P, A);
     NB_LAUNCHED();
     return NNTC_B200_OK;

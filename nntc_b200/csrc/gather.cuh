@@ -245,6 +245,9 @@ __device__ __forceinline__ void visit_sums(TS (&sums)[MAX_MONO], const float4& y
     }
 }
 
+constexpr int MAX_SITES = 5;   // sites of a pixel at the largest K the split assembly takes
+constexpr size_t ANY_SHARED_MAX = 200 * 1024;   // the most a tile of k_gather_any1 may take
+
 // Level 1 planes whose visits are not tabled, in tiles of the same texels (k_gather_any1): the pixels a tile's texels
 // can meet on each axis, at most, per plane.
 struct AnyTiles

@@ -527,14 +527,12 @@ int launch_ls_accumulate_tc(nntc_b200_device* d, const Planes& P, double* partia
     case NO:                                                                                                          \
         if (obj_partial)                                                                                              \
         {                                                                                                             \
-            NB_CUDA(cudaFuncSetAttribute(k_ls_accumulate_tc<NO, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,  \
-                                         (int)TG_SHARED));                                                            \
+            NB_SHARED_LIMIT((k_ls_accumulate_tc<NO, true>), TG_SHARED);                                               \
             k_ls_accumulate_tc<NO, true><<<grid, TG_THREADS, TG_SHARED, stream>>>(P, args);                           \
         }                                                                                                             \
         else                                                                                                          \
         {                                                                                                             \
-            NB_CUDA(cudaFuncSetAttribute(k_ls_accumulate_tc<NO, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                         (int)TG_SHARED));                                                            \
+            NB_SHARED_LIMIT((k_ls_accumulate_tc<NO, false>), TG_SHARED);                                              \
             k_ls_accumulate_tc<NO, false><<<grid, TG_THREADS, TG_SHARED, stream>>>(P, args);                          \
         }                                                                                                             \
         break;

@@ -183,7 +183,7 @@ int fit_grid_device(nntc_b200_device* d, int level0, bool pct, float* lo, float*
         const int bins = 1 << R.width;
         NB_CUDA(cudaMemsetAsync(scratch, 0, (size_t)2 * c * bins * sizeof(unsigned), d->stream));
         const size_t shared = (size_t)2 * c * bins * sizeof(unsigned);
-        NB_CUDA(cudaFuncSetAttribute(k_radix_hist, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared));
+        NB_SHARED_LIMIT(k_radix_hist, (size_t)2 * MAX_CH * (1 << 11) * sizeof(unsigned));
         for (const DevPlane& p : d->planes)
         {
             const size_t n = values(p);

@@ -687,7 +687,7 @@ int bc_refine_passes(nntc_b200_device* d, const nntc_b200_model* m, int passes, 
     const size_t shared = (size_t)per_warp * REFINE_WARPS * sizeof(double);
     void (*kernel)(BcPlanes, RefineArgs) =
         c0 == 1 ? k_bc_refine<1> : (c0 == 2 ? k_bc_refine<2> : (c0 == 3 ? k_bc_refine<3> : k_bc_refine<4>));
-    NB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared));
+    NB_SHARED_LIMIT(kernel, shared);   // the channel count's own
     for (int pass = 0; pass < passes; pass++)
     {
         NB_CUDA(cudaMemsetAsync(d->bc_stats, 0, (size_t)MAX_PLANES * 2 * sizeof(double), d->stream));

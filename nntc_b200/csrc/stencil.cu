@@ -1743,7 +1743,7 @@ static int launch_sweep(nntc_b200_device* d, const Planes& P, const SweepArgs& A
     constexpr bool ROWS = sizeof(TS) == sizeof(float) && C % 2 == 0;
     const int shared =
         TileX<C>::PAIRS * 4 * SWEEP_CELLS * (int)sizeof(double2) + (ROWS ? SWEEP_THREADS<TS> * C * (int)sizeof(double) : 0);
-    NB_CUDA(cudaFuncSetAttribute(k_quant_sweep<C, TS>, cudaFuncAttributeMaxDynamicSharedMemorySize, shared));
+    NB_SHARED_LIMIT((k_quant_sweep<C, TS>), shared);
     k_quant_sweep<C, TS><<<tiles, SWEEP_THREADS<TS>, shared, d->stream>>>(P, A);
     NB_LAUNCHED();
     return NNTC_B200_OK;
@@ -1812,12 +1812,12 @@ int assemble(nntc_b200_device* d, const nntc_b200_model* m, int k, double ridge,
         NB_TRY(assemble_split(d, k, level0, P, nmono, mono.data(), diag_only ? 1 : SLOTS, d->sten_f32[level0]));
     else if (level0)
     {
-        NB_CUDA(cudaFuncSetAttribute(k_assemble<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared));
+        NB_SHARED_LIMIT(k_assemble<true>, (size_t)SLOTS * MAX_MONO * ASM_THREADS * sizeof(double));
         k_assemble<true><<<blocks, ASM_THREADS, shared, d->stream>>>(P, A);
     }
     else
     {
-        NB_CUDA(cudaFuncSetAttribute(k_assemble<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared));
+        NB_SHARED_LIMIT(k_assemble<false>, (size_t)SLOTS * MAX_MONO * ASM_THREADS * sizeof(double));
         k_assemble<false><<<blocks, ASM_THREADS, shared, d->stream>>>(P, A);
     }
     NB_TRY(ktimer_end(d));
