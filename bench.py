@@ -522,6 +522,13 @@ BINDING = {
 }
 
 
+SWEEP_TILES, SWEEP_W, SWEEP_H = 148, 32, 28   # level-0 chains of at most this many tiles are swept in one launch
+
+
+def sweep_tiles(mat):
+    return sum(-(-p[0] // SWEEP_W) * -(-p[1] // SWEEP_H) for p in mat.planes)
+
+
 def roofline(name, stat, mat, hbm, tf, src, form):
     """The dominant kernel against the HBM roofline: its algorithmic bytes per launch over its mean launch time."""
     launches, ms = stat
@@ -530,13 +537,16 @@ def roofline(name, stat, mat, hbm, tf, src, form):
     per = algorithmic_bytes(name, mat, form)
     achieved = per / (ms / launches / 1000.0) / 1e9
     t0 = sum(p[0] * p[1] for p in mat.planes)
-    unit = TRAFFIC_PER_UNIT[form].get(name)
+    unit, binding = TRAFFIC_PER_UNIT[form].get(name), BINDING[form].get(name)
+    if name == "quant_sweep" and sweep_tiles(mat) <= SWEEP_TILES:
+        # a whole sweep a launch, counted as its colours: the figures above are of a launch per colour
+        unit, binding = None, "latency: a whole sweep a launch, its four colours one after another in shared memory"
     traffic = round(unit * t0) if unit else None
     return {"kernel": name, "bound": "hbm", "achieved": round(achieved, 2), "peak": hbm, "unit": "GB/s",
             "frac": round(achieved / hbm, 4), "traffic": traffic, "peak_source": src,
             "traffic_source": "ncu DRAM bytes of the 4x2048x1024 workload scaled by level-0 pixels" if traffic
             else "no ncu DRAM figure recorded for this group's current kernels",
-            "binding": BINDING[form].get(name), "bytes_per_launch": per, "launches": launches,
+            "binding": binding, "bytes_per_launch": per, "launches": launches,
             "ms_per_launch": round(ms / launches, 4)}
 
 

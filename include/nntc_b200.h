@@ -356,7 +356,8 @@ enum nntc_b200_kernel
     NNTC_B200_K_ASSEMBLE1,       /* block (b)'s stencil and gradient gather */
     NNTC_B200_K_ASSEMBLE0,       /* block (c')'s stencil and gradient gather */
     NNTC_B200_K_MATVEC,          /* one conjugate-gradient product over every plane, block (b) (level 1) */
-    NNTC_B200_K_SWEEP,           /* one colour of the quantised sweeps (a whole sweep where the planes are small) */
+    NNTC_B200_K_SWEEP,           /* one colour of the quantised sweeps (a launch of a whole sweep, where the
+                                  * planes are small, counts as its colours) */
     NNTC_B200_K_REFINE,          /* one colour of the BC refinement */
     NNTC_B200_K_MATVEC0,         /* one conjugate-gradient product over every plane, block (c') (level 0) */
     NNTC_B200_K_COUNT

@@ -59,7 +59,7 @@ void count_launch()
     g_launches.fetch_add(1, std::memory_order_relaxed);
 }
 
-int ktimer_begin(nntc_b200_device* d, int kind)
+int ktimer_begin(nntc_b200_device* d, int kind, int count)
 {
     if (!d->ktiming)
         return NNTC_B200_OK;
@@ -74,7 +74,7 @@ int ktimer_begin(nntc_b200_device* d, int kind)
             d->kpool.pop_back();
         }
     }
-    d->kpending.push_back({ kind, e[0], e[1] });
+    d->kpending.push_back({ kind, count, e[0], e[1] });
     NB_CUDA(cudaEventRecord(e[0], d->stream));
     return NNTC_B200_OK;
 }
@@ -93,7 +93,7 @@ int ktimer_harvest(nntc_b200_device* d)
     {
         float t = 0.0f;
         NB_CUDA(cudaEventElapsedTime(&t, p.a, p.b));
-        d->klaunches[p.kind]++;
+        d->klaunches[p.kind] += p.count;
         d->kms[p.kind] += (double)t;
         d->kpool.push_back(p.a);
         d->kpool.push_back(p.b);

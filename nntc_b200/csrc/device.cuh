@@ -172,7 +172,7 @@ struct nntc_b200_device
     // after the block that launched them has been waited for.
     struct Pending
     {
-        int kind;
+        int kind, count;
         cudaEvent_t a, b;
     };
     bool ktiming = false;
@@ -258,8 +258,9 @@ inline Planes planes_for(const nntc_b200_device* d, int level0, F items)
 int block_begin(nntc_b200_device* d);
 int block_end(nntc_b200_device* d, double* ms);
 
-// Brackets of one launch of a hot kernel (no-ops unless kernel timing is on); harvested at every block_end.
-int ktimer_begin(nntc_b200_device* d, int kind);
+// Brackets of one launch of a hot kernel (no-ops unless kernel timing is on); harvested at every block_end. count: the
+// launches it stands for (a whole sweep in one launch is its colours).
+int ktimer_begin(nntc_b200_device* d, int kind, int count = 1);
 int ktimer_end(nntc_b200_device* d);
 int ktimer_harvest(nntc_b200_device* d);
 

@@ -2007,8 +2007,11 @@ int sweep_block(nntc_b200_device* d, const nntc_b200_model* m, int k, double rid
     SweepArgs S{ d->scalars, level0 ? d->lo0 : d->lo1, level0 ? d->hi0 : d->hi1, bits, d->sten_symmetric[level0] ? 1 : 0 };
     S.moved = d->counters + CNT_SWEEP;
     int tiles = 0;
+    bool wide = false, high = false;
     for (int i = P.n - 1; i >= 0; i--)
     {
+        wide = wide || P.p[i].w > 1;
+        high = high || P.p[i].h > 1;
         S.btiles[i] = ((P.p[i].w + SWEEP_W - 1) / SWEEP_W) * ((P.p[i].h + SWEEP_H - 1) / SWEEP_H);
         S.bend[i] = tiles += S.btiles[i];
     }
@@ -2016,7 +2019,7 @@ int sweep_block(nntc_b200_device* d, const nntc_b200_model* m, int k, double rid
     {
         S.first = s == 0;
         S.to_r = (sweeps - 1 - s) & 1;   // the last sweep leaves the corrections in x
-        NB_TRY(ktimer_begin(d, NNTC_B200_K_SWEEP));
+        NB_TRY(ktimer_begin(d, NNTC_B200_K_SWEEP, (wide ? 2 : 1) * (high ? 2 : 1)));   // the colours it has
 #define NB_SWEEP(C)                                                                                                   \
     if (d->sten_f32[level0])                                                                                          \
         NB_TRY((launch_sweep<C, float>(d, P, S, tiles)));                                                             \
