@@ -649,7 +649,7 @@ static int launch_walk(nntc_b200_device* d, int level0, const Planes& P, const T
     return NNTC_B200_OK;
 }
 
-// The gather of every plane: the tabled planes in one launch, the others in one or two more.
+// The gather of every plane: the tabled planes in one launch, the others in one more, or two.
 template <typename TS>
 static int gather_planes(nntc_b200_device* d, int level0, const Planes& P, int nmono, const double* mono, int slots)
 {
@@ -702,10 +702,13 @@ static int gather_planes(nntc_b200_device* d, int level0, const Planes& P, int n
     std::memcpy(A.off, d->gtab_off[level0], sizeof(A.off));
     auto pow2 = [](int v) { return v > 0 && (v & (v - 1)) == 0; };
     // A level-1 plane that is not tabled goes to k_gather_any1 in tiles of the same texels, wherever a tile's sites fit
-    // shared memory: three tiles to an SM while its pixels are about four a texel (up to ANY_SHARED bytes), else, on
-    // the deep planes of an odd chain, as many as fit (up to ANY_SHARED_MAX) - in a launch of their own when the others
-    // would lose their three for it, in the same launch when there are too few tiles for that to matter.
-    constexpr size_t ANY_SHARED = 73 * 1024;
+    // shared memory. At K = 4 a tile of four pixels a texel takes 76.7 KB and those of an odd chain's planes up to
+    // 80.3 KB: two to an SM either way, so that they share a launch. A launch of their own for the deepest planes' few
+    // tiles costs a tile's whole walk on an idle GPU (us, both launches against one: 450 x 333 292 / 200, 1000 x 756 751 /
+    // 638, 2047 x 1023 2073 / 1938). Planes whose tile leaves room for one alone are launched apart, or the others would
+    // lose their second tile - in the same launch when there are too few tiles for that to matter.
+    constexpr size_t SM_SHARED = 228 * 1024, BLOCK_RESERVED = 1024, ANY_STATIC = MAX_MONO * 32 * sizeof(TS);
+    constexpr size_t ANY_SHARED = SM_SHARED / 2 - BLOCK_RESERVED - ANY_STATIC;
     constexpr int ANY_FEW = 2 * 148;
     AnyTiles R{};
     size_t any_bytes[MAX_PLANES] = {};
