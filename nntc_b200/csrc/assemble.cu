@@ -533,7 +533,7 @@ __device__ __forceinline__ void stencil_texel(long long pos, int w, int h, int& 
 }
 
 // The gather of the planes no tile takes (planes one texel wide or high at level 0, level-1 planes whose tile would not
-// fit shared memory): one thread per (texel, slot) tests every site of the two texels' common
+// fit shared memory or that are above any_tiles_line): one thread per (texel, slot) tests every site of the two texels' common
 // footprint, in site order; the self-slot thread also gathers the gradient. Blocks run in (region, colour, slot) order,
 // the slot fastest, so that the five slots of one run of texels and the four colours of one region run side by side
 // and share the region's sites in L2.
@@ -649,6 +649,31 @@ static int launch_walk(nntc_b200_device* d, int level0, const Planes& P, const T
     return NNTC_B200_OK;
 }
 
+// The tiles of k_gather_any1 up to which it takes a level's planes that are not tabled; with more of them the walk does.
+// The tiles test each pixel once for five warps, whatever comes of it, and stage its sites, which pays the more sites a
+// pixel has; a thread a (texel, slot) waits longer but keeps more of them in flight, so that it gains as the launch
+// grows. FP32 terms of four channels are staged side by side with the samples; an odd count of FP64 ones a value at a
+// time. Measured (us, tiles / walk; at 950, 2050, 5460 and 15666 tiles: 700 x 500 to 3000 x 2000), every slot:
+//   K = 0: FP64 2 channels 92 / 104, 159 / 150, 394 / 320, 1061 / 750; 3 channels 154 / 105, 262 / 154, 697 / 323,
+//          1930 / 761; FP32 2 channels 99 / 90, 170 / 143, 463 / 296, 1270 / 700; 4 channels 85 / 128, 149 / 179, 378 / 360,
+//          1034 / 895
+//   K = 1: FP64 2 channels 132 / 197, 229 / 291, 571 / 625, 1528 / 1496; 3 channels 206 / 220, 367 / 312, 939 / 669,
+//          2537 / 1624; FP32 2 channels 142 / 178, 242 / 282, 642 / 601, 1758 / 1448
+//   K = 2: FP64 2 channels 172 / 306, 296 / 434, 739 / 934, 1983 / 2191; 3 channels 259 / 329, 457 / 447, 1162 / 945,
+//          3200 / 2213; FP32 2 channels 182 / 258, 318 / 400, 810 / 849, 2229 / 1994
+//   K = 4: FP64 2 channels (5460 and 15666) 1172 / 1731, 3150 / 3953; 3 channels 2060 / 1771, 5808 / 4011; FP32 2 channels
+//          1265 / 1579, 3454 / 3685; 4 channels 1066 / 1835, 2913 / 4432
+// The diagonal blocks alone leave three of the five warps idle (FP64 2 channels at 400, 2050 and 5460 tiles: K = 0 36 / 66,
+// 139 / 89, 350 / 184; K = 2 69 / 197, 266 / 275, 666 / 570; K = 4 124 / 366, 431 / 532, 1119 / 1028).
+static int any_tiles_line(bool f32, int c, int sites, bool every_slot)
+{
+    const bool staged = f32 && c == MAX_CH;
+    const int base = staged ? 3200 : (!f32 && c % 2 != 0 ? 400 : 800);
+    if (every_slot)
+        return base * sites * sites;
+    return staged ? base / 2 * sites * sites : base * 3 / 4 * sites;
+}
+
 // The gather of every plane: the tabled planes in one launch, the others in one more, or two.
 template <typename TS>
 static int gather_planes(nntc_b200_device* d, int level0, const Planes& P, int nmono, const double* mono, int slots)
@@ -702,7 +727,7 @@ static int gather_planes(nntc_b200_device* d, int level0, const Planes& P, int n
     std::memcpy(A.off, d->gtab_off[level0], sizeof(A.off));
     auto pow2 = [](int v) { return v > 0 && (v & (v - 1)) == 0; };
     // A level-1 plane that is not tabled goes to k_gather_any1 in tiles of the same texels, wherever a tile's sites fit
-    // shared memory. At K = 4 a tile of four pixels a texel takes 76.7 KB and those of an odd chain's planes up to
+    // shared memory and the level has no more tiles than any_tiles_line. At K = 4 a tile of four pixels a texel takes 76.7 KB and those of an odd chain's planes up to
     // 80.3 KB: two to an SM either way, so that they share a launch. A launch of their own for the deepest planes' few
     // tiles costs a tile's whole walk on an idle GPU (us, both launches against one: 450 x 333 292 / 200, 1000 x 756 751 /
     // 638, 2047 x 1023 2073 / 1938). Planes whose tile leaves room for one alone are launched apart, or the others would
@@ -723,8 +748,11 @@ static int gather_planes(nntc_b200_device* d, int level0, const Planes& P, int n
         }
         return most;
     };
-    WalkBlocks B{};
-    long long at = 0, walk = 0;
+    auto any_tiles_of = [&](int i) {
+        return any_bytes[i] ? ((P.p[i].w + TILE1_W - 1) / TILE1_W) * ((P.p[i].h + TILE1_H - 1) / TILE1_H) : 0;
+    };
+    long long at = 0;
+    int any_tiles = 0;
     for (int i = 0; i < P.n; i++)
     {
         const PlaneView& v = P.p[i];
@@ -740,22 +768,28 @@ static int gather_planes(nntc_b200_device* d, int level0, const Planes& P, int n
             R.py[i] = widest(v.h, v.h0, TILE1_H);
             const size_t bytes = any_tile_bytes(R.px[i], R.py[i], 1 + k);
             any_bytes[i] = bytes <= ANY_SHARED_MAX && R.px[i] * (1 + k) < 1024 ? bytes : 0;
+            any_tiles += any_tiles_of(i);
         }
-        const bool walked = !tiled && any_bytes[i] == 0;
+    }
+    A.site0[P.n] = at;
+    if (any_tiles > any_tiles_line(sizeof(TS) == sizeof(float), c, 1 + k, slots == SLOTS))
+        any_tiles = 0;
+    WalkBlocks B{};
+    long long walk = 0;
+    for (int i = 0; i < P.n; i++)
+    {
+        const PlaneView& v = P.p[i];
+        const bool walked = A.btiles[i] == 0 && (any_bytes[i] == 0 || any_tiles == 0);
         B.start[i] = walk;
         const long long largest = (long long)((v.w + 1) / 2) * ((v.h + 1) / 2);   // colour 0
         walk += walked ? (largest + WALK_THREADS - 1) / WALK_THREADS * 4 * slots : 0;
     }
-    A.site0[P.n] = at;
     B.start[P.n] = walk;
     int tiles = 0;
     for (int i = P.n - 1; i >= 0; i--)
         A.bend[i] = tiles += A.btiles[i];
     if (walk > 0)
         NB_TRY(launch_walk<TS>(d, level0, P, A, B));
-    int any_tiles = 0;
-    for (int i = 0; i < P.n; i++)
-        any_tiles += any_bytes[i] ? ((P.p[i].w + TILE1_W - 1) / TILE1_W) * ((P.p[i].h + TILE1_H - 1) / TILE1_H) : 0;
     for (int group = 0; group < 2 && any_tiles > 0; group++)   // the larger tiles, then the others
     {
         TileArgs<TS> G = A;
@@ -764,9 +798,7 @@ static int gather_planes(nntc_b200_device* d, int level0, const Planes& P, int n
         for (int i = P.n - 1; i >= 0; i--)
         {
             const bool large = any_bytes[i] > ANY_SHARED || any_tiles <= ANY_FEW;
-            G.btiles[i] = any_bytes[i] && large == (group == 0)
-                              ? ((P.p[i].w + TILE1_W - 1) / TILE1_W) * ((P.p[i].h + TILE1_H - 1) / TILE1_H)
-                              : 0;
+            G.btiles[i] = large == (group == 0) ? any_tiles_of(i) : 0;
             shared = G.btiles[i] ? std::max(shared, any_bytes[i]) : shared;
             G.bend[i] = blocks += G.btiles[i];
         }

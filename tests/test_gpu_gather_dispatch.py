@@ -54,7 +54,37 @@ def test_launches_of_the_ragged_planes(planes, k, any1, f32):
     assert gather_launches(mat, state, f32, k) == (any1, 0)
 
 
-@pytest.mark.parametrize("planes,textures,c0,c1,k", [(ROUNDS, 2, 2, 4, 4), (ROUNDS, 1, 4, 3, 4), (ROUNDS, 1, 3, 2, 2),
+# ROUNDS has 1004 tiles: above the line between the tiles and the walk at K = 0 but for FP32 terms of four channels, below it
+# at K = 1 and more; with FP64 terms of one or three channels the line is half as far
+@pytest.mark.parametrize("c1,k,f32,tiled", [(2, 0, 0, False), (3, 0, 0, False), (2, 0, 1, False), (4, 0, 1, True),
+                                            (2, 1, 0, True), (3, 1, 0, True), (2, 1, 1, True), (1, 4, 0, True)])
+def test_large_ragged_planes_of_few_sites_are_walked(c1, k, f32, tiled):
+    mat, state = material(ROUNDS, 1, 2, c1, k)
+    assert gather_launches(mat, state, f32, k) == ((1, 0) if tiled else (0, 1))
+
+
+@pytest.mark.parametrize("c1,k", [(2, 0), (3, 1), (4, 1), (4, 4)])   # walked, walked, tiles, tiles
+def test_diagonal_blocks_alone(c1, k):
+    """The matrix-free conjugate gradients' assembly: its gradient and diagonal blocks are the full assembly's bits."""
+    mat, (dw, db, v0, v1) = material(ROUNDS, 1, 2, c1, k)
+    got = []
+    for option in (0, 1):
+        with Session(mat) as s:
+            check(lib().nntc_b200_set_option(s.d, abi.OPT_ADJOINT_CG, option), "option")
+            for i in range(len(mat.planes)):
+                s.set_planes(i, v0[i], v1[i])
+            s.set_decoder(dw, db)
+            s.set_grids(np.full(2, -1.0), np.full(2, 1.0), np.full(c1, -1.0), np.full(c1, 1.0))
+            s.block(False, k=k)
+            got.append([s.workspace(i, False) for i in range(len(mat.planes))])
+    for a, b in zip(*got):
+        assert np.array_equal(a["grad"], b["grad"])
+        diagonals = [x["stencil"].reshape(-1, 5, c1, c1)[:, 0] for x in (a, b)]
+        assert np.array_equal(*diagonals)
+
+
+@pytest.mark.parametrize("planes,textures,c0,c1,k", [(ROUNDS, 1, 2, 3, 0), (ROUNDS, 2, 4, 4, 0), (ROUNDS, 1, 4, 1, 1),
+                                                     (ROUNDS, 2, 2, 4, 4), (ROUNDS, 1, 4, 3, 4), (ROUNDS, 1, 3, 2, 2),
                                                      (APART, 1, 2, 4, 4), (APART, 2, 4, 1, 4)])
 def test_assembly_matches_the_reference_shape(planes, textures, c0, c1, k):
     mat, state = material(planes, textures, c0, c1, k)
