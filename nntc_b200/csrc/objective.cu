@@ -391,8 +391,7 @@ __device__ __forceinline__ void obj_sample_any(const float* plane, int w, int h,
 // k_objective_p with the targets of the next site on their way to shared memory while this one is decoded
 // (row_stage.cuh) and the features that the channel counts do not have skipped (their weights are zero). Bound by issue
 // and the FP64 pipe (about 600 operations a site): 1857 -> 1739 us at 6 x 2048 x 2048, 772 -> 630 us at 4 x 2048 x 1024.
-// With rows of one or two textures (24 or 48 bytes) the lanes' own loads are the cheaper way (163 against 201 us at 1 x
-// 1000 x 1000), and those materials keep k_objective_p.
+// For the materials that objective_staged names; the others keep k_objective_p.
 template <int NOUT>
 __global__ void __launch_bounds__(OBJ_P_THREADS, 5)
     k_objective_staged(Planes P, const __grid_constant__ ObjDecoder W, double* partial, const __grid_constant__ ObjTargets T)
@@ -754,6 +753,27 @@ void objective_from_sums(const nntc_b200_model& m, int k, const double* per_site
 static double g_objective_ms = 0.0;
 static long long g_objective_calls = 0;
 
+// Whether the objective's targets are staged (k_objective_staged) or each lane loads its own (k_objective_p, which takes
+// every one of the 24 features). Staging costs a site the same whatever its features and saves by the row's length; what
+// it saves beside is the features skipped. So a count of features up to which it is the faster, by textures and K, from
+// both kernels at all sixteen channel pairs, 256 x 256 to 2048 x 2048 (us at 1000 x 756, direct / staged, the last pair
+// below the line and the first above it, features in brackets):
+//   3 textures: K = 4 193 / 190 (14), 192 / 202 (15); K = 2 116 / 116 (9), 116 / 119 (11); K = 1 84 / 83 (9), 84 / 85 (11);
+//               K = 0 42 / 44 (3)
+//   4 textures: K = 4 283 / 236 (24); K = 2 156 / 147 (24); K = 1 105 / 103 (24); K = 0 52 / 51 (15), 53 / 55 (19)
+//   5 textures: K = 4 270 / 271 (19), 273 / 291 (24); K = 2 161 / 159 (15), 163 / 167 (19); K = 1 111 / 107 (15), 113 / 114
+//               (19); K = 0 57 / 56 (14), 57 / 57 (15)
+//   6 textures: K = 4 341 / 327 (24); K = 2 193 / 187 (19), 194 / 207 (24); K = 1 126 / 122 (15), 127 / 131 (19); K = 0
+//               66 / 65 (15), 67 / 70 (19)
+// One texture is the other way at every pair (122 / 150 at K = 4, 14), and so is two from 15 on (151 / 164); below that
+// the two are within a tenth of each other (152 / 151 at 14), and the lanes' own loads stay.
+static bool objective_staged(int nout, int features, int kc)
+{
+    constexpr int MOST[4][4] = { { 0, 9, 9, 14 }, { 15, 24, 24, 24 }, { 14, 15, 15, 19 }, { 15, 15, 19, 24 } };
+    const int textures = nout / 3;
+    return textures >= 3 && features <= MOST[textures - 3][kc < 3 ? kc : 3];
+}
+
 // The raw sums of every plane, three per plane, into host memory (acc has 3 nplanes entries).
 int objective_sums(nntc_b200_device* d, int k, std::vector<double>& acc, double* ms)
 {
@@ -859,17 +879,26 @@ int objective_sums(nntc_b200_device* d, int k, std::vector<double>& acc, double*
         return fetch_sums();
     }
     NB_TRY(ktimer_begin(d, NNTC_B200_K_OBJECTIVE));
+    const bool staged = objective_staged(nout, nin, k);
+#define NB_OBJECTIVE(NO)                                                                                              \
+    case NO:                                                                                                          \
+        if (staged)                                                                                                   \
+            k_objective_staged<NO><<<nblocks, OBJ_P_THREADS, 0, d->stream>>>(P, W, d->obj_partial, T);                \
+        else                                                                                                          \
+            k_objective_p<NO><<<nblocks, OBJ_P_THREADS, 0, d->stream>>>(P, W, d->obj_partial, T);                     \
+        break;
     switch (nout)
     {
     case 3: k_objective_p<3><<<nblocks, OBJ_P_THREADS, 0, d->stream>>>(P, W, d->obj_partial, T); break;
     case 6: k_objective_p<6><<<nblocks, OBJ_P_THREADS, 0, d->stream>>>(P, W, d->obj_partial, T); break;
-    case 9: k_objective_staged<9><<<nblocks, OBJ_P_THREADS, 0, d->stream>>>(P, W, d->obj_partial, T); break;
-    case 12: k_objective_staged<12><<<nblocks, OBJ_P_THREADS, 0, d->stream>>>(P, W, d->obj_partial, T); break;
-    case 15: k_objective_staged<15><<<nblocks, OBJ_P_THREADS, 0, d->stream>>>(P, W, d->obj_partial, T); break;
-    case 18: k_objective_staged<18><<<nblocks, OBJ_P_THREADS, 0, d->stream>>>(P, W, d->obj_partial, T); break;
+        NB_OBJECTIVE(9)
+        NB_OBJECTIVE(12)
+        NB_OBJECTIVE(15)
+        NB_OBJECTIVE(18)
     default:
         k_objective<<<nblocks, OBJ_THREADS, 0, d->stream>>>(P, ObjArgs{ d->weights, d->bias, d->cw, d->obj_partial });
     }
+#undef NB_OBJECTIVE
     NB_TRY(ktimer_end(d));
     NB_LAUNCHED();
     k_objective_reduce<<<dim3(P.n, 3), 256, 0, d->stream>>>(P, d->obj_partial, nblocks, sums, bthreads);
