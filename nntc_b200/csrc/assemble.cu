@@ -15,40 +15,24 @@
 //   - the stencil's monomial sums need only the site's sample of the OTHER latent (a bilinear blend of four texels,
 //     which k_site_terms also stores per site) and the tap weights - a few dozen operations. They are gathered per
 //     (texel, slot): each slot's sums receive the same terms in the same site order as the reference's, so every sum,
-//     and the expansion against the monomial matrices after it, is the same bits. gather.cu does it in tiles;
-//     k_gather_walk below takes the few planes no tile fits.
+//     and the expansion against the monomial matrices after it, is the same bits. gather.cu does it in tiles,
+//     gather_any.cu for the planes whose visits are not tabled.
 //
 // Every plane of the chain is in each launch (nb::Planes); the per-site buffer holds every plane's sites.
 
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <type_traits>
 #include <vector>
 
 #include "footprint.cuh"
 #include "gather.cuh"
+#include "site_terms.cuh"
 
 namespace nb
 {
 
 constexpr int SITE_THREADS = 256;
-constexpr int SITE_BLOCK_MAX = 64 * 5;   // threads of a k_site_terms block at K = 4
-// Pixels of one block (planes_for's unit, so that a block has one plane), in rounds that share its set-up; a launch of
-// fewer than SITE_FEW pixels takes a block per round, which its SMs are too few blocks without (1 x 100 x 76: 3.9
-// against 7.4 us; at 4 x 1024 x 1024 the rounds save 2%).
-constexpr int SITE_PIXELS = THREADS, SITE_FEW = 148 * 6 * SITE_PIXELS;
-
-struct SiteArgs
-{
-    void* terms;                        // [site][c] over every plane: doubles, or floats (MIXED)
-    float4* y;                          // [site]: the site's sample of the other latent
-    const float* tgt;                   // [fractional site][NOUT]: the targets of the sites j > 0 (k_site_targets)
-    long long site0[MAX_PLANES + 1];    // the first site of each plane in `terms`
-    long long tsite0[MAX_PLANES + 1];   // the first fractional site of each plane in `tgt`
-    unsigned span;                      // pixels of one block
-};
-
 struct TargetOffsets
 {
     long long site0[MAX_PLANES + 1];    // the first fractional site of each plane
@@ -89,353 +73,6 @@ __global__ void __launch_bounds__(SITE_THREADS) k_site_targets(Planes P, float* 
 
 // One thread per site: t_s[a] = sum_r cw_r G[r][a] res_r (level 1, block b) or sum_r cw_r Q[r][a] res_r (level 0,
 // block c'), in the reference's order of operations (src/solve_level1.cu:335-361, 518-544).
-// The decoder as a launch parameter, each row at a fixed stride of 24 slots, [c_q (4)][s_i (4)][s_i c_q (4 x 4)]: with
-// the row loop unrolled every weight is a constant-bank operand. Slots of channels the layout does not use are never
-// read (the channel loops are guarded), so the arithmetic is the reference's operation for operation.
-// Fused, every weight twice, side by side: the operand of a packed instruction.
-template <bool MIXED>
-struct SiteDecoder
-{
-    using Weight = typename std::conditional<MIXED, unsigned long long, float>::type;
-    Weight w[MAX_NOUT * 24];
-    Weight b[MAX_NOUT];
-    Weight cw[MAX_NOUT];
-    double cwd[MAX_NOUT];   // the outputs' weights in double (the FP64 terms)
-};
-
-// A lane's sites' values of one quantity. Packed: two side by side in a 64-bit register, for the packed FP32 instructions,
-// which do both in one issue slot, each half rounded as the scalar instruction rounds it. The unfused form keeps scalar
-// instructions: a packed multiply whose product is added by a packed add came back fused, whatever the rounding
-// qualifiers (the assembly's own bits gave it away), and the plain form rounds every product.
-template <bool PACKED>
-struct Two;
-
-template <>
-struct Two<true>
-{
-    unsigned long long v;
-    static __device__ __forceinline__ Two make(float a, float b)
-    {
-        Two r;
-        asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
-        return r;
-    }
-    static __device__ __forceinline__ Two weight(unsigned long long twice) { return Two{ twice }; }
-    __device__ __forceinline__ void split(float& a, float& b) const
-    {
-        asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-    }
-    // a + b c
-    static __device__ __forceinline__ Two madd(Two a, Two b, Two c)
-    {
-        Two r;
-        asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(b.v), "l"(c.v), "l"(a.v));
-        return r;
-    }
-    static __device__ __forceinline__ Two mul(Two a, Two b)
-    {
-        Two r;
-        asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-        return r;
-    }
-    static __device__ __forceinline__ Two sub(Two a, float x, float y)
-    {
-        Two r, t = make(-x, -y);   // a sign flipped exactly, then added
-        asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(t.v));
-        return r;
-    }
-};
-
-template <>
-struct Two<false>   // one site
-{
-    float v;
-    static __device__ __forceinline__ Two make(float a, float) { return Two{ a }; }
-    static __device__ __forceinline__ Two weight(float w) { return Two{ w }; }
-    __device__ __forceinline__ void split(float& a, float& b) const { a = b = v; }
-    static __device__ __forceinline__ Two madd(Two a, Two b, Two c) { return Two{ __fadd_rn(a.v, __fmul_rn(b.v, c.v)) }; }
-    static __device__ __forceinline__ Two mul(Two a, Two b) { return Two{ __fmul_rn(a.v, b.v) }; }
-    static __device__ __forceinline__ Two sub(Two a, float x, float) { return Two{ a.v - x }; }
-};
-
-// MIXED (the adjoint form, whose stencil and sums are FP32): the same terms with fused multiply-adds and the gradient
-// term summed and stored in FP32 - half the instructions of the reference's unfused float arithmetic, no FP64 work per
-// output and half the bytes of the terms.
-//
-// A block takes A.span consecutive pixels of a plane in rounds, the last two warps their centre sites and the others
-// their fractional sites, U to a lane: a warp's lanes agree on which kind they are, its targets are one contiguous run, staged in shared
-// memory by 16-byte asynchronous copies while the lanes sample the latents, and a pixel's sites are written by one block
-// (half-written sectors cost a read of DRAM each). A lane reading its own row of targets from global memory touches a
-// line per lane and load, NOUT times over, which together with the 64-bit index divisions and the guards of run-time
-// channel counts was most of the kernel: it is bound by issue, and these are instructions. Fused, a lane's two sites go
-// through the packed FP32 instructions; unfused, one site a lane keeps the occupancy (two: 592 -> 683 us at 4 x 2048 x
-// 1024). C0, C1: the channel counts, or 0, 0 to take the launch's (any count with guarded loops; the counts with C1 = 4,
-// the encoder's default, have their own kernels).
-template <bool LEVEL0, int NOUT, bool MIXED, int C0, int C1>
-__global__ void __launch_bounds__(SITE_BLOCK_MAX) k_site_terms(Planes P, const __grid_constant__ SiteArgs A,
-                                                               const __grid_constant__ SiteDecoder<MIXED> W)
-{
-    constexpr int U = MIXED ? 2 : 1, RUN = 32 * U, PIXELS = 64 * U;   // PIXELS: the pixels of one round of the block
-    extern __shared__ __align__(16) float targets[];   // [warp][RUN][NOUT]
-    const long long base = (long long)blockIdx.x * A.span;
-    const int pl = plane_of(P, base);
-    const PlaneView& V = P.p[pl];
-    const int kc = P.kc, per = 1 + kc, c0 = C0 ? C0 : P.c0, c1 = C1 ? C1 : P.c1;
-    const unsigned pixels = (unsigned)V.w0 * (unsigned)V.h0, pixel00 = (unsigned)(base - P.start[pl]);
-    if (pixel00 >= pixels)
-        return;
-    const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const bool centre = warp >= 2 * (unsigned)kc;
-    const unsigned each = centre ? 1 : (unsigned)kc;            // the warp's sites per pixel
-    const unsigned first = (centre ? warp - 2 * (unsigned)kc : warp) * RUN;   // its first site of a round
-    float* mine = targets + warp * RUN * NOUT;
-    const float* all = centre ? V.src : A.tgt + (size_t)A.tsite0[pl] * NOUT;
-    // a division by a power of two is the product with its exact reciprocal, the same bits; 0: not one
-    const float inv_w = (V.w0 & (V.w0 - 1)) == 0 ? 1.0f / (float)V.w0 : 0.0f;
-    const float inv_h = (V.h0 & (V.h0 - 1)) == 0 ? 1.0f / (float)V.h0 : 0.0f;
-    const unsigned inv_each = (65536 + each - 1) / each;   // n / each = (n inv_each) >> 16, n < 2^10
-    int row0 = (int)(pixel00 / (unsigned)V.w0), col0 = (int)(pixel00 - (unsigned)row0 * (unsigned)V.w0);
-#pragma unroll 1
-    for (unsigned pixel0 = pixel00; pixel0 < min(pixel00 + A.span, pixels); pixel0 += PIXELS, col0 += PIXELS)
-    {
-        const unsigned end = min((unsigned)PIXELS, pixels - pixel0) * each;   // the warp's kind of sites in this round
-        if (first >= end)
-            return;
-        const unsigned run = min((unsigned)RUN, end - first) * NOUT;   // the warp's floats
-        const float* from = all + ((size_t)pixel0 * each + first) * NOUT;
-        __syncwarp();   // the last round's targets are spent
-        if (((size_t)from & 15) == 0)
-        {
-            for (unsigned i = lane; i < run / 4; i += 32)
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(mine + 4 * i)),
-                             "l"(from + 4 * i)
-                             : "memory");
-            for (unsigned i = run / 4 * 4 + lane; i < run; i += 32)
-                mine[i] = __ldg(from + i);
-        }
-        else
-            for (unsigned i = lane; i < run; i += 32)
-                mine[i] = __ldg(from + i);
-        while (col0 >= V.w0)
-        {
-            col0 -= V.w0;
-            row0++;
-        }
-        float s_[2][MAX_CH] = {}, c_[2][MAX_CH] = {};
-        size_t site[2] = { 0, 0 };
-#pragma unroll
-        for (int u = 0; u < U; u++)
-        {
-            const unsigned n = min(first + lane + 32 * u, end - 1);   // past the end: the last site again, not stored
-            const unsigned in = (n * inv_each) >> 16, pixel = pixel0 + in;
-            const int j = centre ? 0 : 1 + (int)(n - in * each);
-            int py = row0, px = col0 + (int)in;
-            while (px >= V.w0)
-            {
-                px -= V.w0;
-                py++;
-            }
-            float dx, dy;
-            dx = dy = 0.0f;
-            if (j > 0)
-                subtexel_turned(kc, j - 1, px, py, dx, dy);
-            const Tap tp = tap_scaled(px, py, dx, dy, V.w0, V.h0, V.w1, V.h1, inv_w, inv_h);
-            if constexpr (C1 > 0)
-                blend_c<C1>(V.v1, V.w1, tp, c_[u]);
-            else
-                blend_u<MAX_CH>(V.v1, V.w1, c1, tp, c_[u]);
-            if (centre)
-            {
-#pragma unroll
-                for (int i = 0; i < MAX_CH; i++)
-                    if (i < c0)
-                        s_[u][i] = __ldg(V.v0 + (size_t)pixel * c0 + i);
-            }
-            else
-            {
-                const Tap t0 = tap_at(px, py, dx, dy, V.w0, V.h0, V.w0, V.h0);
-                if constexpr (C0 > 0)
-                    blend_c<C0>(V.v0, V.w0, t0, s_[u]);
-                else
-                    blend_u<MAX_CH>(V.v0, V.w0, c0, t0, s_[u]);
-            }
-            site[u] = (size_t)A.site0[pl] + (size_t)pixel * per + j;
-        }
-        using F2 = Two<MIXED>;
-        F2 sbar[MAX_CH], cbar[MAX_CH], accf[MAX_CH];
-        double acc[MAX_CH];
-#pragma unroll
-        for (int a = 0; a < MAX_CH; a++)
-        {
-            sbar[a] = F2::make(s_[0][a], s_[1][a]);
-            cbar[a] = F2::make(c_[0][a], c_[1][a]);
-            accf[a] = F2::make(0.0f, 0.0f);
-            acc[a] = 0.0;
-        }
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        __syncwarp();
-        const float* tgt = mine + lane * NOUT;
-        const float* tgt2 = mine + min(lane + 32 * (U - 1), end - 1 - first) * NOUT;
-        // a + b c, unfused (the reference's rounding) or fused (MIXED)
-        auto madd = [](F2 a, F2 b, F2 c) { return F2::madd(a, b, c); };
-#pragma unroll
-        for (int r = 0; r < NOUT; r++)
-        {
-            auto row = [&](int q) { return F2::weight(W.w[r * 24 + q]); };   // [c_q][s_i][s_i c_q]
-            F2 out = F2::weight(W.b[r]);
-            F2 col[MAX_CH];
-            if (!LEVEL0)
-            {
-#pragma unroll
-                for (int i = 0; i < MAX_CH; i++)
-                    if (i < c0)
-                        out = madd(out, row(4 + i), sbar[i]);
-#pragma unroll
-                for (int q = 0; q < MAX_CH; q++)
-                    if (q < c1)
-                    {
-                        F2 gg = row(q);
-#pragma unroll
-                        for (int i = 0; i < MAX_CH; i++)
-                            if (i < c0)
-                                gg = madd(gg, sbar[i], row(8 + i * 4 + q));
-                        col[q] = gg;
-                        out = madd(out, gg, cbar[q]);
-                    }
-            }
-            else
-            {
-#pragma unroll
-                for (int q = 0; q < MAX_CH; q++)
-                    if (q < c1)
-                        out = madd(out, row(q), cbar[q]);
-#pragma unroll
-                for (int i = 0; i < MAX_CH; i++)
-                    if (i < c0)
-                    {
-                        F2 qq = row(4 + i);
-#pragma unroll
-                        for (int q = 0; q < MAX_CH; q++)
-                            if (q < c1)
-                                qq = madd(qq, cbar[q], row(8 + i * 4 + q));
-                        col[i] = qq;
-                        out = madd(out, qq, sbar[i]);
-                    }
-            }
-            const F2 res = F2::sub(out, tgt[r], tgt2[r]);
-            const int c = LEVEL0 ? c0 : c1;
-            if (MIXED)
-            {
-#pragma unroll
-                for (int a = 0; a < MAX_CH; a++)
-                    if (a < c)
-                        accf[a] = madd(accf[a], F2::mul(F2::weight(W.cw[r]), col[a]), res);
-            }
-            else
-            {
-                float r0, g0, unused;
-                res.split(r0, unused);
-                const double d0 = (double)r0, cwd = W.cwd[r];
-#pragma unroll
-                for (int a = 0; a < MAX_CH; a++)
-                    if (a < c)
-                    {
-                        col[a].split(g0, unused);
-                        acc[a] += cwd * (double)g0 * d0;
-                    }
-            }
-        }
-        const int c = LEVEL0 ? c0 : c1, ny = LEVEL0 ? c1 : c0;
-        float f_[2][MAX_CH];
-#pragma unroll
-        for (int a = 0; a < MAX_CH; a++)
-            accf[a].split(f_[0][a], f_[1][a]);
-#pragma unroll
-        for (int u = 0; u < U; u++)
-        {
-            if (first + lane + 32 * u >= end)
-                continue;
-            if (MIXED)
-            {
-                float* out = static_cast<float*>(A.terms) + site[u] * c;
-                if (c == MAX_CH)
-                    *reinterpret_cast<float4*>(out) = make_float4(f_[u][0], f_[u][1], f_[u][2], f_[u][3]);
-                else
-                {
-#pragma unroll
-                    for (int a = 0; a < MAX_CH; a++)
-                        if (a < c)
-                            out[a] = f_[u][a];
-                }
-            }
-            else
-            {
-                double* out = static_cast<double*>(A.terms) + site[u] * c;
-                if (c == MAX_CH)
-                {
-                    reinterpret_cast<double2*>(out)[0] = make_double2(acc[0], acc[1]);
-                    reinterpret_cast<double2*>(out)[1] = make_double2(acc[2], acc[3]);
-                }
-                else
-                {
-#pragma unroll
-                    for (int a = 0; a < MAX_CH; a++)
-                        if (a < c)
-                            out[a] = acc[a];
-                }
-            }
-            // the other latent's sample, which every (texel, slot) of the gather that meets this site needs again
-            float y[MAX_CH];
-#pragma unroll
-            for (int i = 0; i < MAX_CH; i++)
-                y[i] = i < ny ? (LEVEL0 ? c_[u][i] : s_[u][i]) : 0.0f;
-            A.y[site[u]] = make_float4(y[0], y[1], y[2], y[3]);
-        }
-    }
-}
-
-template <bool LEVEL0, int NOUT, bool MIXED>
-static void launch_site_terms(const nntc_b200_device* d, const Planes& S, SiteArgs A, cudaStream_t stream)
-{
-    using Weight = typename SiteDecoder<MIXED>::Weight;
-    SiteDecoder<MIXED> W{};
-    const int nin = d->nin, c0 = d->c0, c1 = d->c1;
-    auto weight = [](float v) {
-        if (!MIXED)
-            return (Weight)v;
-        unsigned bits;
-        std::memcpy(&bits, &v, sizeof(bits));
-        return (Weight)((unsigned long long)bits << 32 | bits);
-    };
-    for (int r = 0; r < d->nout; r++)
-    {
-        for (int q = 0; q < c1; q++)
-            W.w[r * 24 + q] = weight(d->host_weights[(size_t)r * nin + q]);
-        for (int i = 0; i < c0; i++)
-            W.w[r * 24 + 4 + i] = weight(d->host_weights[(size_t)r * nin + c1 + i]);
-        for (int i = 0; i < c0; i++)
-            for (int q = 0; q < c1; q++)
-                W.w[r * 24 + 8 + i * 4 + q] = weight(d->host_weights[(size_t)r * nin + c1 + c0 + i * c1 + q]);
-        W.b[r] = weight(d->host_bias[r]);
-        W.cw[r] = weight(d->m.cw[r]);
-        W.cwd[r] = (double)d->m.cw[r];
-    }
-    constexpr int U = MIXED ? 2 : 1;
-    A.span = S.start[S.n] < SITE_FEW ? 64 * U : SITE_PIXELS;
-    const int blocks = (int)(S.start[S.n] / A.span), threads = 64 * (1 + S.kc);
-    const size_t shared = (size_t)threads * U * NOUT * sizeof(float);
-    if (S.c1 != MAX_CH)
-        k_site_terms<LEVEL0, NOUT, MIXED, 0, 0><<<blocks, threads, shared, stream>>>(S, A, W);
-    else if (S.c0 == 1)
-        k_site_terms<LEVEL0, NOUT, MIXED, 1, 4><<<blocks, threads, shared, stream>>>(S, A, W);
-    else if (S.c0 == 2)
-        k_site_terms<LEVEL0, NOUT, MIXED, 2, 4><<<blocks, threads, shared, stream>>>(S, A, W);
-    else if (S.c0 == 3)
-        k_site_terms<LEVEL0, NOUT, MIXED, 3, 4><<<blocks, threads, shared, stream>>>(S, A, W);
-    else
-        k_site_terms<LEVEL0, NOUT, MIXED, 4, 4><<<blocks, threads, shared, stream>>>(S, A, W);
-}
-
 // ---- the gather's visit tables (gather.cuh)
 
 // Every class's visits, in the reference's site order, for the FP64 sums (tab64) and the FP32 sums (tab32: the product
@@ -503,152 +140,6 @@ static bool build_gather_table(int kc, std::vector<int4>& tab64, std::vector<int
     return true;
 }
 
-// The texel at position `pos` of the stencil's colour-major order (the inverse of stencil_pos).
-__device__ __forceinline__ void stencil_texel(long long pos, int w, int h, int& x, int& y)
-{
-    const long long w0c = (w + 1) >> 1, w1c = w >> 1, h0c = (h + 1) >> 1, h1c = h >> 1;
-    const long long n0 = w0c * h0c, n1 = w1c * h0c, n2 = w0c * h1c;
-    int cx = 0, cy = 0;
-    long long r = pos, rw = w0c;
-    if (r >= n0 + n1 + n2)
-    {
-        r -= n0 + n1 + n2;
-        cx = 1;
-        cy = 1;
-        rw = w1c;
-    }
-    else if (r >= n0 + n1)
-    {
-        r -= n0 + n1;
-        cy = 1;
-    }
-    else if (r >= n0)
-    {
-        r -= n0;
-        cx = 1;
-        rw = w1c;
-    }
-    x = 2 * (int)(r % rw) + cx;
-    y = 2 * (int)(r / rw) + cy;
-}
-
-// The gather of the planes no tile takes (planes one texel wide or high at level 0, level-1 planes whose tile would not
-// fit shared memory or that are above any_tiles_line): one thread per (texel, slot) tests every site of the two texels' common
-// footprint, in site order; the self-slot thread also gathers the gradient. Blocks run in (region, colour, slot) order,
-// the slot fastest, so that the five slots of one run of texels and the four colours of one region run side by side
-// and share the region's sites in L2.
-constexpr int WALK_THREADS = 128;
-
-struct WalkBlocks
-{
-    long long start[MAX_PLANES + 1];   // each plane's first block (a tiled plane has none)
-};
-
-template <bool LEVEL0, typename TS, int NY>
-__global__ void __launch_bounds__(WALK_THREADS) k_gather_walk(Planes P, const __grid_constant__ TileArgs<TS> A,
-                                                               const __grid_constant__ WalkBlocks B)
-{
-    using TT = TS;   // the terms' type
-    int pl = 0;
-    while (pl + 1 < P.n && B.start[pl + 1] <= (long long)blockIdx.x)
-        pl++;
-    const long long lb = (long long)blockIdx.x - B.start[pl];
-    const int slot = (int)(lb % A.slots);
-    const int colour = (int)((lb / A.slots) % 4);
-    const long long region = lb / A.slots / 4;
-    const PlaneView& V = P.p[pl];
-    const int tw_ = V.w, th_ = V.h;
-    const long long w0c = (tw_ + 1) >> 1, w1c = tw_ >> 1, h0c = (th_ + 1) >> 1, h1c = th_ >> 1;
-    const long long n0 = w0c * h0c, n1 = w1c * h0c, n2 = w0c * h1c, n3 = w1c * h1c;
-    const long long ncol = colour == 0 ? n0 : (colour == 1 ? n1 : (colour == 2 ? n2 : n3));
-    const long long within = region * WALK_THREADS + threadIdx.x;
-    if (within >= ncol)
-        return;
-    // the texel's place in the stencil's colour-major order
-    const long long sp = within + (colour == 0 ? 0 : (colour == 1 ? n0 : (colour == 2 ? n0 + n1 : n0 + n1 + n2)));
-    const int kc = P.kc, per = 1 + kc;
-    const int c = LEVEL0 ? P.c0 : P.c1;
-    int tx, ty;
-    stencil_texel(sp, tw_, th_, tx, ty);
-    int ox, oy;
-    slot_offset(slot, ox, oy);
-    const int nbx = tx + ox, nby = ty + oy;
-    const size_t T = (size_t)tw_ * th_;
-    if (nbx < 0 || nbx >= tw_ || nby >= th_)
-    {
-        store_zero_block<TS>(A, V, slot, c, tx, ty, T, (size_t)sp);
-        return;
-    }
-    TS sums[MAX_MONO];
-#pragma unroll
-    for (int i = 0; i < MAX_MONO; i++)
-        sums[i] = (TS)0;
-    double g[MAX_CH];
-#pragma unroll
-    for (int a = 0; a < MAX_CH; a++)
-        g[a] = 0.0;
-    const TT* terms = (const TT*)A.terms + (size_t)A.site0[pl] * c;
-    const float4* ys = A.y + A.site0[pl];
-    // the pixel range of sites that can touch both texels: the intersection of their footprints
-    int px_lo, px_hi, py_lo, py_hi, qx_lo, qx_hi, qy_lo, qy_hi;
-    reach(tx, V.w0, tw_, px_lo, px_hi);
-    reach(ty, V.h0, th_, py_lo, py_hi);
-    reach(nbx, V.w0, tw_, qx_lo, qx_hi);
-    reach(nby, V.h0, th_, qy_lo, qy_hi);
-    px_lo = max(px_lo, qx_lo);
-    px_hi = min(px_hi, qx_hi);
-    py_lo = max(py_lo, qy_lo);
-    py_hi = min(py_hi, qy_hi);
-    for (int py = py_lo; py <= py_hi; py++)
-        for (int px = px_lo; px <= px_hi; px++)
-            for (int j = 0; j <= kc; j++)
-            {
-                float ws, wo;
-                if (!site_touches<LEVEL0>(px, py, j, kc, tx, ty, nbx, nby, V.w0, V.h0, tw_, th_, ws, wo))
-                    continue;
-                const size_t site = ((size_t)py * V.w0 + px) * per + j;
-                if (slot == 0)
-                {
-#pragma unroll
-                    for (int a = 0; a < MAX_CH; a++)
-                        if (a < c)
-                            g[a] += (double)ws * (double)__ldg(terms + site * c + a);
-                }
-                visit_sums<TS, NY, 0, MAX_MONO>(sums, __ldg(ys + site), (TS)ws * (TS)wo);
-            }
-    expand_block<TS, NY>(A, V, sums, slot, c, tx, ty, T, (size_t)sp);
-    if (slot == 0)
-    {
-#pragma unroll
-        for (int a = 0; a < MAX_CH; a++)
-            if (a < c)
-                V.grad[((size_t)ty * tw_ + tx) * c + a] = g[a];
-    }
-}
-
-template <typename TS>
-static int launch_walk(nntc_b200_device* d, int level0, const Planes& P, const TileArgs<TS>& A, const WalkBlocks& B)
-{
-    const unsigned grid = (unsigned)B.start[P.n];
-    const int ny = level0 ? d->c1 : d->c0;
-#define NB_WALK(NY)                                                                                                   \
-    if (level0)                                                                                                       \
-        k_gather_walk<true, TS, NY><<<grid, WALK_THREADS, 0, d->stream>>>(P, A, B);                                   \
-    else                                                                                                              \
-        k_gather_walk<false, TS, NY><<<grid, WALK_THREADS, 0, d->stream>>>(P, A, B);                                  \
-    break;
-    switch (ny)
-    {
-    case 1: NB_WALK(1)
-    case 2: NB_WALK(2)
-    case 3: NB_WALK(3)
-    default: NB_WALK(4)
-    }
-#undef NB_WALK
-    NB_LAUNCHED();
-    return NNTC_B200_OK;
-}
-
 // The tiles of k_gather_any1 up to which it takes a level's planes that are not tabled; with more of them the walk does.
 // The tiles test each pixel once for five warps, whatever comes of it, and stage its sites, which pays the more sites a
 // pixel has; a thread a (texel, slot) waits longer but keeps more of them in flight, so that it gains as the launch
@@ -673,6 +164,19 @@ static int any_tiles_line(bool f32, int c, int sites, bool every_slot)
         return base * sites * sites;
     return staged ? base / 2 * sites * sites : base * 3 / 4 * sites;
 }
+
+// One of the gather's launches, for the other latent's channel count (ny).
+#define NB_GATHER(launch, ...)                                                                                        \
+    do                                                                                                                \
+    {                                                                                                                 \
+        switch (ny)                                                                                                   \
+        {                                                                                                             \
+        case 1: NB_TRY((launch<TS, 1>(__VA_ARGS__))); break;                                                          \
+        case 2: NB_TRY((launch<TS, 2>(__VA_ARGS__))); break;                                                          \
+        case 3: NB_TRY((launch<TS, 3>(__VA_ARGS__))); break;                                                          \
+        default: NB_TRY((launch<TS, 4>(__VA_ARGS__))); break;                                                         \
+        }                                                                                                             \
+    } while (0)
 
 // The gather of every plane: the tabled planes in one launch, the others in one more, or two.
 template <typename TS>
@@ -789,7 +293,7 @@ static int gather_planes(nntc_b200_device* d, int level0, const Planes& P, int n
     for (int i = P.n - 1; i >= 0; i--)
         A.bend[i] = tiles += A.btiles[i];
     if (walk > 0)
-        NB_TRY(launch_walk<TS>(d, level0, P, A, B));
+        NB_GATHER(launch_gather_walk, d, level0, P, A, B);
     for (int group = 0; group < 2 && any_tiles > 0; group++)   // the larger tiles, then the others
     {
         TileArgs<TS> G = A;
@@ -803,10 +307,10 @@ static int gather_planes(nntc_b200_device* d, int level0, const Planes& P, int n
             G.bend[i] = blocks += G.btiles[i];
         }
         if (blocks > 0)
-            NB_TRY(launch_gather_any(d, P, G, R, (unsigned)blocks, shared));
+            NB_GATHER(launch_gather_any, d, P, G, R, (unsigned)blocks, shared);
     }
     if (tiles > 0)
-        NB_TRY(launch_gather_tiles(d, level0, P, A, (unsigned)tiles));
+        NB_GATHER(launch_gather_tiles, d, level0, P, A, (unsigned)tiles);
     return NNTC_B200_OK;
 }
 
@@ -883,17 +387,10 @@ int assemble_split(nntc_b200_device* d, int k, int level0, const Planes& P_texel
     NB_TRY(ensure_site_targets(d, k, level0));
 #define NB_SITES(NO)                                                                                                  \
     case NO:                                                                                                          \
-        if (level0)                                                                                                   \
-        {                                                                                                             \
-            if (f32)                                                                                                  \
-                launch_site_terms<true, NO, true>(d, S, A, d->stream);                                                \
-            else                                                                                                      \
-                launch_site_terms<true, NO, false>(d, S, A, d->stream);                                               \
-        }                                                                                                             \
-        else if (f32)                                                                                                 \
-            launch_site_terms<false, NO, true>(d, S, A, d->stream);                                                   \
+        if (f32)                                                                                                      \
+            launch_site_terms<NO, true>(d, S, A, level0, d->stream);                                                  \
         else                                                                                                          \
-            launch_site_terms<false, NO, false>(d, S, A, d->stream);                                                  \
+            launch_site_terms<NO, false>(d, S, A, level0, d->stream);                                                 \
         break;
     switch (d->nout)
     {

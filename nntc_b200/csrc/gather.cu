@@ -12,28 +12,18 @@
 // load, and the arithmetic (FP64: 41 visits x 40 operations + the expansions at level 0, 800 visits x 40 at level 1)
 // is what is left. The smallest planes run first: their few blocks walk as long as any other's, and at the end of the
 // launch nothing would run beside them.
+//
+// Compiled once per type of the sums and channel count of the other latent (NB_TYPE, NB_NY), a module each: a launch loads
+// the kernels of its own counts alone (site_terms.cu).
 
 #include <type_traits>
 
-#include "footprint.cuh"
 #include "gather.cuh"
 
 namespace nb
 {
 
 constexpr int TILE0_THREADS = 256;   // a warp per texel row and x parity
-constexpr int TILE1_THREADS = 160;   // five warps: see k_gather_tile1
-
-__device__ __forceinline__ void cp_async16(void* dst, const void* src)
-{
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
-                 : "memory");
-}
-
-__device__ __forceinline__ void cp_async_wait_all()
-{
-    asm volatile("cp.async.wait_all;" ::: "memory");
-}
 
 template <typename TS>
 __device__ __forceinline__ TS visit_scale(const int4& e);
@@ -46,17 +36,6 @@ template <>
 __device__ __forceinline__ float visit_scale<float>(const int4& e)
 {
     return __int_as_float(e.z);
-}
-
-// The plane of a block (planes in descending order) and the block's number within the plane.
-template <typename TS>
-__device__ __forceinline__ int tile_plane(const TileArgs<TS>& A, int n, int& tile)
-{
-    int pl = n - 1;
-    while ((int)blockIdx.x >= A.bend[pl])
-        pl--;
-    tile = (int)blockIdx.x - (A.bend[pl] - A.btiles[pl]);
-    return pl;
 }
 
 // The sums of one slot: every visit of the list, in order, GROUP samples loaded ahead of their additions and the next
@@ -232,38 +211,6 @@ __global__ void __launch_bounds__(TILE0_THREADS, (sizeof(TS) == sizeof(float) ? 
     }
 }
 
-// The gradient terms of channels first .. (two of FP64, four of FP32) in the samples' places, asynchronously where a
-// site's are 16 aligned bytes.
-template <typename TS, class Each>
-__device__ __forceinline__ void stage_terms(const TileArgs<TS>& A, float4* sy, int first, int c, Each each_site)
-{
-    constexpr int CH = sizeof(TS) == sizeof(float) ? 4 : 2;
-    if constexpr (sizeof(TS) == sizeof(float))
-    {
-        const float* t = (const float*)A.terms;
-        if (c == MAX_CH)
-            each_site([&](int at, size_t site) { cp_async16(sy + at, t + site * MAX_CH); });
-        else
-            each_site([&](int at, size_t site) {
-                float* dst = reinterpret_cast<float*>(sy + at);
-                for (int a = 0; a < c; a++)
-                    dst[a] = __ldg(t + site * c + a);
-            });
-    }
-    else
-    {
-        const double* t = (const double*)A.terms + first;
-        if (c % 2 == 0)
-            each_site([&](int at, size_t site) { cp_async16(sy + at, t + site * c); });
-        else
-            each_site([&](int at, size_t site) {
-                double* dst = reinterpret_cast<double*>(sy + at);
-                for (int a = 0; a < CH && first + a < c; a++)
-                    dst[a] = __ldg(t + site * c + a);
-            });
-    }
-}
-
 // Level 1: a tile of 8 x 4 texels, one per lane, and five warps of equal work: the self slot's visits (320 inside a
 // plane) are walked by two warps, each summing half of the monomials, the right and the down slot's (160 each) by one
 // warp each, the two diagonal slots' (80 each) by one. The gradient's terms, as many bytes again as the samples or
@@ -392,303 +339,18 @@ __global__ void __launch_bounds__(TILE1_THREADS, 3) k_gather_tile1(Planes P, con
     }
 }
 
-// Level 1 planes of any other ratio or size: the tile's texels, warps and phases of k_gather_tile1, but no two texels
-// share a visit list, so each lane walks the pixels its texel can meet and tests every site. What made that walk slow
-// was recomputing each site's taps (two divisions, two floors and the subtexel's turns) in every (texel, slot) thread,
-// reading the samples of the sites that pass from L2, and a branch around every site, so that nothing of the next site
-// started before this one's sums were done. Here the taps are separable - the column tap of pixel px and site j depends
-// on the pixel row's parity alone, and the other way round - so a block forms each column's and row's once, with
-// tap_at's arithmetic, next to the staged samples; and a pixel's sites are taken side by side, one that misses the texel
-// entering the sums with weight, sample and term zero, whose exact zeros leave them as they were (a sum is never -0).
-struct __align__(16) AxisTap
+template <typename TS, int NY>
+int launch_gather_tiles(nntc_b200_device* d, int level0, const Planes& P, const TileArgs<TS>& A, unsigned grid)
 {
-    int a, b;        // the two texels, clamped
-    float wa, wb;    // 1 - f, f
-};
-
-// The weight with which a site's two taps land on texel (x, y): the corner weights that do, summed in corner order
-// (site_touches). Away from the plane's borders no tap is clamped and at most one corner does (EDGE false).
-template <bool EDGE>
-__device__ __forceinline__ float corner_weight(const AxisTap& ax, const AxisTap& ay, int x, int y, bool& touches)
-{
-    const bool x0 = ax.a == x, x1 = ax.b == x, y0 = ay.a == y, y1 = ay.b == y;
-    touches = (x0 || x1) && (y0 || y1);
-    if (!EDGE)
-        return (x0 ? ax.wa : ax.wb) * (y0 ? ay.wa : ay.wb);
-    float w = 0.0f;
-    if (x0 && y0)
-        w += ax.wa * ay.wa;
-    if (x1 && y0)
-        w += ax.wb * ay.wa;
-    if (x0 && y1)
-        w += ax.wa * ay.wb;
-    if (x1 && y1)
-        w += ax.wb * ay.wb;
-    return w;
-}
-
-// PER: sites a pixel (1 + K), or 0 to take P.kc's.
-template <typename TS, int NY, int PER>
-__global__ void __launch_bounds__(TILE1_THREADS, 3) k_gather_any1(Planes P, const __grid_constant__ TileArgs<TS> A,
-                                                                  const __grid_constant__ AnyTiles R)
-{
-    constexpr int SPLIT = NY == 4 ? 8 : (NY == 3 ? 7 : (NY == 2 ? 3 : 2));
-    extern __shared__ float4 sy[];
-    __shared__ TS other[MAX_MONO][32];
-    int tile;
-    const int pl = tile_plane(A, P.n, tile);
-    const PlaneView& V = P.p[pl];
-    const int w = V.w, h = V.h, kc = P.kc, per = PER ? PER : 1 + kc, c = P.c1;
-    const int tiles_x = (w + TILE1_W - 1) / TILE1_W;
-    const int x0 = tile % tiles_x * TILE1_W, y0 = tile / tiles_x * TILE1_H;
-    const int rw = R.px[pl], rh = R.py[pl], quads = (rw + 3) / 4, run = rw * per, row = quads * 4 * per;
-    const int inv = (65536 + per - 1) / per;
-    int first_x, first_y, unused;
-    reach(x0, V.w0, w, first_x, unused);
-    reach(y0, V.h0, h, first_y, unused);
-    // [column][j][row parity], then [row][j][column parity]; one entry of padding after every four columns, which lanes
-    // are apart, keeps a warp's reads off one bank
-    AxisTap* tap_x = reinterpret_cast<AxisTap*>(sy + (size_t)row * rh);
-    AxisTap* tap_y = tap_x + any_taps(rw, per);
-    auto place = [&](int qx, int qy, int j) { return ((qy * per + j) * 4 + (qx & 3)) * quads + (qx >> 2); };
-    auto each_site = [&](auto f) {
-        for (int r = threadIdx.x; r < run; r += TILE1_THREADS)
-        {
-            const int qx = (r * inv) >> 16, j = r - qx * per, px = first_x + qx;
-            if (px >= V.w0)
-                continue;
-            const size_t site = (size_t)A.site0[pl] + ((size_t)first_y * V.w0 + px) * per + j;
-            const int at = place(qx, 0, j);
-#pragma unroll 4
-            for (int qy = 0; qy < rh; qy++)
-                if (first_y + qy < V.h0)
-                    f(at + qy * row, site + (size_t)qy * V.w0 * per);
-        }
-    };
-    each_site([&](int at, size_t site) { cp_async16(sy + at, A.y + site); });
-    for (int i = threadIdx.x; i < (rw + rh) * per * 2; i += TILE1_THREADS)
-    {
-        const bool col = i < run * 2;
-        const int q = col ? i : i - run * 2, cell = q >> 1, odd = q & 1, at = (cell * inv) >> 16, j = cell - at * per;
-        const int px = col ? first_x + at : odd, py = col ? odd : first_y + at;
-        float dx, dy;
-        site_offset(kc, j, px, py, dx, dy);
-        const Tap t = tap_at(px, py, dx, dy, V.w0, V.h0, w, h);
-        (col ? tap_x : tap_y)[q + (at >> 2)] =
-            col ? AxisTap{ t.x0, t.x1, 1.0f - t.fx, t.fx } : AxisTap{ t.y0, t.y1, 1.0f - t.fy, t.fy };
-    }
-    cp_async_wait_all();
-    __syncthreads();
-
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int tx = x0 + (lane & (TILE1_W - 1)), ty = y0 + lane / TILE1_W;
-    const bool active = tx < w && ty < h;
-    const bool edge = __any_sync(0xffffffffu, active && (tx == 0 || ty == 0 || tx == w - 1 || ty == h - 1));
-    const size_t T = (size_t)w * h, sp = active ? stencil_pos(tx, ty, w, h) : 0;
-    // every site of the pixels that can meet both (tx, ty) and the slot's neighbour, in site order: f(j, place, whether
-    // it touches both, w_self, w_other) for the sites of a pixel, then g() for the pixel
-    auto pixels = [&](auto edges, int slot, auto f, auto g) {
-        constexpr bool EDGE = decltype(edges)::value;
-        int ox, oy;
-        slot_offset(slot, ox, oy);
-        const int nbx = tx + ox, nby = ty + oy;
-        int px_lo, px_hi, py_lo, py_hi, qx_lo, qx_hi, qy_lo, qy_hi;
-        reach(tx, V.w0, w, px_lo, px_hi);
-        reach(ty, V.h0, h, py_lo, py_hi);
-        reach(nbx, V.w0, w, qx_lo, qx_hi);
-        reach(nby, V.h0, h, qy_lo, qy_hi);
-        px_lo = max(px_lo, qx_lo);
-        px_hi = min(px_hi, qx_hi);
-        py_lo = max(py_lo, qy_lo);
-        py_hi = min(py_hi, qy_hi);
-        for (int py = py_lo; py <= py_hi; py++)
-            for (int px = px_lo; px <= px_hi; px++)
-            {
-                const int qx = px - first_x, qy = py - first_y;
-                const AxisTap* cols = tap_x + qx * per * 2 + (qx >> 2) + (py & 1);
-                const AxisTap* rows = tap_y + qy * per * 2 + (qy >> 2) + (px & 1);
-                const int at = place(qx, qy, 0);
-#pragma unroll
-                for (int j = 0; j < (PER ? PER : MAX_SITES); j++)
-                {
-                    if (!PER && j >= per)
-                        break;
-                    const AxisTap ax = cols[2 * j], ay = rows[2 * j];
-                    bool self, both = true;
-                    const float ws = corner_weight<EDGE>(ax, ay, tx, ty, self);
-                    const float wo = slot ? corner_weight<EDGE>(ax, ay, nbx, nby, both) : ws;
-                    f(j, at + j * 4 * quads, self && both, ws, wo);
-                }
-                g();
-            }
-    };
-    TS sums[MAX_MONO];
-#pragma unroll
-    for (int i = 0; i < MAX_MONO; i++)
-        sums[i] = (TS)0;
-    auto sum_slot = [&](auto lo, auto hi, int slot) {
-        constexpr int LO = decltype(lo)::value, HI = decltype(hi)::value;
-        float4 y[MAX_SITES];
-        TS scale[MAX_SITES];
-        auto site = [&](int j, int at, bool hit, float ws, float wo) {
-            const float4 v = sy[at];
-            y[j] = hit ? v : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            scale[j] = hit ? (TS)ws * (TS)wo : (TS)0;
-        };
-        auto pixel = [&]() {
-#pragma unroll
-            for (int j = 0; j < (PER ? PER : MAX_SITES); j++)
-                if (PER || j < per)
-                    visit_sums<TS, NY, LO, HI>(sums, y[j], scale[j]);
-        };
-        if (edge)
-            pixels(std::true_type{}, slot, site, pixel);
-        else
-            pixels(std::false_type{}, slot, site, pixel);
-    };
-    using Lo = std::integral_constant<int, 0>;
-    using Mid = std::integral_constant<int, SPLIT>;
-    using Hi = std::integral_constant<int, MAX_MONO>;
-    if (active && warp == 0)
-        sum_slot(Lo{}, Mid{}, 0);
-    else if (active && warp == 4)
-    {
-        sum_slot(Mid{}, Hi{}, 0);
-#pragma unroll
-        for (int L = SPLIT; L < MAX_MONO; L++)
-            if (mono_used(L, NY))
-                other[L][lane] = sums[L];
-    }
-    else if (active)
-    {
-        const int s0 = warp == 1 ? 1 : (warp == 2 ? 3 : 2), s1 = warp == 3 ? 4 : s0;
-#pragma unroll 1
-        for (int slot = s0; slot <= s1 && slot < A.slots; slot += 2)
-        {
-            int ox, oy;
-            slot_offset(slot, ox, oy);
-            if (tx + ox < 0 || tx + ox >= w || ty + oy >= h)
-            {
-                store_zero_block<TS>(A, V, slot, c, tx, ty, T, sp);
-                continue;
-            }
-#pragma unroll
-            for (int i = 0; i < MAX_MONO; i++)
-                sums[i] = (TS)0;
-            sum_slot(Lo{}, Hi{}, slot);
-            expand_block<TS, NY>(A, V, sums, slot, c, tx, ty, T, sp);
-        }
-    }
-    __syncthreads();
-    constexpr int CH = sizeof(TS) == sizeof(float) ? 4 : 2;
-    for (int p = 0; p * CH < c; p++)
-    {
-        const int first = p * CH;
-        stage_terms<TS>(A, sy, first, c, each_site);
-        if (p == 0 && warp == 0 && active)
-        {
-#pragma unroll
-            for (int L = SPLIT; L < MAX_MONO; L++)
-                if (mono_used(L, NY))
-                    sums[L] = other[L][lane];
-            expand_block<TS, NY>(A, V, sums, 0, c, tx, ty, T, sp);
-        }
-        cp_async_wait_all();
-        __syncthreads();
-        const int ch = 2 * (warp - 1);
-        if (active && ch >= first && ch < first + CH && ch < c)
-        {
-            using T2 = typename std::conditional<sizeof(TS) == sizeof(float), float2, double2>::type;
-            double g0 = 0.0, g1 = 0.0;
-            T2 t[MAX_SITES];
-            float weight[MAX_SITES];
-            auto site = [&](int j, int at, bool hit, float ws, float) {
-                const T2 v = *reinterpret_cast<const T2*>(reinterpret_cast<const TS*>(sy + at) + (ch - first));
-                t[j].x = hit ? v.x : 0;
-                t[j].y = hit ? v.y : 0;
-                weight[j] = hit ? ws : 0.0f;
-            };
-            auto pixel = [&]() {
-#pragma unroll
-                for (int j = 0; j < (PER ? PER : MAX_SITES); j++)
-                    if (PER || j < per)
-                    {
-                        g0 += (double)weight[j] * (double)t[j].x;
-                        g1 += (double)weight[j] * (double)t[j].y;
-                    }
-            };
-            if (edge)
-                pixels(std::true_type{}, 0, site, pixel);
-            else
-                pixels(std::false_type{}, 0, site, pixel);
-            double* out = V.grad + ((size_t)ty * w + tx) * c + ch;
-            out[0] = g0;
-            if (ch + 1 < c)
-                out[1] = g1;
-        }
-        __syncthreads();
-    }
-}
-
-template <typename TS>
-static int launch_any(nntc_b200_device* d, const Planes& P, const TileArgs<TS>& A, const AnyTiles& S, unsigned grid,
-                      size_t shared)
-{
-    void (*kernel)(Planes, const TileArgs<TS>, const AnyTiles) = nullptr;
-#define NB_ANY(NY)                                                                                                    \
-    case NY: kernel = P.kc == 4 ? k_gather_any1<TS, NY, 5> : k_gather_any1<TS, NY, 0>; break;
-    switch (d->c0)
-    {
-        NB_ANY(1)
-        NB_ANY(2)
-        NB_ANY(3)
-    default: kernel = P.kc == 4 ? k_gather_any1<TS, 4, 5> : k_gather_any1<TS, 4, 0>; break;
-    }
-#undef NB_ANY
-    NB_SHARED_LIMIT(kernel, ANY_SHARED_MAX);
-    kernel<<<grid, TILE1_THREADS, shared, d->stream>>>(P, A, S);
-    NB_LAUNCHED();
-    return NNTC_B200_OK;
-}
-
-int launch_gather_any(nntc_b200_device* d, const Planes& P, const TileArgs<double>& A, const AnyTiles& S,
-                      unsigned grid, size_t shared)
-{
-    return launch_any<double>(d, P, A, S, grid, shared);
-}
-
-int launch_gather_any(nntc_b200_device* d, const Planes& P, const TileArgs<float>& A, const AnyTiles& S, unsigned grid,
-                      size_t shared)
-{
-    return launch_any<float>(d, P, A, S, grid, shared);
-}
-
-template <typename TS>
-static int launch_tiles(nntc_b200_device* d, int level0, const Planes& P, const TileArgs<TS>& A, unsigned grid)
-{
-    const int per = 1 + P.kc, ny = level0 ? d->c1 : d->c0;
+    const int per = 1 + P.kc;
     const int site = (level0 ? TILE0_PX * TILE0_PY : TILE1_PX * TILE1_PY) * (int)sizeof(float4), shared = site * per;
-    void (*kernel)(Planes, const TileArgs<TS>) = nullptr;
-    if (level0)
-        kernel = ny == 1 ? k_gather_tile0<TS, 1>
-                         : (ny == 2 ? k_gather_tile0<TS, 2> : (ny == 3 ? k_gather_tile0<TS, 3> : k_gather_tile0<TS, 4>));
-    else
-        kernel = ny == 1 ? k_gather_tile1<TS, 1>
-                         : (ny == 2 ? k_gather_tile1<TS, 2> : (ny == 3 ? k_gather_tile1<TS, 3> : k_gather_tile1<TS, 4>));
+    void (*kernel)(Planes, const TileArgs<TS>) = level0 ? k_gather_tile0<TS, NY> : k_gather_tile1<TS, NY>;
     NB_SHARED_LIMIT(kernel, site * MAX_SITES);
     kernel<<<grid, level0 ? TILE0_THREADS : TILE1_THREADS, shared, d->stream>>>(P, A);
     NB_LAUNCHED();
     return NNTC_B200_OK;
 }
 
-int launch_gather_tiles(nntc_b200_device* d, int level0, const Planes& P, const TileArgs<double>& A, unsigned grid)
-{
-    return launch_tiles<double>(d, level0, P, A, grid);
-}
-
-int launch_gather_tiles(nntc_b200_device* d, int level0, const Planes& P, const TileArgs<float>& A, unsigned grid)
-{
-    return launch_tiles<float>(d, level0, P, A, grid);
-}
+template int launch_gather_tiles<NB_TYPE, NB_NY>(nntc_b200_device*, int, const Planes&, const TileArgs<NB_TYPE>&, unsigned);
 
 }   // namespace nb

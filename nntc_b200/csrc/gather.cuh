@@ -1,5 +1,5 @@
 // gather.cuh: what the two gathers of the stencil assembly share - the tiled gather of gather.cu (planes whose visits
-// are tabled) and the walk of assemble.cu (any other plane) - the monomial layout, the visit tables, the launch
+// are tabled) and those of gather_any.cu (any other plane) - the monomial layout, the visit tables, the launch
 // arguments and the expansion of a slot's sums into its stored block.
 #pragma once
 
@@ -54,6 +54,7 @@ __host__ __device__ __forceinline__ int axis_class(int t, int n)
 // pixels of one (row, j) split by their place relative to the lanes (two apart at level 0, four at level 1) so that the
 // lanes of a warp, whose texels are that far apart, read consecutive 16-byte samples.
 constexpr int TILE0_W = 64, TILE0_H = 4, TILE0_PX = TILE0_W + 2, TILE0_PY = TILE0_H + 2;
+constexpr int TILE1_THREADS = 160;   // five warps: see k_gather_tile1
 constexpr int TILE1_W = 8, TILE1_H = 4, TILE1_PX = 4 * TILE1_W + 4, TILE1_PY = 4 * TILE1_H + 4;
 
 // Where site j of the tile's pixel (qx, qy) (from the margin's first pixel) sits in the tile.
@@ -268,11 +269,74 @@ inline size_t any_tile_bytes(int px, int py, int per)
            (size_t)(any_taps(px, per) + any_taps(py, per)) * 16;
 }
 
-int launch_gather_any(nntc_b200_device* d, const Planes& P, const TileArgs<double>& A, const AnyTiles& S,
-                      unsigned grid, size_t shared);
-int launch_gather_any(nntc_b200_device* d, const Planes& P, const TileArgs<float>& A, const AnyTiles& S, unsigned grid,
+constexpr int WALK_THREADS = 128;   // threads of a k_gather_walk block
+
+struct WalkBlocks
+{
+    long long start[MAX_PLANES + 1];   // each plane's first block (a tiled plane has none)
+};
+
+__device__ __forceinline__ void cp_async16(void* dst, const void* src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+
+__device__ __forceinline__ void cp_async_wait_all()
+{
+    asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
+// The plane of a block (planes in descending order) and the block's number within the plane.
+template <typename TS>
+__device__ __forceinline__ int tile_plane(const TileArgs<TS>& A, int n, int& tile)
+{
+    int pl = n - 1;
+    while ((int)blockIdx.x >= A.bend[pl])
+        pl--;
+    tile = (int)blockIdx.x - (A.bend[pl] - A.btiles[pl]);
+    return pl;
+}
+
+// The gradient terms of channels first .. (two of FP64, four of FP32) in the samples' places, asynchronously where a
+// site's are 16 aligned bytes.
+template <typename TS, class Each>
+__device__ __forceinline__ void stage_terms(const TileArgs<TS>& A, float4* sy, int first, int c, Each each_site)
+{
+    constexpr int CH = sizeof(TS) == sizeof(float) ? 4 : 2;
+    if constexpr (sizeof(TS) == sizeof(float))
+    {
+        const float* t = (const float*)A.terms;
+        if (c == MAX_CH)
+            each_site([&](int at, size_t site) { cp_async16(sy + at, t + site * MAX_CH); });
+        else
+            each_site([&](int at, size_t site) {
+                float* dst = reinterpret_cast<float*>(sy + at);
+                for (int a = 0; a < c; a++)
+                    dst[a] = __ldg(t + site * c + a);
+            });
+    }
+    else
+    {
+        const double* t = (const double*)A.terms + first;
+        if (c % 2 == 0)
+            each_site([&](int at, size_t site) { cp_async16(sy + at, t + site * c); });
+        else
+            each_site([&](int at, size_t site) {
+                double* dst = reinterpret_cast<double*>(sy + at);
+                for (int a = 0; a < CH && first + a < c; a++)
+                    dst[a] = __ldg(t + site * c + a);
+            });
+    }
+}
+
+// The launches, one module per type of the sums and channel count NY of the other latent (gather.cu, gather_any.cu).
+template <typename TS, int NY>
+int launch_gather_tiles(nntc_b200_device* d, int level0, const Planes& P, const TileArgs<TS>& A, unsigned grid);
+template <typename TS, int NY>
+int launch_gather_any(nntc_b200_device* d, const Planes& P, const TileArgs<TS>& A, const AnyTiles& S, unsigned grid,
                       size_t shared);
-int launch_gather_tiles(nntc_b200_device* d, int level0, const Planes& P, const TileArgs<double>& A, unsigned grid);
-int launch_gather_tiles(nntc_b200_device* d, int level0, const Planes& P, const TileArgs<float>& A, unsigned grid);
+template <typename TS, int NY>
+int launch_gather_walk(nntc_b200_device* d, int level0, const Planes& P, const TileArgs<TS>& A, const WalkBlocks& B);
 
 }   // namespace nb

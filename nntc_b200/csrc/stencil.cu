@@ -14,7 +14,7 @@
 // - every plane of the chain in ONE launch (nb::Planes), one stream, no per-plane fan-out;
 // - the FP64 stencil stored structure-of-arrays [slot][i][j][texel], coalesced for a warp of consecutive texels, the FP32
 //   one by texel, whose kernels take a lane per row of a block;
-// - the assembly is assemble.cu's and gather.cu's; the reference-shaped one here, behind an option, keeps its 5 x nmono
+// - the assembly is assemble.cu's; the reference-shaped one here, behind an option, keeps its 5 x nmono
 //   monomial sums in shared memory (registers spill at C = 4);
 // - the conjugate-gradient iteration is 5 launches (matvec + <p,Ap>, alpha, update + preconditioner + <r,r> +
 //   <r,z>, beta, direction) and nothing else instead of 13, all planes in lockstep, and the stop is decided ON THE
