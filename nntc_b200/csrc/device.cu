@@ -675,9 +675,9 @@ static int device_create_impl(const nntc_b200_model* m, const float* const* chai
         const int mm = m->nin + 1;
         NB_CK(cudaMemset(d->reduction, 0, (size_t)(mm * (mm + 1) / 2 + m->nout * mm) * sizeof(double)));
     }
-    NB_CK(cudaMallocHost(&d->host_scalars, (size_t)MAX_PLANES * S_COUNT * sizeof(double)));
-    NB_CK(cudaMallocHost(&d->host_counters, (size_t)COUNTERS * sizeof(unsigned int)));
     NB_CK(cudaMallocHost(&d->host_stage, HOST_STAGE));
+    d->host_scalars = reinterpret_cast<double*>(d->host_stage + HOST_SCALARS);
+    d->host_counters = reinterpret_cast<unsigned int*>(d->host_stage + HOST_COUNTERS);
     // the set-up's copies and clears went to the legacy stream; the model's own stream does not wait for it
     NB_CK(cudaDeviceSynchronize());
     d->m.has_decoder = 0;
@@ -727,8 +727,6 @@ void nntc_b200_device_destroy(nntc_b200_device* d)
     if (d->stream)
         cudaStreamSynchronize(d->stream);
     cudaFree(d->arena);
-    cudaFreeHost(d->host_scalars);
-    cudaFreeHost(d->host_counters);
     cudaFreeHost(d->host_stage);
     for (const nntc_b200_device::Pending& p : d->kpending)
     {

@@ -155,12 +155,12 @@ struct nntc_b200_device
     size_t scratch_floats = 0, scratch_bytes = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev[4] = {};
-    double* host_scalars = nullptr;      // pinned, MAX_PLANES * S_COUNT
-    unsigned int* host_counters = nullptr;
     // Pinned staging of this handle's small transfers (one allocation, HOST_STAGE bytes): a ring that small uploads are
     // copied through without waiting for them, then fixed places that small results are fetched to and read after the
     // wait that ends their block.
     unsigned char* host_stage = nullptr;
+    double* host_scalars = nullptr;      // of the same allocation: MAX_PLANES * S_COUNT
+    unsigned int* host_counters = nullptr;
     size_t stage_at = 0;                 // the ring's next byte
     void* arena = nullptr;               // the one device allocation every buffer above is a slice of
     void* keep = nullptr;                // bc8: the outer repack loop's copy of both latents and the BC state
@@ -285,7 +285,9 @@ enum Fetched
     FETCH_BC_STATS = 3200,   // 2 doubles per plane
     FETCH_BYTES = 4096
 };
-constexpr size_t STAGE_RING = 60 * 1024, HOST_STAGE = STAGE_RING + FETCH_BYTES;
+constexpr size_t STAGE_RING = 60 * 1024, HOST_SCALARS = STAGE_RING + FETCH_BYTES;
+constexpr size_t HOST_COUNTERS = HOST_SCALARS + (size_t)MAX_PLANES * S_COUNT * sizeof(double);
+constexpr size_t HOST_STAGE = HOST_COUNTERS + (size_t)COUNTERS * sizeof(unsigned int);
 int fetch(nntc_b200_device* d, Fetched place, const void* src, size_t bytes);
 template <typename T>
 inline const T* fetched(const nntc_b200_device* d, Fetched place)
