@@ -1471,9 +1471,11 @@ __global__ void __launch_bounds__(THREADS, PER_SM) k_quant_colour(Planes P, Colo
 
 // A whole sweep, its four colours in order, in one launch, for planes of at most a tile an SM. A block takes a tile of
 // SWEEP_W x SWEEP_H texels, holds the corrections of the tile and a margin in shared memory, and takes the colours one
-// after another; what a later colour of the tile needs of the texels outside it is computed by the block itself - colour 0
-// three texels out (two up and down), colour 1 two, colour 2 one - from the corrections before the sweep, so that every
-// texel's step has exactly the inputs it has in four launches of one colour each, and blocks need not wait on one another.
+// after another; what a later colour of the tile needs of the texels outside it is computed by the block itself, from the
+// corrections before the sweep, so that every texel's step has exactly the inputs it has in four launches of one colour each,
+// and blocks need not wait on one another. Across, colour 3 reads colour 2 one texel out, that colour 1 and that colour 0:
+// colour 0 goes three texels out, colour 1 two, colour 2 one. Down, a tile starts and ends between an odd row and an even one:
+// its rows of colours 2 and 3 read colours 0 and 1 in the row below it and nothing else that is new, and none reads above.
 // The corrections are read from one vector and written to another (x and r in turn), and a tile's own texels alone are
 // written.
 //
@@ -1482,8 +1484,8 @@ __global__ void __launch_bounds__(THREADS, PER_SM) k_quant_colour(Planes P, Colo
 // 100 x 76: 58 -> 26 us). With more tiles than SMs the tiles' second wave costs as much again (175 k level-1 texels: 71
 // against 35 us), and at level 0 of 4 x 2048 x 1024 the colours side by side, at four blocks an SM, read a quarter less from
 // DRAM and still took 675 against 560 us (FP64: 1314 against 732 us), waiting at the colours' barriers.
-constexpr int SWEEP_W = 32, SWEEP_H = 28, SWEEP_MARGIN = 4;
-constexpr int SWEEP_COLS = (SWEEP_W + 2 * SWEEP_MARGIN) / 2, SWEEP_ROWS = (SWEEP_H + 2 * SWEEP_MARGIN) / 2;   // a colour's
+constexpr int SWEEP_W = 32, SWEEP_H = 28, SWEEP_MARGIN_X = 4, SWEEP_MARGIN_Y = 2;   // (even: a cell's colour is its texel's)
+constexpr int SWEEP_COLS = (SWEEP_W + 2 * SWEEP_MARGIN_X) / 2, SWEEP_ROWS = (SWEEP_H + 2 * SWEEP_MARGIN_Y) / 2;   // a colour's
 constexpr int SWEEP_CELLS = SWEEP_COLS * SWEEP_ROWS;
 constexpr int SWEEP_TILES = 148;
 // Threads: a colour's texels in one pass (FP64), or its rows in two or three (FP32).
@@ -1543,9 +1545,9 @@ __device__ __forceinline__ unsigned sweep_colour(const PlaneView& V, const Sweep
     constexpr int cx = COLOUR & 1, cy = COLOUR >> 1, cc = C * C;
     // this colour's texels of the tile and as far outside it as the later colours read
     constexpr int hx = COLOUR == 0 ? 3 : (COLOUR == 1 ? 2 : (COLOUR == 2 ? 1 : 0));
-    constexpr int hy = COLOUR <= 1 ? 2 : (COLOUR == 2 ? 1 : 0);
-    constexpr int rx0 = SWEEP_MARGIN - hx + ((SWEEP_MARGIN - hx) % 2 != cx), ry0 = SWEEP_MARGIN - hy + ((SWEEP_MARGIN - hy) % 2 != cy);
-    constexpr int nx = (SWEEP_MARGIN + SWEEP_W - 1 + hx - rx0) / 2 + 1, ny = (SWEEP_MARGIN + SWEEP_H - 1 + hy - ry0) / 2 + 1;
+    constexpr int rx0 = SWEEP_MARGIN_X - hx + ((SWEEP_MARGIN_X - hx) % 2 != cx), ry0 = SWEEP_MARGIN_Y + cy;
+    constexpr int nx = (SWEEP_MARGIN_X + SWEEP_W - 1 + hx - rx0) / 2 + 1, ny = SWEEP_H / 2 + (cy == 0 ? 1 : 0);
+    static_assert(SWEEP_H % 2 == 0 && SWEEP_W % 2 == 0, "tiles start at even texels");
     constexpr int TASKS = nx * ny;
     const int w = V.w, h = V.h;
     const size_t T = (size_t)w * h;
@@ -1561,7 +1563,7 @@ __device__ __forceinline__ unsigned sweep_colour(const PlaneView& V, const Sweep
             {
                 const int task = batch + (q * SWEEP_THREADS<TS> + (int)threadIdx.x) / C, i = (int)threadIdx.x % C;
                 const int rx = rx0 + 2 * (task % nx), ry = ry0 + 2 * (task / nx);
-                const int gx = x0 - SWEEP_MARGIN + rx, gy = y0 - SWEEP_MARGIN + ry;
+                const int gx = x0 - SWEEP_MARGIN_X + rx, gy = y0 - SWEEP_MARGIN_Y + ry;
                 double acc = 0.0;
                 if (task < TASKS && gx >= 0 && gx < w && gy >= 0 && gy < h)
                 {
@@ -1613,12 +1615,12 @@ __device__ __forceinline__ unsigned sweep_colour(const PlaneView& V, const Sweep
         }
         const int task = batch + (int)threadIdx.x;
         const int rx = rx0 + 2 * (task % nx), ry = ry0 + 2 * (task / nx);
-        const int gx = x0 - SWEEP_MARGIN + rx, gy = y0 - SWEEP_MARGIN + ry;
+        const int gx = x0 - SWEEP_MARGIN_X + rx, gy = y0 - SWEEP_MARGIN_Y + ry;
         if (task < TASKS && gx >= 0 && gx < w && gy >= 0 && gy < h)
         {
             const size_t t = (size_t)gy * w + gx, sp = stencil_pos(gx, gy, w, h);
-            const bool own = rx >= SWEEP_MARGIN && rx < SWEEP_MARGIN + SWEEP_W && ry >= SWEEP_MARGIN &&
-                             ry < SWEEP_MARGIN + SWEEP_H;
+            const bool own = rx >= SWEEP_MARGIN_X && rx < SWEEP_MARGIN_X + SWEEP_W && ry >= SWEEP_MARGIN_Y &&
+                             ry < SWEEP_MARGIN_Y + SWEEP_H;
             double nb[C];
             if constexpr (ROWS)
                 load_texel<C>(coupling + threadIdx.x * C, nb);
@@ -1721,7 +1723,7 @@ __global__ void __launch_bounds__(SWEEP_THREADS<TS>, 1) k_quant_sweep(Planes P, 
     for (int i = threadIdx.x; i < 4 * SWEEP_CELLS; i += SWEEP_THREADS<TS>)
     {
         const int rx = i % (2 * SWEEP_COLS), ry = i / (2 * SWEEP_COLS);
-        const int gx = x0 - SWEEP_MARGIN + rx, gy = y0 - SWEEP_MARGIN + ry;
+        const int gx = x0 - SWEEP_MARGIN_X + rx, gy = y0 - SWEEP_MARGIN_Y + ry;
         double x[2 * TileX<C>::PAIRS] = {};
         if (!A.first && gx >= 0 && gx < V.w && gy >= 0 && gy < V.h)
             load_texel<C>(xin + ((size_t)gy * V.w + gx) * C, x);
