@@ -144,25 +144,35 @@ static bool build_gather_table(int kc, std::vector<int4>& tab64, std::vector<int
 // The tiles test each pixel once for five warps, whatever comes of it, and stage its sites, which pays the more sites a
 // pixel has; a thread a (texel, slot) waits longer but keeps more of them in flight, so that it gains as the launch
 // grows. FP32 terms of four channels are staged side by side with the samples; an odd count of FP64 ones a value at a
-// time. Measured (us, tiles / walk; at 950, 2050, 5460 and 15666 tiles: 700 x 500 to 3000 x 2000), every slot:
-//   K = 0: FP64 2 channels 92 / 104, 159 / 150, 394 / 320, 1061 / 750; 3 channels 154 / 105, 262 / 154, 697 / 323,
-//          1930 / 761; FP32 2 channels 99 / 90, 170 / 143, 463 / 296, 1270 / 700; 4 channels 85 / 128, 149 / 179, 378 / 360,
-//          1034 / 895
-//   K = 1: FP64 2 channels 132 / 197, 229 / 291, 571 / 625, 1528 / 1496; 3 channels 206 / 220, 367 / 312, 939 / 669,
-//          2537 / 1624; FP32 2 channels 142 / 178, 242 / 282, 642 / 601, 1758 / 1448
-//   K = 2: FP64 2 channels 172 / 306, 296 / 434, 739 / 934, 1983 / 2191; 3 channels 259 / 329, 457 / 447, 1162 / 945,
-//          3200 / 2213; FP32 2 channels 182 / 258, 318 / 400, 810 / 849, 2229 / 1994
-//   K = 4: FP64 2 channels (5460 and 15666) 1172 / 1731, 3150 / 3953; 3 channels 2060 / 1771, 5808 / 4011; FP32 2 channels
-//          1265 / 1579, 3454 / 3685; 4 channels 1066 / 1835, 2913 / 4432
-// The diagonal blocks alone leave three of the five warps idle (FP64 2 channels at 400, 2050 and 5460 tiles: K = 0 36 / 66,
-// 139 / 89, 350 / 184; K = 2 69 / 197, 266 / 275, 666 / 570; K = 4 124 / 366, 431 / 532, 1119 / 1028).
-static int any_tiles_line(bool f32, int c, int sites, bool every_slot)
+// time. The diagonal blocks alone leave three of the five warps idle. Where the lines lie, from both at 179 to 57404 tiles
+// (300 x 200 to 5500 x 4000), level 0 of two and of four channels: the assembly's time in the walk over that in tiles, at
+// about 950, 2050, 5450 and 15700 tiles (31400 where it says so), mean of the two level-0 counts:
+//   every slot     K = 0                 K = 1                 K = 2                 K = 4
+//   FP64  1  .90 .82 .65 .61      1.16 1.06 .89 .83     1.40 1.17 1.00 .94    1.68 1.33 1.09 1.01
+//         2  1.03 .91 .76 .71     1.33 1.16 .98 .93     1.51 1.32 1.10 1.04   1.89 1.54 1.27 1.19 (1.17)
+//         3  .69 .62 .50 .46      1.00 .88 .73 .69      1.13 .97 .81 .76      1.33 1.08 .87 .79
+//         4  .88 .77 .64 .60      1.17 1.01 .86 .82     1.36 1.17 1.00 .94    1.74 1.38 1.11 1.02 (1.00)
+//   FP32 1-3 .91 .82 .63 .58      1.21 1.09 .87 .81     1.37 1.17 .96 .90     1.76 1.39 1.12 1.03 (1.00)
+//         4  1.31 1.06 .88 .81    1.66 1.34 1.11 1.04   1.85 1.48 1.23 1.16   2.34 1.84 1.47 1.35 (1.32)
+//   the diagonal blocks alone
+//   FP64  1  .78 .57 .41 .36      .99 .74 .57 .51       1.19 .85 .67 .59      1.46 .94 .70 .61
+//         2  .91 .69 .57 .50      1.12 .83 .73 .65      1.31 .99 .84 .74      1.67 1.15 .90 .79
+//         3  .61 .44 .34 .30      .82 .62 .55 .49       .95 .72 .58 .51       1.14 .78 .59 .52
+//         4  .71 .56 .55 .49      .94 .75 .71 .65       1.07 .90 .82 .74      1.55 1.02 .87 .78
+//   FP32 1-3 .80 .60 .42 .34      1.05 .78 .62 .53      1.24 .87 .68 .57      1.59 1.00 .74 .61
+//         4  .98 .84 .78 .67      1.21 1.02 .95 .82     1.39 1.13 1.06 .91    1.85 1.30 1.13 .98
+static int any_tiles_line(bool f32, int c, int kc, bool every_slot)
 {
-    const bool staged = f32 && c == MAX_CH;
-    const int base = staged ? 3200 : (!f32 && c % 2 != 0 ? 400 : 800);
-    if (every_slot)
-        return base * sites * sites;
-    return staged ? base / 2 * sites * sites : base * 3 / 4 * sites;
+    constexpr int ALL = 1 << 30;
+    constexpr int LINE[2][5][4] = {   // the sums' type and channels as above, then K = 0, 1, 2, 4
+        { { 700, 2500, 5000, 20000 }, { 1000, 5000, ALL, ALL }, { 400, 1050, 1700, 2700 }, { 500, 1800, 4500, 30000 },
+          { 700, 2800, 4000, 30000 } },
+        { { 650, 950, 1350, 1800 }, { 800, 1300, 2000, 2800 }, { 500, 700, 850, 1300 }, { 600, 850, 1200, 2100 },
+          { 700, 950, 1400, 2000 } }
+    };
+    constexpr int LINE_FP32_4[2][4] = { { 2500, ALL, ALL, ALL }, { 950, 1900, 5000, 10000 } };
+    const int slots = every_slot ? 0 : 1, k = kc < 3 ? kc : 3;
+    return f32 && c == MAX_CH ? LINE_FP32_4[slots][k] : LINE[slots][f32 ? 4 : c - 1][k];
 }
 
 // One of the gather's launches, for the other latent's channel count (ny).
@@ -276,7 +286,7 @@ static int gather_planes(nntc_b200_device* d, int level0, const Planes& P, int n
         }
     }
     A.site0[P.n] = at;
-    if (any_tiles > any_tiles_line(sizeof(TS) == sizeof(float), c, 1 + k, slots == SLOTS))
+    if (any_tiles > any_tiles_line(sizeof(TS) == sizeof(float), c, k, slots == SLOTS))
         any_tiles = 0;
     WalkBlocks B{};
     long long walk = 0;

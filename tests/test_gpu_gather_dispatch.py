@@ -63,7 +63,15 @@ def test_large_ragged_planes_of_few_sites_are_walked(c1, k, f32, tiled):
     assert gather_launches(mat, state, f32, k) == ((1, 0) if tiled else (0, 1))
 
 
-@pytest.mark.parametrize("c1,k", [(2, 0), (3, 1), (4, 1), (4, 4)])   # walked, walked, tiles, tiles
+# 7939 and 4428 tiles: the tiles are the faster up to any number at K = 2 and two FP64 channels, up to some thousands at K = 1
+@pytest.mark.parametrize("w,h,c1,k,f32,tiled", [(2000, 1500, 2, 2, 0, True), (1400, 1200, 2, 1, 0, True),
+                                                (1400, 1200, 3, 2, 0, False), (1400, 1200, 2, 2, 1, False)])
+def test_large_ragged_planes_by_channels_and_sites(w, h, c1, k, f32, tiled):
+    mat, state = material(materials.plane_sizes(w, h), 1, 2, c1, k)
+    assert gather_launches(mat, state, f32, k) == ((1, 0) if tiled else (0, 1))
+
+
+@pytest.mark.parametrize("c1,k", [(2, 0), (3, 1), (4, 1), (4, 4)])   # the diagonal blocks alone: walked, walked, walked, tiles
 def test_diagonal_blocks_alone(c1, k):
     """The matrix-free conjugate gradients' assembly: its gradient and diagonal blocks are the full assembly's bits."""
     mat, (dw, db, v0, v1) = material(ROUNDS, 1, 2, c1, k)
