@@ -322,15 +322,16 @@ int nntc_b200_objective_gradient(nntc_b200_device* d, const nntc_b200_model* m, 
 enum nntc_b200_option
 {
     /* 1: assemble the stencils with one thread per texel recomputing every site it touches, the reference's shape
-     * (src/solve_level1.cu:259-581); 0 (default): one pass per site for the gradient terms, then one thread per
-     * (texel, slot) for the monomial sums. */
+     * (src/solve_level1.cu:259-581); 0 (default): one pass per site for the gradient terms, then the monomial sums in
+     * tiles of texels whose sites are staged in shared memory (planes that no tile fits, and large level-1 planes of few
+     * sites a pixel, with one thread per texel and slot). */
     NNTC_B200_OPT_REFERENCE_SHAPED_ASSEMBLY = 0,
     /* 1: block (a)'s normal equations on the tcgen05 tensor cores with the site rows split into BF16 hi + lo parts
      * and FP32 accumulators, added in FP64 per 256 sites (the mixed-precision form; NOT the same bits: the sums hold
      * to about 1e-6 relative); 0 (default): exact products summed in FP64 (src/solve_decoder.cu:87-161). */
     NNTC_B200_OPT_MIXED_PRECISION_GRAM = 1,
     /* 1: the conjugate gradients of blocks (b) and (c') apply (H + lambda I) matrix-free from the decode's forward pass
-     * and its adjoint in FP32, with FP64 inner products and recurrences, and stop at 1e-6 of the right-hand side; only
+     * and its adjoint in FP32, with FP64 inner products and recurrences, and stop at 1e-7 of the right-hand side; only
      * the gradient and the diagonal blocks are assembled (the adjoint form; NOT the same bits). 0 (default): the
      * assembled FP64 stencil (src/solve_level1.cu:781-828, 1222-1338). The quantised sweeps assemble in full either way. */
     NNTC_B200_OPT_ADJOINT_CG = 2,

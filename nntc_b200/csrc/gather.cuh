@@ -36,7 +36,8 @@ __host__ __device__ constexpr bool mono_used(int L, int ny)
 // once, in the reference's site order, by running site_touches on a texel of that class; every texel of such a plane
 // walks its list instead of testing every site of its footprint. A class is a pair of per-axis classes: level 1's are
 // first / inner / last texel, level 0's first (even) / inner even / inner odd / last even / last odd. A plane one
-// texel wide or high, whose one texel would be both first and last, is left to the walk.
+// texel wide or high, whose one texel would be both first and last, is not tabled; level-1 planes that are not go to
+// k_gather_any1 where its tiles fit and are the faster, the rest, and level 0's, to k_gather_walk.
 
 constexpr int AXIS_CLASSES0 = 5, AXIS_CLASSES1 = 3;
 constexpr int GATHER_CLASSES = AXIS_CLASSES0 * AXIS_CLASSES0;
@@ -86,7 +87,7 @@ struct TileArgs
     int off[GATHER_CLASSES][SLOTS + 1];
     long long site0[MAX_PLANES + 1];
     int bend[MAX_PLANES];   // one past each plane's last block, the planes in descending order (the smallest first)
-    int btiles[MAX_PLANES]; // each plane's blocks (0: left to the walk)
+    int btiles[MAX_PLANES]; // each plane's blocks (0: not of this launch)
     int slots;              // slots gathered: SLOTS, or 1 for the diagonal blocks and the gradient alone
     int bc_copy;            // level 0, FP64, for the BC refinement: each block also into the block-major copy
     int plain;              // every monomial matrix is symmetric bit for bit and finite
